@@ -114,6 +114,18 @@ struct DevState {
   double skin;
 };
 
+// Programmatic dependent launch. Kernels of the step sequence are launched
+// with programmatic stream serialisation, so each may be scheduled while its
+// predecessor's last blocks still run. pdl_entry() is the first statement of
+// such a kernel: it lets the next kernel be scheduled, then waits until the
+// predecessor has completed and its writes are visible (griddepcontrol.wait
+// returns at once for a kernel launched without the attribute). Every kernel
+// therefore starts its real work only after all earlier work on the stream.
+__device__ __forceinline__ void pdl_entry() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 __device__ __forceinline__ uint32_t attr_state(uint32_t a) { return a & 15u; }
 __device__ __forceinline__ bool attr_old(uint32_t a) { return (a >> 4) & 1u; }
 __device__ __forceinline__ uint32_t attr_sfm(uint32_t a) { return (a >> 5) & 3u; }

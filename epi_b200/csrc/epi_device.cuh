@@ -12,18 +12,6 @@ inline int stride_blocks(int64_t n, int b, const LaunchCfg& lc) {
   return need < cap ? (need > 0 ? need : 1) : cap;
 }
 
-// Programmatic dependent launch. Kernels of the step sequence are launched
-// with programmatic stream serialisation, so each may be scheduled while its
-// predecessor's last blocks still run. pdl_entry() is the first statement of
-// such a kernel: it lets the next kernel be scheduled, then waits until the
-// predecessor has completed and its writes are visible (griddepcontrol.wait
-// returns at once for a kernel launched without the attribute). Every kernel
-// therefore starts its real work only after all earlier work on the stream.
-__device__ __forceinline__ void pdl_entry() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-}
-
 // One count per kernel launch (the first thread of the first block).
 __device__ __forceinline__ void count_launch(unsigned long long* launches) {
   if (launches && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) atomicAdd(launches, 1ull);

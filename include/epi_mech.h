@@ -313,7 +313,7 @@ int epi_adjoint(epi_ctx* ctx, int32_t nsteps, int32_t checkpoint_every, const ep
  * another allocator (a framework's caching allocator, or a pool sized once at
  * start-up against a fixed memory budget) and loops that must not allocate
  * once they run. The caller owns every buffer; the working storage is one
- * fixed file-scope device array (about 0.75 MB) that exists on every GPU
+ * fixed file-scope device array (about 1.4 MB) that exists on every GPU
  * that loads the library until the process exits.
  *
  * Inputs x, y, z, radius (n doubles each) and outputs conn (n * max_conn
