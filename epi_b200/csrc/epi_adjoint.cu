@@ -655,14 +655,7 @@ __global__ void k_gate_check(DevState S) {
     const TissueDev& T = S.tissues[t];
     const double4 p = S.pos_cur[i];
     const float4 b = S.bpos[i];
-    double ex = p.x - (double)b.x, ey = p.y - (double)b.y;
-    if (ex > T.hlx) ex -= T.lx;
-    else if (ex < -T.hlx) ex += T.lx;
-    if (ey > T.hly) ey -= T.ly;
-    else if (ey < -T.hly) ey += T.ly;
-    const double ez = p.z - (double)b.z;
-    const double lim = 0.5 * S.skin - 1e-3;
-    if (!(ex * ex + ey * ey + ez * ez <= lim * lim)) {
+    if (moved_too_far(S.skin, T, p.x, p.y, p.z, b)) {
       S.gate[1 + t] = 1;
       S.gate[0] = 1;
     }

@@ -369,6 +369,12 @@ bool conditional_rebuild(const epi_ctx* c) {
   return c->cfg.rebuild_gate == 1 || (c->cfg.rebuild_gate == 0 && c->ntissues == 1);
 }
 
+// The step-kernel form of a configuration: 0 is the faster of the register
+// forms for the precision (see launch_step_w).
+int32_t step_form(const epi_config& c) {
+  return c.variant != 0 ? c.variant : (c.precision == EPI_PREC_MIXED ? 4 : 3);
+}
+
 // Skin, step-kernel variant, candidate-search switch and rebuild node of the
 // context; the captured graphs hold them, so they are dropped.
 void apply_tuning(epi_ctx* c, double skin, int32_t variant, int32_t search_switch,
@@ -377,7 +383,7 @@ void apply_tuning(epi_ctx* c, double skin, int32_t variant, int32_t search_switc
   c->cfg.variant = variant;
   c->cfg.search_switch = search_switch;
   c->cfg.rebuild_gate = rebuild_gate;
-  c->lc.variant = variant == 0 ? 3 : variant;
+  c->lc.variant = step_form(c->cfg);
   c->lc.search_switch = search_switch > 0 ? search_switch : kDefaultSearchSwitch;
   destroy_graphs(c);
 }
@@ -746,7 +752,7 @@ int epi_create(epi_ctx** out, const epi_config* cfg) {
   EPI_CUDA(cudaSetDevice(c.device));
   epi_ctx* ctx = new epi_ctx();
   ctx->cfg = c;
-  ctx->lc.variant = c.variant == 0 ? 3 : c.variant;
+  ctx->lc.variant = step_form(c);
   ctx->lc.search_switch = c.search_switch > 0 ? c.search_switch : kDefaultSearchSwitch;
   int sms = 0;
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device) == cudaSuccess &&

@@ -190,114 +190,247 @@ __device__ __forceinline__ bool connected_pred(double d2, double lt, double ri, 
   return d2 <= __dmul_rn(__dmul_rn(__dmul_rn(lt, lt), rs), rs);
 }
 
-// Division and square root of the force laws: IEEE in the FP64 path, the
-// hardware approximations (MUFU reciprocal / reciprocal square root, about
-// 2 ulp) in the FP32 path.
-__device__ __forceinline__ double ldiv(double a, double b) { return a / b; }
+// Arithmetic of the forces with every rounding written out: one operation, one
+// rounding, and a multiply-add only where xfma says so. The compiler then
+// contracts nothing by itself, and every kernel that evaluates a force -- one
+// thread per particle or several lanes per particle -- gets the same bits.
+__device__ __forceinline__ float xmul(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ float xadd(float a, float b) { return __fadd_rn(a, b); }
+__device__ __forceinline__ float xsub(float a, float b) { return __fsub_rn(a, b); }
+__device__ __forceinline__ float xfma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double xmul(double a, double b) { return __dmul_rn(a, b); }
+__device__ __forceinline__ double xadd(double a, double b) { return __dadd_rn(a, b); }
+__device__ __forceinline__ double xsub(double a, double b) { return __dsub_rn(a, b); }
+__device__ __forceinline__ double xfma(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+// a . b of two vectors
+template <typename R>
+__device__ __forceinline__ R xdot(R ax, R ay, R az, R bx, R by, R bz) {
+  return xfma(az, bz, xfma(ax, bx, xmul(ay, by)));
+}
+
+// Division and reciprocal square root of the force laws: IEEE division and
+// CUDA's rsqrt (1 ulp) in the FP64 path, the hardware approximations (MUFU
+// reciprocal / reciprocal square root, about 2 ulp) in the FP32 path.
+__device__ __forceinline__ double ldiv(double a, double b) { return __ddiv_rn(a, b); }
 __device__ __forceinline__ float ldiv(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double lsqrt(double v) { return sqrt(v); }
-__device__ __forceinline__ float lsqrt(float v) { return v * rsqrtf(v); }
+__device__ __forceinline__ double lrsqrt(double v) { return rsqrt(v); }
+__device__ __forceinline__ float lrsqrt(float v) { return rsqrtf(v); }
+__device__ __forceinline__ float rcp_approx(float v) {
+  float r;
+  asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(v));
+  return r;
+}
+
+// Two FP32 values in one register pair: sm_100 adds, multiplies and
+// multiply-adds both with one instruction, each rounded as the scalar
+// operation would.
+struct F2 {
+  unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float lo, float hi) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(lo), "f"(hi));
+  return r;
+}
+__device__ __forceinline__ void f2_out(F2 a, float& lo, float& hi) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a.v));
+}
+__device__ __forceinline__ F2 xadd(F2 a, F2 b) {
+  F2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 xmul(F2 a, F2 b) {
+  F2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+  return r;
+}
+__device__ __forceinline__ F2 xfma(F2 a, F2 b, F2 c) {
+  F2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+  return r;
+}
+
+// FP64 path: the distance sqrt(d2) and 1 / d2 from i = 1 / sqrt(d2), each
+// corrected to within an ulp, as a square root and a division would give
+// (the laws subtract nearly equal numbers, so it would show). One rsqrt and
+// four multiply-adds stand for a square root and two divisions.
+__device__ __forceinline__ double dist_of(double d2, double i) {
+  const double d = xmul(d2, i);
+  return xfma(xmul(0.5, i), xfma(-d, d, d2), d);
+}
+__device__ __forceinline__ double inv_sq(double d2, double i) {
+  const double v = xmul(i, i);
+  return xfma(v, xfma(-d2, v, 1.0), v);
+}
 
 template <typename R>
-__device__ __forceinline__ R pow6(R v) { return v * v * v * v * v * v; }
+__device__ __forceinline__ R pow3(R v) { return xmul(xmul(v, v), v); }
 template <typename R>
-__device__ __forceinline__ R pow3(R v) { return v * v * v; }
+__device__ __forceinline__ R pow6(R v) {
+  return xmul(xmul(xmul(xmul(xmul(v, v), v), v), v), v);
+}
 
 // Force laws (epi5_MT/cell_interaction.cpp:77-285). Each takes the squared
 // distance d2 and radius sum rs of the pair and returns the coefficient that
-// cell_interaction_apply multiplies by DT and the separation (:48-66).
+// cell_interaction_apply multiplies by DT and the separation (:48-66). The
+// FP32 forms follow the reference's expressions with MUFU divisions; the
+// FP64 forms take the distance and its reciprocals from one rsqrt, because
+// the square root and the divisions of the plain expressions are a chain of
+// several hundred cycles per pair.
 template <typename R>
 struct Laws {
   R eps4, p_memb, der_der_const, k_total, k_desmosome, kspring, kspring_d, delta_r, para_ljp2,
       kspring_division, lj_thresh, ljt1sq;
+  R ljt1;        // LJ_THRESH - 1
+  R inv_ljt1sq;  // 1 / (LJ_THRESH - 1)^2
+  R memb_far;    // der_der_const (1 - p_memb) / p_memb
+  static constexpr bool kF32 = sizeof(R) == 4;
 
+  // eps4 u (u - 1)
+  __device__ __forceinline__ R lj_factor(R u) const {
+    return xmul(xmul(eps4, u), xsub(u, R(1)));
+  }
+  // the same for u = (q inv)^3, and divided by 1/inv, FP64
+  __device__ __forceinline__ R lj_inv(R q, R inv) const {
+    return xmul(lj_factor(pow3(xmul(q, inv))), inv);
+  }
   // ljmain, :103-111
   __device__ __forceinline__ R ljmain(R d2, R rs) const {
-    const R lj6 = ldiv(pow6(rs), pow3(d2));
-    return ldiv(eps4 * lj6 * (lj6 - R(1)), d2);
+    if constexpr (kF32) return ldiv(lj_factor(ldiv(pow6(rs), pow3(d2))), d2);
+    else return lj_inv(xmul(rs, rs), ldiv(R(1), d2));
   }
-  // adhesion, :113-124
-  __device__ __forceinline__ R adhesion(R d2, R rs, R k) const {
-    const R d = lsqrt(d2);
-    const R m1 = ldiv(d, rs) - R(1);
-    return (m1 + R(1) > lj_thresh) ? R(0) : -ldiv(k, d) * m1 * (R(1) - ldiv(m1 * m1, ljt1sq));
+  // adhesion, :113-124; inv_d = 1 / sqrt(d2)
+  __device__ __forceinline__ R adhesion(R d2, R inv_d, R rs, R k) const {
+    if constexpr (kF32) {
+      const R d = xmul(d2, inv_d);
+      const R m1 = xsub(ldiv(d, rs), R(1));
+      const R h = xsub(R(1), ldiv(xmul(m1, m1), ljt1sq));
+      return xadd(m1, R(1)) > lj_thresh ? R(0) : xmul(xmul(-ldiv(k, d), m1), h);
+    } else {
+      const R ratio = ldiv(dist_of(d2, inv_d), rs);
+      const R m1 = xsub(ratio, R(1));
+      const R c = xmul(xmul(xmul(-k, inv_d), m1), xfma(-xmul(m1, m1), inv_ljt1sq, R(1)));
+      return ratio > lj_thresh ? R(0) : c;
+    }
   }
   // is_near, :90-93
-  __device__ __forceinline__ bool near(R d2, R rs) const { return d2 < rs * rs; }
+  __device__ __forceinline__ bool near(R d2, R rs) const { return d2 < xmul(rs, rs); }
   // CI_der_to_der, :129-139
   __device__ __forceinline__ R der_der(R d2, R rs) const {
-    const R d = lsqrt(d2);
-    const R dd = d + delta_r;
-    if (dd < rs) {
-      const R lj6 = ldiv(pow6(rs), pow6(dd));
-      return ldiv(eps4 * lj6 * (lj6 - R(1)), d * dd) + para_ljp2;
+    const R inv_d = lrsqrt(d2);
+    R d, dd;
+    if constexpr (kF32) {
+      d = xmul(d2, inv_d);
+      dd = xfma(d2, inv_d, delta_r);
+    } else {
+      d = dist_of(d2, inv_d);
+      dd = xadd(d, delta_r);
     }
-    if (near(d2, rs)) return para_ljp2;
-    const R lj6 = ldiv(pow6(rs), pow6(dd));
-    return ldiv(eps4 * lj6 * (lj6 - R(1)), d * d) + para_ljp2;
+    const bool in = dd < rs;
+    if (!in && near(d2, rs)) return para_ljp2;
+    return xadd(ldiv(lj_factor(ldiv(pow6(rs), pow6(dd))), xmul(d, in ? dd : d)), para_ljp2);
   }
-  // CI_al_air_de_to_al_air_de_fix_mu, :141-152
+  // CI_al_air_de_to_al_air_de_fix_mu, :141-152. FP64: both sides from one
+  // rsqrt, then a select.
   __device__ __forceinline__ R aad(R d2, R rs, bool both_old) const {
-    if (near(d2, rs)) return ljmain(d2, rs);
-    return adhesion(d2, rs, both_old ? k_total : k_desmosome);
+    const R k = both_old ? k_total : k_desmosome;
+    if constexpr (kF32) {
+      if (near(d2, rs)) return ljmain(d2, rs);
+      return adhesion(d2, lrsqrt(d2), rs, k);
+    } else {
+      const R inv_d = lrsqrt(d2);
+      const R r2 = xmul(rs, rs);
+      const R c_lj = lj_inv(r2, inv_sq(d2, inv_d));
+      const R c_ad = adhesion(d2, inv_d, rs, k);
+      return d2 < r2 ? c_lj : c_ad;
+    }
   }
   // The same law in FP32 without a branch: both sides from one reciprocal
   // square root, then a select, so lanes of a warp on either side of
-  // is_near do not run both paths one after the other.
+  // is_near do not run both paths one after the other. Two MUFU operations
+  // in all (the reciprocal of rs is the other).
   __device__ __forceinline__ float aad_fused(float d2, float rs, bool both_old) const {
     const float inv_d = rsqrtf(d2);
-    const float inv_d2 = inv_d * inv_d;
-    const float r2 = rs * rs;
-    const float s = r2 * inv_d2;
-    const float lj6 = s * s * s;
-    const float c_lj = eps4 * lj6 * (lj6 - 1.f) * inv_d2;
-    const float m1 = __fdividef(d2 * inv_d, rs) - 1.f;
+    const float inv_d2 = xmul(inv_d, inv_d);
+    const float r2 = xmul(rs, rs);
+    const float u = pow3(xmul(r2, inv_d2));
+    const float c_lj = xmul(xfma(u, u, -u), xmul(eps4, inv_d2));
+    const float m1 = xfma(xmul(d2, inv_d), rcp_approx(rs), -1.f);
     const float k = both_old ? k_total : k_desmosome;
-    const float c_ad =
-        (m1 + 1.f > lj_thresh) ? 0.f : -k * inv_d * m1 * (1.f - __fdividef(m1 * m1, ljt1sq));
+    const float h = xfma(-xmul(m1, m1), inv_ljt1sq, 1.f);
+    const float c_ad = m1 > ljt1 ? 0.f : xmul(xmul(xmul(-k, inv_d), m1), h);
     return d2 < r2 ? c_lj : c_ad;
   }
   // CI_fix_mu_to_fix_mu, :154-162
   __device__ __forceinline__ R fixmu(R d2, R rs) const {
     if (near(d2, rs)) return ljmain(d2, rs);
-    return adhesion(d2, rs, k_desmosome);
+    return adhesion(d2, lrsqrt(d2), rs, k_desmosome);
   }
   // CI_mu_to_memb, :164-172 (spring = the MUSUME's spring_force_to_memb)
   __device__ __forceinline__ R mu_memb(R d2, R rs, R spring) const {
     if (near(d2, rs)) return ljmain(d2, rs);
-    return adhesion(d2, rs, spring);
+    return adhesion(d2, lrsqrt(d2), rs, spring);
+  }
+  // -(k / d) (d / a - 1)
+  __device__ __forceinline__ R spring(R d2, R inv_d, R a, R k) const {
+    if constexpr (kF32) {
+      const R d = xmul(d2, inv_d);
+      return xmul(-ldiv(k, d), xsub(ldiv(d, a), R(1)));
+    } else {
+      return xmul(xmul(-k, inv_d), xsub(ldiv(dist_of(d2, inv_d), a), R(1)));
+    }
   }
   // CI_fix_to_memb, :174-183
   __device__ __forceinline__ R fix_memb(R d2, R rs) const {
     if (near(d2, rs)) return ljmain(d2, rs);
-    const R d = lsqrt(d2);
-    return -ldiv(kspring, d) * (ldiv(d, rs) - R(1));
+    return spring(d2, lrsqrt(d2), rs, kspring);
   }
   // CI_memb_to_memb, :185-234; *bad set when |coef| > 100 (the reference aborts)
   __device__ __forceinline__ R memb_memb(R d2, R rs, bool* bad) const {
-    const R rs2 = rs * rs;
-    const R cr2 = rs2 * p_memb * p_memb;
+    const R rs2 = xmul(rs, rs);
+    const R cr2 = xmul(xmul(rs2, p_memb), p_memb);
+    const R rp = xmul(rs, p_memb);
     R tmp;
     if (d2 < cr2) {
-      const R lj6 = ldiv(pow3(cr2), pow3(d2));
-      tmp = ldiv(eps4 * lj6 * (lj6 - R(1)), d2);
+      if constexpr (kF32) tmp = ldiv(lj_factor(ldiv(pow3(cr2), pow3(d2))), d2);
+      else tmp = lj_inv(cr2, ldiv(R(1), d2));
     } else if (d2 < rs2) {
-      const R d = lsqrt(d2);
-      tmp = -ldiv(der_der_const, d) * (ldiv(d, rs * p_memb) - R(1));
+      tmp = spring(d2, lrsqrt(d2), rp, der_der_const);
     } else {
-      const R d = lsqrt(d2);
-      const R lam = (R(1) + p_memb) * rs;
-      const R lj6 = ldiv(pow6(rs * p_memb), pow6(lam - d));
-      tmp = -ldiv(der_der_const, rs) * ldiv(R(1) - p_memb, p_memb) -
-            ldiv(eps4 * (lj6 * (lj6 - R(1))), (lam - d) * d);
+      const R inv_d = lrsqrt(d2);
+      if constexpr (kF32) {
+        const R d = xmul(d2, inv_d);
+        const R v = xfma(xadd(R(1), p_memb), rs, -d);
+        const R u = ldiv(pow6(rp), pow6(v));
+        const R e = xmul(eps4, xmul(u, xsub(u, R(1))));
+        tmp = xfma(-ldiv(der_der_const, rs), ldiv(xsub(R(1), p_memb), p_memb),
+                   -ldiv(e, xmul(v, d)));
+      } else {
+        const R d = dist_of(d2, inv_d);
+        const R v = xfma(xadd(R(1), p_memb), rs, -d);
+        const R q = ldiv(rp, v);
+        tmp = xsub(ldiv(-memb_far, rs), ldiv(lj_factor(pow3(xmul(q, q))), xmul(v, d)));
+      }
     }
     *bad = fabs(tmp) > R(100);
     return tmp;
   }
   // CI_pair, :281-285 (rest = the first cell's spr_nat_len)
   __device__ __forceinline__ R pair(R d2, R rest) const {
-    const R d = lsqrt(d2);
-    return ldiv(-(kspring_division * (d - rest)), d);
+    const R inv_d = lrsqrt(d2);
+    if constexpr (kF32)
+      return ldiv(-xmul(kspring_division, xfma(d2, inv_d, -rest)), xmul(d2, inv_d));
+    else
+      return xmul(xmul(-kspring_division, xsub(dist_of(d2, inv_d), rest)), inv_d);
+  }
+  // wall_interaction, :287-294: the z displacement of a particle of radius r
+  // at height z
+  __device__ __forceinline__ R wall(R dt, R z, R r) const {
+    const R z2 = xmul(R(2), z);
+    const R ljm = lj_factor(pow6(r) / pow6(z)) / xmul(z2, z2);
+    return xmul(xmul(xmul(dt, ljm), R(2)), z);
   }
 };
 
@@ -317,6 +450,9 @@ __host__ __device__ inline Laws<R> make_laws(const Params& P) {
   L.kspring_division = R(P.kspring_division);
   L.lj_thresh = R(P.lj_thresh);
   L.ljt1sq = R((P.lj_thresh - 1.0) * (P.lj_thresh - 1.0));
+  L.ljt1 = R(P.lj_thresh - 1.0);
+  L.inv_ljt1sq = R(1.0 / ((P.lj_thresh - 1.0) * (P.lj_thresh - 1.0)));
+  L.memb_far = R(P.der_der_const * ((1.0 - P.p_memb) / P.p_memb));
   return L;
 }
 

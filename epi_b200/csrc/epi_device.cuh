@@ -36,10 +36,19 @@ void launch_pdl(void (*kernel)(Params...), int grid, int block, cudaStream_t s, 
   for (int64_t i = (lo) + (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (hi); \
        i += (int64_t)gridDim.x * blockDim.x)
 
-// _memb_bend_diff_factor with NEW_BEND_POT (cell_interaction.cpp:349-360)
-template <typename R>
-__device__ __forceinline__ R bend_factor(R c) {
-  return c >= R(0) ? (R(1) - c) : R(1) / ((R(1) + c) * (R(1) + c));
+// Has a particle of tissue T at (x, y, z) moved skin/2 from b, its position at
+// the tissue's last candidate rebuild? (The margin covers the float rounding
+// of b; NaN counts as moved.)
+__device__ __forceinline__ bool moved_too_far(double skin, const TissueDev& T, double x, double y,
+                                              double z, const float4& b) {
+  double ex = x - (double)b.x, ey = y - (double)b.y;
+  if (ex > T.hlx) ex -= T.lx;
+  else if (ex < -T.hlx) ex += T.lx;
+  if (ey > T.hly) ey -= T.ly;
+  else if (ey < -T.hly) ey += T.ly;
+  const double ez = z - (double)b.z;
+  const double lim = 0.5 * skin - 1e-3;
+  return !(xfma(ez, ez, xfma(ey, ey, xmul(ex, ex))) <= xmul(lim, lim));
 }
 
 // Separation of a pair as cell_interaction_apply computes it for its c1
@@ -57,13 +66,6 @@ __device__ __forceinline__ void pair_sep(const double4& p, const double4& pq, bo
   }
 }
 
-// Reciprocal square root and division: correctly rounded in the FP64 path,
-// the hardware approximations (about 2 ulp) in the FP32 path.
-__device__ __forceinline__ float frsqrt(float v) { return rsqrtf(v); }
-__device__ __forceinline__ double frsqrt(double v) { return 1.0 / sqrt(v); }
-__device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ double fdiv(double a, double b) { return a / b; }
-
 template <typename R>
 struct Vec3 {
   R x, y, z;
@@ -75,30 +77,5 @@ __device__ __forceinline__ Vec3<R> offset_of(const double4& q, const double4& p,
   return Vec3<R>{R(pdiff_h(q.x, p.x, T.lx, T.hlx)), R(pdiff_h(q.y, p.y, T.ly, T.hly)),
                  R(q.z - p.z)};
 }
-// Unit vector and length of b - a: the nv / dn (or mv / dm) that
-// _memb_bend_calc1 stores for a membrane particle (cell_interaction.cpp:296-309).
-template <typename R>
-struct Unit {
-  R x, y, z, d;
-};
-template <typename R>
-__device__ __forceinline__ Unit<R> unit_of(R x, R y, R z) {
-  const R s = x * x + y * y + z * z;
-  const R inv = frsqrt(s);
-  return Unit<R>{x * inv, y * inv, z * inv, s * inv};
-}
-template <typename R>
-__device__ __forceinline__ Unit<R> unit_ab(const Vec3<R>& a, const Vec3<R>& b) {
-  return unit_of(b.x - a.x, b.y - a.y, b.z - a.z);
-}
-template <typename R>
-__device__ __forceinline__ R dotu(const Unit<R>& a, const Unit<R>& b) {
-  return a.x * b.x + a.y * b.y + a.z * b.z;
-}
-template <typename R>
-__device__ __forceinline__ R cmp(const Unit<R>& v, int k) {
-  return k == 0 ? v.x : (k == 1 ? v.y : v.z);
-}
-
 }  // namespace
 }  // namespace epi

@@ -122,14 +122,13 @@ typedef struct epi_config {
                          extra); the reference allows 400 (define.h:80) */
   int32_t max_cand;   /* candidates per particle (>= max_conn) */
   double skin;        /* candidate margin, > 0 (default 0.1) */
-  int32_t variant;    /* step-kernel form: 0 = default (3); 1, 2 = the
+  int32_t variant;    /* step-kernel form: 0 = default (4; FP64: 3); 1, 2 = the
                          neighbours' positions copied asynchronously into
                          shared memory, 8 / 15 per thread at once (FP64: 4 /
-                         8); 3, 4 = gathered into registers four at a time
-                         (FP64: two), 3 / 4 resident 256-thread blocks per SM
-                         (FP64: 3 / 2). Same formulas; the compiler may fuse
-                         multiply-adds differently, so results agree to
-                         rounding. */
+                         8); 3, 4 = gathered into registers: four at a time
+                         with 3 resident 256-thread blocks per SM / two at a
+                         time with 4 (FP64: one with 3 / two with 2). The same
+                         arithmetic in every form. */
   int32_t search_switch; /* candidate search: rebuilds of at least this many
                          particles take one thread per particle, smaller ones
                          one warp per particle; 0 = default (49152) */
