@@ -19,7 +19,7 @@ LIB = PKG / "libepi_mech.so"
 # is checked before use (EPI_ERR_CHECK); for tests, not for timing
 LIB_CHECK = PKG / "libepi_mech_check.so"
 
-SOURCES = ["epi_kernels.cu", "epi_adjoint.cu", "epi_field.cu", "epi_capi.cu", "epi_noalloc.cu"]
+SOURCES = ["epi_kernels.cu", "epi_resident.cu", "epi_adjoint.cu", "epi_field.cu", "epi_capi.cu", "epi_noalloc.cu"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 

@@ -93,6 +93,7 @@ struct epi_ctx {
   int32_t ntissues = 0;
   int64_t n = 0;
   int32_t nbins = 0;
+  int32_t scan_bins = 0, scan_chunks = 0;  // the bin scan's cut (see rebuild_scan)
   int32_t nprep = 0, nprep_memb = 0;
   std::vector<TissueDev> tissues_h;
   // what the candidate lists depend on besides positions, as last uploaded
@@ -142,6 +143,8 @@ struct epi_ctx {
   unsigned long long* rebuilds = nullptr;
   int32_t* loop_left = nullptr;  // passes left in the step graph's device loop
   unsigned long long* launches = nullptr;  // step-sequence kernels executed
+  int32_t* res_sync = nullptr;   // grid barrier words of the resident kernel
+  int coop = 0;                  // the device takes cooperative launches
   ScanScratch scan{};
   // graphs: one per buffer parity, each replaying two steps
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -273,6 +276,8 @@ DevState make_state(epi_ctx* c, int cur) {
   S.rl_ppre = c->rl ? c->rl + 1 + c->ntissues : nullptr;
   S.rl_bpre = c->rl ? c->rl + 2 + 2 * c->ntissues : nullptr;
   S.ntissues = c->ntissues;
+  S.scan_bins = c->scan_bins;
+  S.scan_chunks = c->scan_chunks;
   S.prep = c->prep;
   S.nprep = c->nprep;
   S.nprep_memb = c->nprep_memb;
@@ -358,6 +363,37 @@ void enqueue_step(epi_ctx* c, int& cur, Timer* tm) {
     launch_step(make_state(c, cur), whole(c), c->cfg.precision, c->lc, c->stream, tm);
   }
   cur ^= 1;
+}
+
+// Whether the batch steps in one resident kernel (epi_resident.cu) instead of
+// the kernel sequence; the results are the same bits.
+bool resident(const epi_ctx* c, ResidentPlan* P) {
+  return c->coop && resident_plan(c->tissues_h.data(), c->ntissues, c->n, c->cfg.precision,
+                                  c->cfg.max_cand, c->lc, P);
+}
+
+bool conditional_rebuild(const epi_ctx* c);
+
+// nsteps steps in the resident kernel. graph: what the launch count stands
+// for, the replayed graph or the eager sequence (see epi_launch_count).
+int enqueue_resident(epi_ctx* c, const ResidentPlan& P, int32_t nsteps, bool graph) {
+  ensure_posf(c);
+  ResidentCfg rc{};
+  rc.sync = c->res_sync;
+  const int own = (c->nprep_memb > 0 ? 1 : 0) + (c->nprep > c->nprep_memb ? 1 : 0) + 1;
+  const bool skips = graph && conditional_rebuild(c);
+  rc.per_step = own + (skips ? 1 : 6);
+  rc.per_pair = graph ? 1 : 0;
+  rc.per_rebuild = skips ? 5 : 0;
+  // bounded runs: a kernel of a thousand steps lasts a few milliseconds
+  for (int32_t done = 0; done < nsteps;) {
+    const int32_t k = std::min(nsteps - done, 1024);
+    EPI_CUDA(launch_resident(make_state(c, c->cur), P, c->tissues_h[0], k, c->cfg.precision, rc,
+                             c->lc, c->stream));
+    c->cur ^= k & 1;
+    done += k;
+  }
+  return EPI_OK;
 }
 
 // Whether the step graph puts the candidate rebuild in a conditional node
@@ -501,6 +537,11 @@ int check_status(epi_ctx* c) {
 // (both parities' graphs captured on first use), plus one eager step for
 // an odd count.
 int enqueue_graph_steps(epi_ctx* c, int32_t nsteps) {
+  ResidentPlan P;
+  if (nsteps > 0 && resident(c, &P)) {
+    c->lists_fresh = false;
+    return enqueue_resident(c, P, nsteps, true);
+  }
   ensure_posf(c);  // never inside the captured graph
   const int32_t pairs = nsteps / 2;
   if (pairs > 0) {
@@ -515,6 +556,15 @@ int enqueue_graph_steps(epi_ctx* c, int32_t nsteps) {
   }
   if (nsteps % 2) enqueue_step(c, c->cur, nullptr);
   if (nsteps > 0) c->lists_fresh = false;
+  return EPI_OK;
+}
+
+// nsteps steps without a graph.
+int enqueue_steps(epi_ctx* c, int32_t nsteps) {
+  if (nsteps > 0) c->lists_fresh = false;
+  ResidentPlan P;
+  if (nsteps > 0 && resident(c, &P)) return enqueue_resident(c, P, nsteps, false);
+  for (int32_t k = 0; k < nsteps; ++k) enqueue_step(c, c->cur, nullptr);
   return EPI_OK;
 }
 
@@ -542,6 +592,10 @@ int set_device(epi_ctx* c) {
   catch (...) {                   \
     return EPI_ERR_CUDA;          \
   }
+
+// Entries of a tissue of nb bins in the bin arrays: the bins, a sentinel (the
+// tissue's end offset), and up to a multiple of four.
+int64_t bin_span(int64_t nb) { return (nb + 1 + 3) & ~(int64_t)3; }
 
 // Smallest non-negative double x <= hi with pred(x) true, for a predicate that
 // is false then true as x grows; +inf when pred(hi) is false. Non-negative
@@ -758,6 +812,8 @@ int epi_create(epi_ctx** out, const epi_config* cfg) {
   if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c.device) == cudaSuccess &&
       sms > 0)
     ctx->lc.num_sms = sms;
+  if (cudaDeviceGetAttribute(&ctx->coop, cudaDevAttrCooperativeLaunch, c.device) != cudaSuccess)
+    ctx->coop = 0;
   // The step sequence's stream gets the highest priority and the membrane
   // sums' side stream the lowest, so the rebuild chain (the critical path
   // of a step) takes SM slots first and the membrane blocks fill the rest.
@@ -778,6 +834,7 @@ int epi_create(epi_ctx** out, const epi_config* cfg) {
   if (rc == EPI_OK) rc = dev_alloc(&ctx->rebuilds, 1);
   if (rc == EPI_OK) rc = dev_alloc(&ctx->loop_left, 1);
   if (rc == EPI_OK) rc = dev_alloc(&ctx->launches, 1);
+  if (rc == EPI_OK) rc = dev_alloc(&ctx->res_sync, 2);
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->launches, 0, sizeof(unsigned long long)));
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->rebuilds, 0, sizeof(unsigned long long)));
   if (rc != EPI_OK) {
@@ -798,6 +855,7 @@ void epi_destroy(epi_ctx* ctx) {
   if (ctx->rebuilds) cudaFree(ctx->rebuilds);
   if (ctx->loop_left) cudaFree(ctx->loop_left);
   if (ctx->launches) cudaFree(ctx->launches);
+  if (ctx->res_sync) cudaFree(ctx->res_sync);
   if (ctx->status_h) cudaFreeHost(ctx->status_h);
   if (ctx->upin) cudaFreeHost(ctx->upin);
   if (ctx->copy_in) cudaStreamSynchronize(ctx->copy_in);
@@ -823,15 +881,17 @@ int epi_upload(epi_ctx* c, int32_t ntissues, const epi_tissue_view* tv, const ep
   int rc = set_device(c);
   if (rc) return rc;
   int64_t n = 0;
-  int64_t nbins = 0;
+  int64_t nbins = 0, max_bins = 0;
   for (int t = 0; t < ntissues; ++t) {
     epi_params P;
     if (params) P = params[t];
     else epi_params_default(&P);
     if ((rc = validate_tissue(tv[t], P))) return rc;
     n += tv[t].n;
-    nbins += (int64_t)((int)(tv[t].lx / 2.0 + 0.5)) * (int)(tv[t].ly / 2.0 + 0.5) *
-                 (int)(tv[t].lz / 2.0) + 1;
+    const int64_t nb = (int64_t)((int)(tv[t].lx / 2.0 + 0.5)) * (int)(tv[t].ly / 2.0 + 0.5) *
+                       (int)(tv[t].lz / 2.0);
+    nbins += bin_span(nb);
+    max_bins = std::max(max_bins, nb);
   }
   if (n > (int64_t)0x7fffffff || nbins > (int64_t)0x7ffffff0 || ntissues >= (1 << 24))
     return EPI_ERR_UNSUPPORTED;
@@ -880,6 +940,9 @@ int epi_upload(epi_ctx* c, int32_t ntissues, const epi_tissue_view* tv, const ep
   c->ntissues = ntissues;
   c->n = n;
   c->nbins = (int32_t)nbins;
+  // the bin scan: blocks of 4096 bins or more, at most 64 per tissue
+  c->scan_bins = (int32_t)std::max<int64_t>(4096, (max_bins + 63) / 64 + 3) & ~3;
+  c->scan_chunks = (int32_t)std::max<int64_t>(1, (max_bins + c->scan_bins - 1) / c->scan_bins);
   c->cand16 = cand16;
   c->cand_chunks = chunks;
   const std::vector<TissueDev> old_tissues = reuse ? c->tissues_h : std::vector<TissueDev>();
@@ -972,7 +1035,7 @@ int epi_upload(epi_ctx* c, int32_t ntissues, const epi_tissue_view* tv, const ep
     set_fp32_bounds(T);
     H.nfm = (int32_t)prep_f.size() - H.prep_f;
     pbase += v.n;
-    binbase += T.anx * T.any * T.anz + 1;  // + sentinel (end offset of the tissue)
+    binbase += (int32_t)bin_span((int64_t)T.anx * T.any * T.anz);
   }
   c->lc.simple = simple ? 1 : 0;
   c->lc.any_old = any_old ? 1 : 0;
@@ -1307,8 +1370,7 @@ int epi_interact_commit(epi_ctx* c) {
   Nvtx nvtx_range("epi_interact_commit");
   int rc = set_device(c);
   if (rc) return rc;
-  enqueue_step(c, c->cur, nullptr);
-  c->lists_fresh = false;
+  if ((rc = enqueue_steps(c, 1))) return rc;
   return check_status(c);
   EPI_GUARD_END
 }
@@ -1320,8 +1382,7 @@ int epi_step(epi_ctx* c, int32_t nsteps) {
   Nvtx nvtx_range("epi_step");
   int rc = set_device(c);
   if (rc) return rc;
-  for (int32_t k = 0; k < nsteps; ++k) enqueue_step(c, c->cur, nullptr);
-  if (nsteps > 0) c->lists_fresh = false;
+  if ((rc = enqueue_steps(c, nsteps))) return rc;
   return check_status(c);
   EPI_GUARD_END
 }

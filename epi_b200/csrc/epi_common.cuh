@@ -104,6 +104,8 @@ struct DevState {
   int32_t* rl_ppre;   // prefix sums of their particle counts (count + 1 entries)
   int32_t* rl_bpre;   // prefix sums of their bin counts
   int32_t ntissues;
+  int32_t scan_bins, scan_chunks;  // bins per block of the bin scan, blocks of the
+                                   // batch's largest tissue
   const int32_t* prep;  // membrane particles, then FIX/MUSUME cells
   int32_t nprep, nprep_memb;
   DevStatus* status;
@@ -513,7 +515,7 @@ __device__ __forceinline__ R eval_law(int law, const Laws<R>& L, R d2, R rs, boo
 struct TissueDev {
   int32_t pbase, n, nmemb, nder, nmx, nmy;
   int32_t anx, any, anz;  // reference grid (cell_connection.cpp:22-26)
-  int32_t binbase;        // first bin; a tissue owns anx*any*anz bins + 1 sentinel
+  int32_t binbase;        // first bin (a multiple of 4); anx*any*anz bins + 1 sentinel
   int32_t lattice;        // kLatticeSquare / kLatticeTriangular
   int32_t nadj;           // lattice links per membrane particle (4 / 6)
   int32_t mbase;          // index in prep of the tissue's first membrane particle

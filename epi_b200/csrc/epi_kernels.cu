@@ -26,6 +26,8 @@
 // deterministic and repeatable bit for bit.
 #include "epi_kernels.h"
 
+#include <algorithm>
+
 #include "epi_device.cuh"
 #include "epi_rebuild.cuh"
 #include "epi_step.cuh"
@@ -591,7 +593,8 @@ void launch_rebuild(const DevState& S, const Range& r, const ScanScratch&,
   timer_end(tm, KC_REBUILD_BIN, s);
   timer_begin(tm, KC_REBUILD_SCAN, s);
   const int nt = r.t1 - r.t0;
-  launch_pdl(k_scan_tissue, nt < lc.num_sms * 4 ? (nt > 0 ? nt : 1) : lc.num_sms * 4,
+  const int64_t units = (int64_t)nt * S.scan_chunks;
+  launch_pdl(k_scan_tissue, (int)std::max<int64_t>(1, std::min<int64_t>(units, lc.num_sms * 4)),
              kTissueScanThreads, s, S);
   timer_end(tm, KC_REBUILD_SCAN, s);
   timer_begin(tm, KC_REBUILD_SORT, s);

@@ -66,6 +66,28 @@ void launch_dermis(const DevState& S, int32_t f0, int32_t f1, const LaunchCfg& l
 // skin/2 since their last rebuild.
 void launch_step(const DevState& S, const Range& r, int precision, const LaunchCfg& lc,
                  cudaStream_t s, Timer* tm);
+// The same for nsteps steps of a small batch in one cooperative kernel
+// (epi_resident.cu), candidate rebuilds included.
+struct ResidentCfg {
+  int32_t* sync;      // two device words: the barrier's count and its abort flag
+  int32_t per_step, per_pair, per_rebuild;  // kernels of the sequence each step, each
+                      // second step and each rebuilding step stands for
+  double4* hist;      // null: S's two position buffers in turn; else step k reads
+                      // hist + k n, writes hist + (k + 1) n
+};
+// How a batch is laid out over the blocks; false: the batch is beyond what
+// the resident kernel takes (particles, or shared memory per block).
+struct ResidentPlan {
+  int32_t slots, grid, membs, tasks, terms, dealt, smem;
+};
+// beyond this the kernel sequence fills the GPU and is the faster one (both
+// 17 us per step at 147,456 particles)
+constexpr int64_t kResidentParticles = 131072;
+bool resident_plan(const TissueDev* tissues_h, int32_t ntissues, int64_t n, int precision,
+                   int max_cand, const LaunchCfg& lc, ResidentPlan* out);
+cudaError_t launch_resident(const DevState& S, const ResidentPlan& plan, const TissueDev& first,
+                            int32_t nsteps, int precision, const ResidentCfg& rc,
+                            const LaunchCfg& lc, cudaStream_t s);
 // Exact connection lists (connect_cell's result) into S.nbr / S.nn.
 void launch_exact_lists(const DevState& S, const Range& r, const LaunchCfg& lc,
                         cudaStream_t s);

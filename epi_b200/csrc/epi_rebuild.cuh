@@ -65,15 +65,22 @@ __device__ __forceinline__ int32_t block_excl_scan_n(int32_t v, int32_t* total) 
 // Reference grid checks: grid_init's bin (cell_connection.cpp:44-53) and the
 // range assert of connect_proc (:95-99). Returns the tissue-local bin or -1.
 // ---------------------------------------------------------------------------
+// (int)(v / AREA_GRID) of the IEEE division, by a multiplication wherever the
+// quotient is not within 1e-9 of an integer.
+__device__ __forceinline__ int32_t grid_index(double v) {
+  const double q = v * (1.0 / kAreaGrid);
+  const int32_t k = (int32_t)q;
+  const double f = q - (double)k;
+  return f > 1e-9 && f < 1.0 - 1e-9 ? k : (int32_t)(v / kAreaGrid);
+}
 __device__ __forceinline__ int32_t ref_bin(const TissueDev& T, double x, double y, double z,
                                            bool memb) {
-  const int32_t aix = (int32_t)((0.5 * T.lx - pdiff(0.5 * T.lx, x, T.lx)) / kAreaGrid);
-  const int32_t aiy = (int32_t)((0.5 * T.ly - pdiff(0.5 * T.ly, y, T.ly)) / kAreaGrid);
-  const int32_t aiz = (int32_t)(fmax(z, 0.0) / kAreaGrid);  // min0, utils.h:55-57
+  const int32_t aix = grid_index(0.5 * T.lx - pdiff(0.5 * T.lx, x, T.lx));
+  const int32_t aiy = grid_index(0.5 * T.ly - pdiff(0.5 * T.ly, y, T.ly));
+  const int32_t aiz = grid_index(fmax(z, 0.0));  // min0, utils.h:55-57
   bool bad = aix >= T.anx || aiy >= T.any || aiz >= T.anz || aix < 0 || aiy < 0 || aiz < 0;
   if (!memb) {
-    const int32_t cx = (int32_t)(x / kAreaGrid), cy = (int32_t)(y / kAreaGrid),
-                  cz = (int32_t)(z / kAreaGrid);
+    const int32_t cx = grid_index(x), cy = grid_index(y), cz = grid_index(z);
     bad |= cx >= T.anx || cy >= T.any || cz >= T.anz || cx < 0 || cy < 0 || cz < 0;
   }
   return bad ? -1 : (aix * T.any + aiy) * T.anz + aiz;
@@ -96,6 +103,19 @@ __device__ __forceinline__ void gate_compact(const DevState& S, int32_t t0, int3
       S.rl_count[0] = 0;
       S.rl_ppre[0] = 0;
       S.rl_bpre[0] = 0;
+    }
+    return;
+  }
+  if (t1 - t0 == 1) {  // one tissue: no scan
+    if (threadIdx.x == 0) {
+      const TissueDev& T = S.tissues[t0];
+      const bool g = S.gate[1 + t0] != 0;
+      if (clear) S.gate[0] = 0;
+      S.rl_count[0] = g ? 1 : 0;
+      S.rl_list[0] = t0;
+      S.rl_ppre[0] = S.rl_bpre[0] = 0;
+      S.rl_ppre[g ? 1 : 0] = g ? T.n : 0;
+      S.rl_bpre[g ? 1 : 0] = g ? T.anx * T.any * T.anz : 0;
     }
     return;
   }
@@ -192,40 +212,58 @@ __device__ __forceinline__ void rebuild_bin(const DevState& S) {
   }
 }
 
-// Per gated tissue, one block: exclusive scan of its bin counts into
-// starts, offset by the tissue's first particle, so each tissue's sorted
-// particles occupy its own slots [pbase, pbase + n). Each tissue's bins end
-// with a sentinel entry that receives the end offset. NT threads scan
-// 8 NT bins per tile.
+// Exclusive scan of the bin counts of every listed tissue into starts, offset
+// by the tissue's first particle, so each tissue's sorted particles occupy
+// its own slots [pbase, pbase + n). Each tissue's bins end with a sentinel
+// entry that receives the end offset. A tissue's bins are cut into chunks
+// (S.scan_chunks for the batch's largest tissue), a block each: it sums the
+// counts before its chunk, then scans the chunk, NT threads 8 NT bins at a
+// time. Cutting costs reads (of chunks before one's own) and saves the
+// serial chain: 262,144 bins took one block 192 us.
 template <int NT>
 __device__ __forceinline__ void rebuild_scan(const DevState& S) {
   const int32_t cnt = S.rl_count[0];
-  for (int32_t k = blockIdx.x; k < cnt; k += gridDim.x) {
+  __shared__ int32_t s_sum[NT / 32];
+  for (int32_t u = blockIdx.x; u < cnt * S.scan_chunks; u += gridDim.x) {
+    const int32_t k = u / S.scan_chunks, c = u - k * S.scan_chunks;
     const TissueDev& T = S.tissues[S.rl_list[k]];
     const int32_t nb = T.anx * T.any * T.anz;
+    const int32_t lo = c * S.scan_bins;
+    if (lo >= nb) continue;
+    const int32_t hi = lo + S.scan_bins < nb ? lo + S.scan_bins : nb;
     const int32_t* in = S.counts + T.binbase;
     int32_t* out = S.starts + T.binbase;
+    // binbase and lo are multiples of four
+    int32_t before = 0;
+    for (int32_t b = 4 * (int32_t)threadIdx.x; b < lo; b += 4 * NT) {
+      const int4 v = *reinterpret_cast<const int4*>(in + b);
+      before += (v.x + v.y) + (v.z + v.w);
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = before;
+    __syncthreads();
     int32_t carry = T.pbase;
+    for (int w = 0; w < NT / 32; ++w) carry += s_sum[w];
     constexpr int32_t kTile = NT * kScanItems;
-    for (int32_t base = 0; base < nb; base += kTile) {
+    for (int32_t base = lo; base < hi; base += kTile) {
       const int32_t b0 = base + threadIdx.x * kScanItems;
       int32_t v[kScanItems];
       int32_t sum = 0;
 #pragma unroll
       for (int q = 0; q < kScanItems; ++q) {
-        v[q] = b0 + q < nb ? in[b0 + q] : 0;
+        v[q] = b0 + q < hi ? in[b0 + q] : 0;
         sum += v[q];
       }
       int32_t tot;
       int32_t run = carry + block_excl_scan_n<NT>(sum, &tot);
 #pragma unroll
       for (int q = 0; q < kScanItems; ++q) {
-        if (b0 + q < nb) out[b0 + q] = run;
+        if (b0 + q < hi) out[b0 + q] = run;
         run += v[q];
       }
       carry += tot;
     }
-    if (threadIdx.x == 0) out[nb] = carry;
+    if (hi == nb && threadIdx.x == 0) out[nb] = carry;
     __syncthreads();
   }
 }
@@ -244,71 +282,92 @@ __device__ __forceinline__ void rebuild_scatter(const DevState& S) {
   }
 }
 
-// Sorts the particles of one bin (slots [s0, s1)) by index -- the
-// deterministic order the candidate search emits them in -- then tags
-// membrane particles and writes the sorted FP32 copy of their positions (x
-// and y as grid_init bins them, in [0, L)). Bins hold a few to a few dozen
-// particles: up to 24 are sorted in registers.
-__device__ __forceinline__ void sort_bin(const DevState& S, const TissueDev& T, int32_t s0,
-                                         int32_t s1) {
-  constexpr int kLocal = 24;  // a bin holds about 8 particles at unit density
-  if (s1 - s0 <= kLocal) {
-    uint32_t key[kLocal];
-    const int m = s1 - s0;
-    for (int k = 0; k < m; ++k) {
-      const uint32_t v = S.skey[s0 + k];
-      int q = k - 1;
-      while (q >= 0 && key[q] > v) {
-        key[q + 1] = key[q];
-        --q;
-      }
-      key[q + 1] = v;
-    }
-    for (int k = 0; k < m; ++k) S.skey[s0 + k] = key[k];
-  } else {
-    for (int32_t s = s0 + 1; s < s1; ++s) {
-      const uint32_t v = S.skey[s];
-      int32_t q = s - 1;
-      while (q >= s0 && S.skey[q] > v) {
-        S.skey[q + 1] = S.skey[q];
-        --q;
-      }
-      S.skey[q + 1] = v;
-    }
-  }
-  for (int32_t s = s0; s < s1; ++s) {
-    const uint32_t gi = S.skey[s];
-    if (!EPI_CHECKED(gi >= (uint32_t)T.pbase && gi < (uint32_t)(T.pbase + T.n), S.status,
-                     (int32_t)gi, s))
-      continue;
-    const bool memb = attr_state(S.attr[gi]) == ST_MEMB;
-    S.skey[s] = gi | (memb ? 0x80000000u : 0u);
-    S.rank[gi] = s;  // the particle's slot from here on (the search skips it)
-    // x and y as grid_init bins them (ref_bin): in [0, L); w: LJ_THRESH *
-    // radius, negative for a membrane particle (the search's reach and its
-    // membrane test)
-    const double4 pg = S.pos_cur[gi];
-    const double xc = 0.5 * T.lx - pdiff(0.5 * T.lx, pg.x, T.lx);
-    const double yc = 0.5 * T.ly - pdiff(0.5 * T.ly, pg.y, T.ly);
-    const float lw = (float)(T.P.lj_thresh * pg.w);
-    S.spos[s] = make_float4((float)xc, (float)yc, (float)pg.z, memb ? -lw : lw);
-  }
+// One sorted particle: its slot, the membrane tag and the FP32 copy of its
+// position (x and y as grid_init bins them, in [0, L)).
+__device__ __forceinline__ void place_particle(const DevState& S, const TissueDev& T, int32_t s,
+                                               uint32_t gi) {
+  if (!EPI_CHECKED(gi >= (uint32_t)T.pbase && gi < (uint32_t)(T.pbase + T.n), S.status,
+                   (int32_t)gi, s))
+    return;
+  const bool memb = attr_state(S.attr[gi]) == ST_MEMB;
+  S.skey[s] = gi | (memb ? 0x80000000u : 0u);
+  S.rank[gi] = s;  // the particle's slot from here on (the search skips it)
+  // x and y as grid_init bins them (ref_bin): in [0, L); w: LJ_THRESH *
+  // radius, negative for a membrane particle (the search's reach and its
+  // membrane test)
+  const double4 pg = S.pos_cur[gi];
+  const double xc = 0.5 * T.lx - pdiff(0.5 * T.lx, pg.x, T.lx);
+  const double yc = 0.5 * T.ly - pdiff(0.5 * T.ly, pg.y, T.ly);
+  const float lw = (float)(T.P.lj_thresh * pg.w);
+  S.spos[s] = make_float4((float)xc, (float)yc, (float)pg.z, memb ? -lw : lw);
 }
 
-// Per-bin insertion sort by particle index (bins hold a few to a few dozen
-// particles), then the sorted position copy the search streams through.
+// Sorts every bin's particles by index -- the deterministic order the
+// candidate search emits them in -- and writes the sorted FP32 copy the
+// search streams through. Eight lanes per bin: a lane holds every eighth
+// particle of it (a bin of 2.0 holds about six at unit density), finds its
+// rank by counting smaller indices and places it; bins of more than 32 are
+// sorted in place by one lane.
+constexpr int kBinLanes = 8;
 __device__ __forceinline__ void rebuild_sort(const DevState& S) {
   const int32_t cnt = S.rl_count[0];
   if (cnt == 0) return;
   const int32_t nbg = S.rl_bpre[cnt];
-  for (int32_t g = blockIdx.x * blockDim.x + threadIdx.x; g < nbg; g += gridDim.x * blockDim.x) {
-    const int32_t k = locate(S.rl_bpre, cnt, g);
-    const TissueDev& T = S.tissues[S.rl_list[k]];
-    const int32_t b = T.binbase + (g - S.rl_bpre[k]);
-    const int32_t s0 = S.starts[b], s1 = S.starts[b + 1];
-    if (s1 <= s0) continue;
-    S.counts[b] = 0;  // ready for the next binning
-    sort_bin(S, T, s0, s1);
+  const int sub = (int)threadIdx.x & (kBinLanes - 1), grp = ((int)threadIdx.x & 31) / kBinLanes;
+  constexpr int kBins = 32 / kBinLanes;  // bins per warp, in step with each other
+  const int32_t warps = (int32_t)((gridDim.x * blockDim.x) >> 5);
+  for (int32_t w = (int32_t)((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w * kBins < nbg;
+       w += warps) {
+    const int32_t g = w * kBins + grp;
+    int32_t s0 = 0, m = 0;
+    const TissueDev* T = S.tissues;
+    if (g < nbg) {
+      const int32_t k = locate(S.rl_bpre, cnt, g);
+      T = S.tissues + S.rl_list[k];
+      const int32_t b = T->binbase + (g - S.rl_bpre[k]);
+      s0 = S.starts[b];
+      m = S.starts[b + 1] - s0;
+      if (m > 0 && sub == 0) S.counts[b] = 0;  // ready for the next binning
+    }
+    if (m > 4 * kBinLanes) {
+      if (sub == 0) {
+        for (int32_t s = s0 + 1; s < s0 + m; ++s) {
+          const uint32_t v = S.skey[s];
+          int32_t q = s - 1;
+          while (q >= s0 && S.skey[q] > v) {
+            S.skey[q + 1] = S.skey[q];
+            --q;
+          }
+          S.skey[q + 1] = v;
+        }
+        for (int32_t s = s0; s < s0 + m; ++s) place_particle(S, *T, s, S.skey[s]);
+      }
+      m = 0;
+    }
+    __syncwarp();
+    const int32_t most = __reduce_max_sync(0xffffffffu, m);
+    uint32_t own[4];
+    int32_t rank[4] = {0, 0, 0, 0};
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int32_t e = u * kBinLanes + sub;
+      own[u] = e < m ? S.skey[s0 + e] : 0xffffffffu;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (u * kBinLanes >= most) break;
+#pragma unroll
+      for (int l = 0; l < kBinLanes; ++l) {
+        const uint32_t o = __shfl_sync(0xffffffffu, own[u], l, kBinLanes);
+#pragma unroll
+        for (int v = 0; v < 4; ++v) rank[v] += o < own[v] ? 1 : 0;
+      }
+    }
+    // (the shuffles keep every read of a key ahead of its replacement)
+    __syncwarp();
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (u * kBinLanes + sub < m) place_particle(S, *T, s0 + rank[u], own[u]);
   }
 }
 
@@ -437,35 +496,39 @@ __device__ __forceinline__ void finish_search(const DevState& S, int32_t i, int3
   S.bpos[i] = make_float4((float)p.x, (float)p.y, (float)p.z, 0.f);
 }
 
-// Few gated particles (a tissue or two): G = 32 lanes (one warp) per
-// particle, so the GPU has work for all its warps. The group's lanes fetch
-// the slot ranges of G bin columns at a time; a scan within the group lays
-// the ranges end to end, the group sweeps the concatenation G slots at a
-// time, and ballots keep the slot order. (Groups of 4 to 16 lanes emit the
-// same rows; they measured slower than one thread per particle for large
-// rebuilds, whose window set-up they repeat on every lane.)
+// Few gated particles (a tissue or two): G lanes per particle, so the GPU has
+// work for all its warps. The group's lanes fetch the slot ranges of G bin
+// columns at a time; a scan within the group lays the ranges end to end, the
+// group sweeps the concatenation G slots at a time, and ballots keep the slot
+// order. The groups of a warp run in step (to the longest of their loops):
+// left to their own lengths they ran one after the other.
 template <int G>
 __device__ __forceinline__ void cand_search_groups(const DevState& S, int32_t cnt,
                                                    int32_t ngated) {
   static_assert(G == 4 || G == 8 || G == 16 || G == 32, "group of 4 to 32 lanes");
+  constexpr unsigned kAll = 0xffffffffu;
   const int lane = threadIdx.x & 31;
   const int gl = lane & (G - 1);          // lane within the group
   const int gbase = lane & ~(G - 1);      // the group's first lane
-  const unsigned gmask = G == 32 ? 0xffffffffu : ((0xffffffffu >> (32 - G)) << gbase);
+  const unsigned gmask = G == 32 ? kAll : (1u << G) - 1u;
   const unsigned lt_mask = (1u << gl) - 1u;
   const int32_t groups = (gridDim.x * blockDim.x) / G;
   const int32_t cap = S.max_cand;
-  for (int32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / G; g < ngated; g += groups) {
+  for (int32_t g = (blockIdx.x * blockDim.x + threadIdx.x) / G; g - gbase / G < ngated;
+       g += groups) {
+    // a group past the end repeats the last particle and writes nothing
+    const bool in = g < ngated;
     int32_t t;
-    const int32_t i = gated_particle(S, cnt, g, &t);
+    const int32_t i = gated_particle(S, cnt, in ? g : ngated - 1, &t);
     const TissueDev& T = S.tissues[t];
     const SearchWindow W(S, T, i);
     const int32_t nx0 = W.xhi[0] - W.xlo[0] + 1, ny0 = W.yhi[0] - W.ylo[0] + 1;
     const int32_t ncx = nx0 + (W.nxr > 1 ? W.xhi[1] - W.xlo[1] + 1 : 0);
     const int32_t ncy = ny0 + (W.nyr > 1 ? W.yhi[1] - W.ylo[1] + 1 : 0);
     const int32_t ncol = ncx * ncy;  // column c = cx * ncy + cy
+    const int32_t most_col = G == 32 ? ncol : __reduce_max_sync(kAll, ncol);
     int32_t count = 0;
-    for (int32_t c0 = 0; c0 < ncol; c0 += G) {
+    for (int32_t c0 = 0; c0 < most_col; c0 += G) {
       const int32_t c = c0 + gl;
       int32_t lo = 0, len = 0;
       float cex = 0.f, cey = 0.f;
@@ -482,37 +545,38 @@ __device__ __forceinline__ void cand_search_groups(const DevState& S, int32_t cn
       int32_t incl = len;
 #pragma unroll
       for (int o = 1; o < G; o <<= 1) {
-        const int32_t v = __shfl_up_sync(gmask, incl, o, G);
+        const int32_t v = __shfl_up_sync(kAll, incl, o, G);
         if (gl >= o) incl += v;
       }
       const int32_t excl = incl - len;
-      const int32_t total = __shfl_sync(gmask, incl, G - 1, G);
-      for (int32_t base = 0; base < total; base += G) {
+      const int32_t total = __shfl_sync(kAll, incl, G - 1, G);
+      const int32_t most = G == 32 ? total : __reduce_max_sync(kAll, total);
+      for (int32_t base = 0; base < most; base += G) {
         const int32_t f = base + gl;
         // the last column whose range starts at or before f (k + step <= G - 1)
         int32_t k = 0;
 #pragma unroll
         for (int32_t step = G / 2; step > 0; step >>= 1) {
-          const int32_t e = __shfl_sync(gmask, excl, k + step, G);
+          const int32_t e = __shfl_sync(kAll, excl, k + step, G);
           if (e <= f) k += step;
         }
-        const int32_t s = __shfl_sync(gmask, lo, k, G) + (f - __shfl_sync(gmask, excl, k, G));
-        const float ex = __shfl_sync(gmask, cex, k, G), ey = __shfl_sync(gmask, cey, k, G);
+        const int32_t s = __shfl_sync(kAll, lo, k, G) + (f - __shfl_sync(kAll, excl, k, G));
+        const float ex = __shfl_sync(kAll, cex, k, G), ey = __shfl_sync(kAll, cey, k, G);
         bool hit = false;
         uint32_t key = 0;
         if (f < total) {
           key = S.skey[s];
           hit = W.hit(s, S.spos[s], ex, ey);
         }
-        const unsigned m = (__ballot_sync(gmask, hit) & gmask) >> gbase;
-        if (hit) {
+        const unsigned m = (__ballot_sync(kAll, hit) >> gbase) & gmask;
+        if (hit && in) {
           const int32_t kk = count + __popc(m & lt_mask);
           if (kk < cap) cand_set(S, i, kk + 1, (key & 0x7fffffffu) - (uint32_t)T.pbase);
         }
         count += __popc(m);
       }
     }
-    if (gl == 0) finish_search(S, i, count);
+    if (gl == 0 && in) finish_search(S, i, count);
   }
 }
 
@@ -564,6 +628,7 @@ struct RowWriter {
 template <bool k16, bool kWrap>
 __device__ __forceinline__ void search_particle(const DevState& S, const TissueDev& T,
                                                 const SearchWindow& W, int32_t i) {
+  constexpr int kWide = 2;  // slots in flight (four: 0.076 against 0.065 ms per step)
   const int32_t cap = S.max_cand;
   const int32_t nx0 = W.xhi[0] - W.xlo[0] + 1, ny0 = W.yhi[0] - W.ylo[0] + 1;
   const int32_t ncx = nx0 + (W.nxr > 1 ? W.xhi[1] - W.xlo[1] + 1 : 0);
@@ -609,22 +674,21 @@ __device__ __forceinline__ void search_particle(const DevState& S, const TissueD
       fetch();
     }
     if (!live) break;
-    const bool two = s + 1 < s_hi;
-    const uint32_t k0 = S.skey[s];
-    const float4 q0 = S.spos[s];
-    const uint32_t k1 = two ? S.skey[s + 1] : 0u;
-    const float4 q1 = two ? S.spos[s + 1] : make_float4(0.f, 0.f, 0.f, 0.f);
-    const bool h0 = W.template hit_t<kWrap>(s, q0, ex, ey);
-    const bool h1 = two && W.template hit_t<kWrap>(s + 1, q1, ex, ey);
-    if (h0) {
-      if (count < cap) row.put(S, i, (k0 & 0x7fffffffu) - pbase);
-      ++count;
+    uint32_t key[kWide];
+    float4 q[kWide];
+#pragma unroll
+    for (int u = 0; u < kWide; ++u) {
+      key[u] = s + u < s_hi ? S.skey[s + u] : 0u;
+      q[u] = s + u < s_hi ? S.spos[s + u] : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if (h1) {
-      if (count < cap) row.put(S, i, (k1 & 0x7fffffffu) - pbase);
-      ++count;
+#pragma unroll
+    for (int u = 0; u < kWide; ++u) {
+      if (s + u < s_hi && W.template hit_t<kWrap>(s + u, q[u], ex, ey)) {
+        if (count < cap) row.put(S, i, (key[u] & 0x7fffffffu) - pbase);
+        ++count;
+      }
     }
-    s += 2;
+    s += kWide;
   }
   row.close(S, i);
   finish_search(S, i, count);
@@ -647,17 +711,22 @@ __device__ __forceinline__ void cand_search_threads(const DevState& S, int32_t c
   }
 }
 
-// Below `thread_from` gated particles the warp-per-particle search (which
-// keeps the GPU busy with few particles) runs, from there on one thread per
-// particle. Both emit every row in the same order.
+// Below `thread_from` gated particles several lanes per particle search (which
+// keeps the GPU busy with few particles): a warp, or as many lanes, at least
+// four, as leave every particle a group of its own; from there on one thread
+// per particle. All emit every row in the same order.
 template <bool k16>
 __device__ __forceinline__ void rebuild_search(const DevState& S, int32_t thread_from) {
   const int32_t cnt = S.rl_count[0];
   if (blockIdx.x == 0) gate_clear(S, cnt);
   if (cnt == 0) return;
   const int32_t ngated = S.rl_ppre[cnt];
-  if (ngated < thread_from) cand_search_groups<32>(S, cnt, ngated);
-  else cand_search_threads<k16>(S, cnt, ngated);
+  const int64_t threads = (int64_t)gridDim.x * blockDim.x;
+  if (ngated >= thread_from) cand_search_threads<k16>(S, cnt, ngated);
+  else if ((int64_t)ngated * 32 <= threads) cand_search_groups<32>(S, cnt, ngated);
+  else if ((int64_t)ngated * 16 <= threads) cand_search_groups<16>(S, cnt, ngated);
+  else if ((int64_t)ngated * 8 <= threads) cand_search_groups<8>(S, cnt, ngated);
+  else cand_search_groups<4>(S, cnt, ngated);
 }
 
 }  // namespace

@@ -1,0 +1,583 @@
+// Resident stepping: one cooperative kernel that runs a whole sequence of
+// steps of a small batch.
+//
+// A small batch (a tissue or a few dozen) does not fill the GPU: a step of
+// the kernel sequence is then a chain of launches and of dependent loads by
+// few threads -- 768 particles took 55 us per call, 36,864 took 19 us per
+// step of the replayed graph, of which the arithmetic is under 2. Here every
+// block stays on its SM for all steps:
+//   * every term of a step -- a candidate of a particle, a bending term or a
+//     lattice spring of a membrane particle -- is a task of its own thread,
+//     so the chain of a step is one gather and one evaluation deep whatever
+//     the row's length;
+//   * the terms meet in shared memory and one thread per particle sums them
+//     in the row's order and commits: the same operations in the same order
+//     as the thread-per-particle kernels, so the same bits;
+//   * the block's own positions, rows and constants stay in shared memory;
+//   * blocks meet at a grid barrier after every step (and between the phases
+//     of a candidate rebuild, which runs in the same kernel when some tissue
+//     is flagged).
+// Bound by latency: per step one barrier (about 1.5 us), one gather from L2
+// (0.4 us), and the evaluation, summing and committing chains. A step costs
+// 4.9 us for 768 particles (FP64; 21 in the graph), 6.9 for 36,864 (13.5),
+// 11.7 for 92,160 (16.1), and meets the sequence at 147,456 (17 both); FP64
+// forces 9.9 for 36,864 (18.1). Batches: 5 tissues of 57,984 particles 11.6
+// (19.4), 16 all-states tissues 21 (99).
+#include "epi_kernels.h"
+
+#include <algorithm>
+
+#include "epi_device.cuh"
+#include "epi_rebuild.cuh"
+#include "epi_step.cuh"
+
+namespace epi {
+namespace {
+
+constexpr int kTile = 8;
+constexpr int kResidentMaxLog = 4;  // consecutive particles dealt to a block at a time
+
+// Positions the run works on: step k reads pos(k), writes pos(k + 1).
+struct ResidentArgs {
+  int32_t nsteps;
+  int32_t slots;            // particles per block
+  int32_t membs;            // membrane particles a block may hold
+  int32_t tasks;            // pair terms a block holds at a time
+  int32_t terms;            // bending threads per membrane particle
+  int32_t dealt;            // tiles of particles are dealt round the blocks
+  int32_t thread_from;      // candidate search: a thread per particle from here on
+  unsigned* bar;            // barrier arrivals (zero at launch)
+  int32_t* abort;           // set when a barrier wait gave up (zero at launch)
+  int32_t per_step, per_pair, per_rebuild;  // launches counted (see epi_launch_count)
+  double4* hist;            // non-null: step k's positions go to hist + k n_total
+};
+
+// Waits of thread 0 of every block; a wait that is not met in kSpinLimit
+// polls (seconds) gives up: the error is recorded and every block leaves at
+// its next check.
+constexpr int kSpinLimit = 1 << 23;
+
+struct GridBarrier {
+  unsigned* bar;
+  int32_t* abort;
+  DevStatus* status;
+  unsigned target;
+  // flag: a word read by thread 0 after the barrier and returned to all
+  // threads of the block (the same value in every block: nothing writes it
+  // between this barrier and the next). False: some block gave up.
+  __device__ __forceinline__ bool sync(const int32_t* word, int32_t* value) {
+    __shared__ int32_t s_word, s_ok;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      target += gridDim.x;
+      // release: the block's writes (ordered before by the block barrier)
+      // are visible to whoever sees the count; acquire: and the other way
+      asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
+      unsigned seen;
+      int spins = 0;
+      int32_t ok = 1;
+      for (;;) {
+        asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+        if ((int32_t)(seen - target) >= 0) break;
+        if (++spins >= kSpinLimit || ((spins & 1023) == 0 && *(volatile int32_t*)abort)) {
+          if (spins >= kSpinLimit) {
+            raise_error(status, E_TIMEOUT, (int32_t)blockIdx.x, -1, (double)seen);
+            *(volatile int32_t*)abort = 1;
+          }
+          ok = 0;
+          break;
+        }
+      }
+      s_ok = ok;
+      s_word = word ? *(volatile const int32_t*)word : 0;
+    }
+    __syncthreads();
+    if (value) *value = s_word;
+    return s_ok != 0;
+  }
+};
+
+// The candidate rebuild of the flagged tissues, the phases of launch_rebuild
+// between barriers. The flag every block acted on (gate[0]) is cleared only
+// once all blocks are past the first barrier here.
+template <int NT>
+__device__ __noinline__ bool resident_rebuild(const DevState& S0, double4* pos, int32_t thread_from,
+                                              GridBarrier& B) {
+  DevState S = S0;
+  S.pos_cur = pos;
+  if (blockIdx.x == 0) gate_compact<NT>(S, 0, S.ntissues, false);
+  if (!B.sync(nullptr, nullptr)) return false;
+  if (blockIdx.x == 0 && threadIdx.x == 0) S.gate[0] = 0;
+  rebuild_bin(S);
+  if (!B.sync(nullptr, nullptr)) return false;
+  rebuild_scan<NT>(S);
+  if (!B.sync(nullptr, nullptr)) return false;
+  rebuild_scatter(S);
+  if (!B.sync(nullptr, nullptr)) return false;
+  rebuild_sort(S);
+  if (!B.sync(nullptr, nullptr)) return false;
+  if (S.cand16) rebuild_search<true>(S, thread_from);
+  else rebuild_search<false>(S, thread_from);
+  return B.sync(nullptr, nullptr);
+}
+
+constexpr int kLinks = kMembAdjTri + 1;  // springs of a membrane particle, and its wall
+constexpr int kTissues = 8;  // tissues of a block whose constants it keeps
+
+// What a block keeps of its particles (slots) in shared memory between steps:
+// an L2 load costs 700 cycles and more here, and after a barrier L1 holds
+// nothing. R: the arithmetic type of the forces.
+template <typename R>
+struct Slots {
+  using Pos = typename SiteOffsets<R>::Pos;
+  double4* pos;     // positions
+  double* sum;      // pair sums, 3 per slot
+  double* msum;     // membrane sums, 3 per membrane slot
+  Pos* own;         // the same as the forces see them (FP64 path: pos itself)
+  float4* bpos;     // positions at the last candidate rebuild
+  R* term;          // pair terms x | y | z (tasks each)
+  R* bend;          // bending terms t, g: 4 x terms per membrane slot
+  R* link;          // spring terms and the wall: 3 x kLinks per membrane slot
+  uint32_t* attr;
+  int32_t* off;     // slots + 1: first pair task of each slot
+  int32_t* at;      // membrane slot: its place in list
+  int32_t* list;    // slots of membrane particles
+  int32_t* jk;      // their lattice column and row (16 bits each)
+  uint32_t* task;   // pair tasks: partner (global index, 20 bits) | slot << 20
+  static constexpr bool kOwn = sizeof(R) == 4;
+  // terms: bending threads per membrane particle (kTriTerms, or with square
+  // lattices only kSquareTerms + 2)
+  static __host__ __device__ constexpr size_t bytes(int slots, int membs, int tasks, int terms) {
+    return (size_t)slots * (sizeof(double4) + 24 + (kOwn ? sizeof(float4) : 0) + sizeof(float4) + 8) +
+           (size_t)membs * 24 +
+           sizeof(R) * 3 * tasks + sizeof(R) * (4 * terms + 3 * kLinks) * membs +
+           4 * (slots + 4 + 2 * membs + tasks);
+  }
+  __device__ Slots(unsigned char* m, int slots, int membs, int tasks, int terms) {
+    pos = reinterpret_cast<double4*>(m);
+    bpos = reinterpret_cast<float4*>(pos + slots);
+    unsigned char* rest = reinterpret_cast<unsigned char*>(bpos + slots);
+    if constexpr (kOwn) {
+      own = reinterpret_cast<float4*>(rest);
+      rest += sizeof(float4) * slots;
+    } else {
+      own = pos;
+    }
+    sum = reinterpret_cast<double*>(rest);
+    msum = sum + 3 * slots;
+    bend = reinterpret_cast<R*>(msum + 3 * membs);
+    link = bend + 4 * terms * membs;
+    term = link + 3 * kLinks * membs;
+    attr = reinterpret_cast<uint32_t*>(term + 3 * tasks);
+    off = reinterpret_cast<int32_t*>(attr + slots);
+    at = off + slots + 1;
+    list = at + slots;
+    jk = list + membs;
+    task = reinterpret_cast<uint32_t*>(jk + membs);
+  }
+};
+
+// Bending term e of membrane particle i, evaluated by all lanes of a warp for
+// the terms they hold (live: this lane holds one). Square terms (square_term's
+// order) are taken over three consecutive sites of the row or column, s[0] ->
+// s[1] and s[1] -> s[2]; the last one (e = 5) takes its cosine from the row
+// two below (the reference reads memb_bb's ipn, :380), which the next lane
+// (e = 6) forms. Triangular ones (tri_term1, tri_term2) over three
+// neighbours. All sites are loaded before one is used.
+template <typename R>
+__device__ __forceinline__ BendTerm<R> bend_task(const DevState& S, int32_t i,
+                                                 const SiteOffsets<R>& off, const MembSites& M,
+                                                 bool tri, int e, bool live) {
+  using Pos = typename SiteOffsets<R>::Pos;
+  int32_t site[3] = {i, i, i};
+  const int kind = square_kind(e < 6 ? e : 0);
+  if (!live) {
+  } else if (tri) {
+    const int k = e < 6 ? e : e - 6;
+    site[0] = M.tri(k);
+    site[1] = M.tri(k == 5 ? 0 : k + 1);
+    site[2] = e < 6 ? M.tri_ring(k) : M.tri(k >= 4 ? k - 4 : k + 2);
+  } else {
+    const bool col = e >= 3 && e < 6;
+    const int d = e == 6 ? 0 : (kind == 0 ? -1 : (kind == 1 ? 0 : -2));
+#pragma unroll
+    for (int k = 0; k < 3; ++k)
+      site[k] = M.square(S, col ? 0 : d + k, col ? d + k : (e == 6 ? -2 : 0));
+  }
+  Pos at[3];
+#pragma unroll
+  for (int k = 0; k < 3; ++k) at[k] = off.at(site[k]);
+  const Vec3<R> a = off.from(at[0]), b = off.from(at[1]), c = off.from(at[2]);
+  BendTerm<R> t{Vec3<R>{R(0), R(0), R(0)}, R(0)};
+  if (live && tri) t = e < 6 ? tri_term1(a, b, c) : tri_term2(a, b, c);
+  if (__any_sync(0xffffffffu, live && !tri)) {
+    const Unit<R> u = unit_ab(a, b), v = unit_ab(b, c);
+    R cs = v3_dot(u.v, v.v);
+    const R next = __shfl_down_sync(0xffffffffu, cs, 1);
+    if (e == 5) cs = next;
+    if (live && !tri && e < 6)
+      t = square_term(kind, kind == 0 ? v : u, kind == 0 ? u : v, cs);
+  }
+  return t;
+}
+
+// NT threads per block, one block per SM (more threads would halve their
+// registers: at 64 a thread spilled 45 words a step, and a reload misses L1
+// after a barrier: 9.2 us per step on 36,864 particles against 7.0). Block
+// b's particles (slots): of up to kTissues tissues, tiles of kTile particles
+// dealt round the blocks, so every block gets its share of the membrane; of
+// more, consecutive ones, so a block meets few tissues. The constants of its
+// tissues are in shared memory, those of a single one (kOne) arguments.
+template <typename R, bool kSimple, bool kOld, bool kOne, int NT, int kMin>
+__global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ DevState S0,
+                                                       const __grid_constant__ ResidentArgs A,
+                                                       const __grid_constant__ TissueDev T0) {
+  using Part = Particle<R, kSimple, kOld>;
+  using Pos = typename Part::Pos;
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ __align__(16) unsigned char s_tissue[kTissues][sizeof(TissueDev)];
+  __shared__ int32_t s_nm, s_t0;
+  const int slots = A.slots;
+  const Slots<R> K(smem, slots, A.membs, A.tasks, A.terms);
+  const int32_t n = (int32_t)S0.n_total;
+  const int tid = (int)threadIdx.x;
+  DevState S = S0;
+  if (A.hist) S.pos_cur = A.hist;
+  if (A.hist) S.pos_nxt = A.hist + n;
+  GridBarrier B{A.bar, A.abort, S0.status, 0u};
+  unsigned long long counted = 0;
+  int32_t flagged = *(volatile const int32_t*)S0.gate;
+  auto particle = [&](int slot) {
+    return kOne || A.dealt ? (slot / kTile * (int32_t)gridDim.x + (int32_t)blockIdx.x) * kTile + slot % kTile
+                : (int32_t)blockIdx.x * slots + slot;
+  };
+  // once: the slots' attributes, positions and membrane list, and the
+  // constants of the block's first tissues
+  if (tid == 0) {
+    s_nm = 0;
+    s_t0 = !A.dealt && particle(0) < n ? (int32_t)attr_tissue(S0.attr[particle(0)]) : 0;
+  }
+  __syncthreads();
+  for (int s = tid; s < slots; s += NT) {
+    const int32_t i = particle(s);
+    if (i >= n) continue;
+    const uint32_t a = S0.attr[i];
+    const double4 p = S.pos_cur[i];
+    K.attr[s] = a;
+    K.pos[s] = p;
+    if constexpr (Slots<R>::kOwn) K.own[s] = Part::own(p);
+    if (attr_state(a) == ST_MEMB) {
+      const TissueDev& T = S0.tissues[attr_tissue(a)];
+      const int32_t j = i - T.pbase, at = atomicAdd(&s_nm, 1);
+      K.list[at] = s;
+      K.jk[at] = j % T.nmx | (j / T.nmx) << 16;
+      K.at[s] = at;
+    }
+  }
+  if constexpr (!kOne) {
+    for (int t = 0; t < kTissues && s_t0 + t < S0.ntissues; ++t) {
+      const uint32_t* from = reinterpret_cast<const uint32_t*>(S0.tissues + s_t0 + t);
+      for (int w = tid; w < (int)(sizeof(TissueDev) / 4); w += NT)
+        reinterpret_cast<uint32_t*>(s_tissue[t])[w] = from[w];
+    }
+  }
+  auto tissue = [&](uint32_t a) -> const TissueDev& {
+    if constexpr (kOne) return T0;
+    const int32_t t = (int32_t)attr_tissue(a) - s_t0;
+    return t < kTissues ? *reinterpret_cast<const TissueDev*>(s_tissue[t])
+                        : S0.tissues[attr_tissue(a)];
+  };
+  // slots [c0, c1) hold the pair tasks listed in K.task
+  int c0 = 0, c1 = 0;
+  bool fresh = true;  // rows and rebuild positions are to be read
+  for (int32_t step = 0; step < A.nsteps; ++step) {
+    counted += A.per_step + ((step & 1) ? A.per_pair : 0);
+    if (flagged) {
+      counted += A.per_rebuild;
+      if (!resident_rebuild<NT>(S0, S.pos_cur, A.thread_from, B)) break;
+      fresh = true;
+    }
+    if (fresh) {
+      fresh = false;
+      int32_t carry = 0;
+      for (int base = 0; base < slots; base += NT) {
+        const int s = base + tid;
+        const int32_t i = s < slots ? particle(s) : n;
+        int32_t nc = 0;
+        if (i < n) {
+          nc = cand_count(S, i);
+          K.bpos[s] = S.bpos[i];
+        }
+        int32_t total;
+        const int32_t before = block_excl_scan_n<NT>(nc, &total);
+        if (s < slots) K.off[s] = carry + before;
+        carry += total;
+      }
+      if (tid == 0) K.off[slots] = carry;
+      c0 = c1 = 0;
+      __syncthreads();
+    }
+    if (!kSimple && S.nprep > S.nprep_memb) {
+      const int warps = (int)(gridDim.x * NT) >> 5;
+      for (int32_t e = S.nprep_memb + (int32_t)((blockIdx.x * NT + tid) >> 5); e < S.nprep;
+           e += warps)
+        dermis_cell(S, S.prep[e], tid & 31);
+      if (!B.sync(nullptr, nullptr)) break;
+    }
+    for (int from = 0; from < slots; from = c1) {
+      // the slots from `from` on whose pair tasks fit; listed once per
+      // rebuild when all do
+      if (c0 != from || c1 == from) {
+        __syncthreads();
+        c0 = from;
+        int lo = from + 1, hi = slots;
+        while (lo < hi) {
+          const int mid = (lo + hi + 1) >> 1;
+          if (K.off[mid] - K.off[c0] <= A.tasks) lo = mid;
+          else hi = mid - 1;
+        }
+        c1 = lo;
+        const int32_t t0 = K.off[c0], nt = K.off[c1] - t0;
+        for (int t = tid; t < nt; t += NT) {
+          int a = c0, b = c1;  // the slot of task t: off[a] <= t0 + t < off[b]
+          while (b - a > 1) {
+            const int mid = (a + b) >> 1;
+            if (K.off[mid] <= t0 + t) a = mid;
+            else b = mid;
+          }
+          const int32_t i = particle(a);
+          const int32_t q = tissue(K.attr[a]).pbase +
+                            (int32_t)cand_entry(S, i, t0 + t - K.off[a] + 1);
+          K.task[t] = (uint32_t)(EPI_CHECKED(q >= 0 && q < n, S.status, i, q) ? q : i) |
+                      (uint32_t)a << 20;
+        }
+        __syncthreads();
+      }
+      // every term of these slots: a thread each
+      const int32_t t0 = K.off[c0], np = K.off[c1] - t0;
+      R *tx = K.term, *ty = tx + A.tasks, *tz = ty + A.tasks;
+      const Pos* src;
+      if constexpr (Part::kFloatPos) src = S.posf_cur;
+      else src = S.pos_cur;
+      constexpr int kU = Part::kFloatPos ? 4 : 2;  // gathers in flight per thread
+      for (int base = tid; base < np; base += kU * NT) {
+        uint32_t w[kU];
+        Pos pq[kU];
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          if (base + u * NT < np) {
+            w[u] = K.task[base + u * NT];
+            pq[u] = src[w[u] & 0xfffffu];
+          }
+        }
+#pragma unroll
+        for (int u = 0; u < kU; ++u) {
+          const int t = base + u * NT;
+          if (t < np) {
+            const int slot = (int)(w[u] >> 20);
+            const uint32_t a = K.attr[slot];
+            Part P(S, particle(slot), a, K.own[slot], tissue(a));
+            const Vec3<R> v = P.term((int32_t)(w[u] & 0xfffffu), pq[u]);
+            P.report_bad();
+            tx[t] = v.x;
+            ty[t] = v.y;
+            tz[t] = v.z;
+          }
+        }
+      }
+      if (from == 0) {
+        // the membrane: bending terms, then lattice springs, A.terms and
+        // kLinks threads per particle, from the first warp on that took
+        // no or one pair task less
+        const int nm = s_nm, nb32 = (nm * A.terms + 31) & ~31, nl = nm * kLinks;
+        for (int t = (tid + NT - (np & ~31) % NT) % NT; t < nb32 + nl; t += NT) {
+          const bool spring = t >= nb32;
+          const int r = spring ? t - nb32 : t;
+          const int m = r / (spring ? kLinks : A.terms);
+          const int e = r - m * (spring ? kLinks : A.terms);
+          const bool in = m < nm;
+          const int slot = in ? K.list[m] : 0;
+          const int32_t i = particle(slot);
+          const TissueDev& T = tissue(K.attr[slot]);
+          const bool tri = T.lattice == kLatticeTriangular;
+          const SiteOffsets<R> off(S, K.own[slot], T);
+          const int32_t jk = in ? K.jk[m] : 0;
+          const MembSites M(T, i, jk & 0xffff, jk >> 16);
+          if (spring) {
+            if (!in) continue;
+            if (e == kMembAdjTri) {  // the wall
+              const double4 p = K.pos[slot];
+              K.link[3 * r] = p.z < p.w ? T.laws<R>().wall(R(T.P.dt), R(p.z), R(p.w)) : R(0);
+              continue;
+            }
+            if (e >= T.nadj) continue;
+            const int32_t q = M.link(S, tri, e);
+            const Vec3<R> v = link_term<R>(S, off, T, T.laws<R>(), R(T.P.dt), i, q, off.at(q));
+            R* o = K.link + 3 * r;
+            o[0] = v.x;
+            o[1] = v.y;
+            o[2] = v.z;
+          } else {
+            const bool live = in && e < (tri ? kTriTerms : kSquareTerms + 1);
+            const BendTerm<R> b = bend_task<R>(S, i, off, M, tri, e, live);
+            if (!live) continue;
+            R* o = K.bend + 4 * r;
+            o[0] = b.t.x;
+            o[1] = b.t.y;
+            o[2] = b.t.z;
+            o[3] = b.g;
+          }
+        }
+      }
+      __syncthreads();
+      // sums in the order of the thread-per-particle kernels, a thread per
+      // component: the slots' pair terms, then the membrane's
+      const int ns = c1 - c0, nm = from == 0 ? s_nm : 0;
+      for (int r = tid; r < 3 * (ns + nm); r += NT) {
+        if (r < 3 * ns) {
+          const int s = c0 + r / 3, c = r % 3;
+          const R* v = K.term + c * A.tasks;
+          double sum = 0.0;
+          const int end = K.off[s + 1] - t0;
+#pragma unroll 4
+          for (int t = K.off[s] - t0; t < end; ++t) sum = xadd(sum, double(v[t]));
+          K.sum[3 * s + c] = sum;
+        } else {
+          const int m = (r - 3 * ns) / 3, c = (r - 3 * ns) % 3, slot = K.list[m];
+          const TissueDev& T = tissue(K.attr[slot]);
+          const int nb = T.lattice == kLatticeTriangular ? kTriTerms : kSquareTerms;
+          const R* b = K.bend + 4 * A.terms * m;
+          R v = R(0);
+#pragma unroll 4
+          for (int e = 0; e < nb; ++e) v = xfma(b[4 * e + 3], b[4 * e + c], v);
+          double sum = double(xmul(R(T.P.dt * T.P.kbend), v));
+          const R* l = K.link + 3 * kLinks * m + c;
+#pragma unroll 2
+          for (int e = 0; e < T.nadj; ++e) sum = xadd(sum, double(l[3 * e]));
+          // (adding no wall, +0, changes nothing: the sum is not -0)
+          if (c == 2) sum = xadd(sum, double(l[3 * kMembAdjTri - 2]));
+          K.msum[3 * m + c] = sum;
+        }
+      }
+      __syncthreads();
+      // the commit, a thread per particle
+      for (int s = c0 + tid; s < c1; s += NT) {
+        const int32_t i = particle(s);
+        if (i >= n) continue;
+        const uint32_t a = K.attr[s];
+        const double4 p = K.pos[s];
+        Part P(S, i, a, K.own[s], tissue(a));
+        P.ax = K.sum[3 * s];
+        P.ay = K.sum[3 * s + 1];
+        P.az = K.sum[3 * s + 2];
+        double4 f = make_double4(0.0, 0.0, 0.0, 0.0);
+        if (attr_state(a) == ST_MEMB) {
+          const double* v = K.msum + 3 * K.at[s];
+          f = make_double4(v[0], v[1], v[2], 0.0);
+        }
+        const double4 q = P.finish(p, K.bpos[s], f);
+        K.pos[s] = q;
+        if constexpr (Slots<R>::kOwn) K.own[s] = Part::own(q);
+      }
+    }
+    if (A.hist) {
+      S.pos_cur = S.pos_nxt;
+      S.pos_nxt += n;
+    } else {
+      double4* t = S.pos_cur;
+      S.pos_cur = S.pos_nxt;
+      S.pos_nxt = t;
+    }
+    float4* tf = S.posf_cur;
+    S.posf_cur = S.posf_nxt;
+    S.posf_nxt = tf;
+    if (!B.sync(S0.gate, &flagged)) break;
+  }
+  if (blockIdx.x == 0 && tid == 0 && S0.launches) atomicAdd(S0.launches, counted);
+}
+
+// Kernel of a batch's form.
+constexpr int kThreads = 512;
+template <typename R, bool kOne>
+const void* kernel_of(const LaunchCfg& lc) {
+  if (lc.simple && lc.any_old) return (const void*)k_resident<R, true, true, kOne, kThreads, 1>;
+  if (lc.simple) return (const void*)k_resident<R, true, false, kOne, kThreads, 1>;
+  return (const void*)k_resident<R, false, true, kOne, kThreads, 1>;
+}
+
+constexpr size_t kSmemPerBlock = 216 * 1024;  // of 227 KB, less the static parts
+constexpr int kLeastSlots = 16;
+// pair terms per slot a block must have room for: all of a step's at unit
+// density, a part of them for batches of every cell state, whose membrane rows
+// are short and cell rows long (the rest of a step's follow in turns)
+constexpr int kLeastTasks = 8, kLeastTasksGeneral = 3;
+
+}  // namespace
+
+bool resident_plan(const TissueDev* T, int32_t ntissues, int64_t n, int precision, int max_cand,
+                   const LaunchCfg& lc, ResidentPlan* out) {
+  if (n <= 0 || n > kResidentParticles) return false;
+  ResidentPlan P{};
+  // an even share of the particles over all SMs, one block each
+  const int64_t share = ((n + lc.num_sms - 1) / lc.num_sms + kTile - 1) / kTile * kTile;
+  P.slots = (int32_t)std::max<int64_t>(share, kLeastSlots);
+  P.grid = (int32_t)((n + P.slots - 1) / P.slots);
+  P.dealt = ntissues <= kTissues ? 1 : 0;
+  bool tri = false;
+  int64_t membs = 0;
+  for (int32_t t = 0; t < ntissues; ++t) {
+    tri |= T[t].lattice == kLatticeTriangular;
+    // tiles the tissue's membrane touches, dealt round the blocks
+    const int64_t tiles = (T[t].pbase + T[t].nmemb + kTile - 1) / kTile - T[t].pbase / kTile;
+    membs += (tiles + P.grid - 1) / P.grid * kTile;
+  }
+  P.membs = (int32_t)std::min<int64_t>(P.slots, P.dealt ? membs : P.slots);
+  P.terms = tri ? kTriTerms : kSquareTerms + 2;
+  auto bytes = [&](int tasks) {
+    return precision == 1 ? Slots<float>::bytes(P.slots, P.membs, tasks, P.terms)
+                          : Slots<double>::bytes(P.slots, P.membs, tasks, P.terms);
+  };
+  // room for the pair terms of all slots at 24 partners each, as far as it
+  // goes, and for the longest row
+  const int least =
+      std::max(P.slots * (lc.simple ? kLeastTasks : kLeastTasksGeneral), max_cand);
+  P.tasks = std::max(P.slots * 24, max_cand);
+  while (P.tasks > least && bytes(P.tasks) > kSmemPerBlock) P.tasks -= std::min(64, P.tasks - least);
+  P.smem = (int32_t)bytes(P.tasks);
+  if (bytes(P.tasks) > kSmemPerBlock || P.slots > 4095) return false;
+  *out = P;
+  return true;
+}
+
+cudaError_t launch_resident(const DevState& S, const ResidentPlan& P, const TissueDev& first,
+                            int32_t nsteps, int precision, const ResidentCfg& rc,
+                            const LaunchCfg& lc, cudaStream_t s) {
+  const bool one = S.ntissues == 1;
+  const void* kernel = precision == 1 ? (one ? kernel_of<float, true>(lc) : kernel_of<float, false>(lc))
+                                      : (one ? kernel_of<double, true>(lc) : kernel_of<double, false>(lc));
+  cudaError_t e =
+      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P.smem);
+  if (e != cudaSuccess) return e;
+  ResidentArgs A;
+  A.nsteps = nsteps;
+  A.slots = P.slots;
+  A.membs = P.membs;
+  A.tasks = P.tasks;
+  A.terms = P.terms;
+  A.dealt = P.dealt;
+  A.thread_from = lc.search_switch;
+  A.bar = reinterpret_cast<unsigned*>(rc.sync);
+  A.abort = rc.sync + 1;
+  A.per_step = rc.per_step;
+  A.per_pair = rc.per_pair;
+  A.per_rebuild = rc.per_rebuild;
+  A.hist = rc.hist;
+  if ((e = cudaMemsetAsync(rc.sync, 0, 2 * sizeof(int32_t), s)) != cudaSuccess) return e;
+  DevState S1 = S;
+  TissueDev T0 = first;
+  void* args[] = {&S1, &A, &T0};
+  return cudaLaunchCooperativeKernel(kernel, dim3((unsigned)P.grid), dim3((unsigned)kThreads), args,
+                                     (size_t)P.smem, s);
+}
+
+}  // namespace epi

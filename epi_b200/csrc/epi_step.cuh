@@ -36,31 +36,40 @@ template <typename R>
 struct SiteOffsets;
 template <>
 struct SiteOffsets<double> {
+  using Pos = double4;
   const DevState& S;
   const double4 p;
   const TissueDev& T;
-  __device__ __forceinline__ SiteOffsets(const DevState& S_, int32_t, const double4& p_,
-                                         const TissueDev& T_)
+  __device__ __forceinline__ SiteOffsets(const DevState& S_, const double4& p_, const TissueDev& T_)
       : S(S_), p(p_), T(T_) {}
-  __device__ __forceinline__ Vec3<double> operator()(int32_t q) const {
-    return offset_of<double>(S.pos_cur[q], p, T);
+  static __device__ __forceinline__ double4 own(const DevState&, int32_t, const double4& p) {
+    return p;
   }
+  __device__ __forceinline__ double4 at(int32_t q) const { return S.pos_cur[q]; }
+  __device__ __forceinline__ Vec3<double> from(const double4& o) const {
+    return offset_of<double>(o, p, T);
+  }
+  __device__ __forceinline__ Vec3<double> operator()(int32_t q) const { return from(at(q)); }
 };
 template <>
 struct SiteOffsets<float> {
+  using Pos = float4;
   const DevState& S;
-  const float4 pf;
+  const float4 p;
   const TissueDev& T;
-  __device__ __forceinline__ SiteOffsets(const DevState& S_, int32_t i, const double4&,
-                                         const TissueDev& T_)
-      : S(S_), pf(S_.posf_cur[i]), T(T_) {}
-  __device__ __forceinline__ Vec3<float> operator()(int32_t q) const {
-    const float4 o = S.posf_cur[q];
-    // minimum image as d - L rint(d / L): lattice neighbours lie far
-    // closer than L/2, where it equals the compare-and-shift form
-    return Vec3<float>{wrap_f(xsub(o.x, pf.x), T.lxf, T.ilxf),
-                       wrap_f(xsub(o.y, pf.y), T.lyf, T.ilyf), xsub(o.z, pf.z)};
+  __device__ __forceinline__ SiteOffsets(const DevState& S_, const float4& p_, const TissueDev& T_)
+      : S(S_), p(p_), T(T_) {}
+  static __device__ __forceinline__ float4 own(const DevState& S, int32_t i, const double4&) {
+    return S.posf_cur[i];
   }
+  __device__ __forceinline__ float4 at(int32_t q) const { return S.posf_cur[q]; }
+  // minimum image as d - L rint(d / L): lattice neighbours lie far closer
+  // than L/2, where it equals the compare-and-shift form
+  __device__ __forceinline__ Vec3<float> from(const float4& o) const {
+    return Vec3<float>{wrap_f(xsub(o.x, p.x), T.lxf, T.ilxf),
+                       wrap_f(xsub(o.y, p.y), T.lyf, T.ilyf), xsub(o.z, p.z)};
+  }
+  __device__ __forceinline__ Vec3<float> operator()(int32_t q) const { return from(at(q)); }
 };
 
 // _memb_bend_diff_factor with NEW_BEND_POT (cell_interaction.cpp:349-360)
@@ -185,8 +194,9 @@ __device__ __forceinline__ BendTerm<R> tri_term2(const Vec3<R>& a, const Vec3<R>
 struct MembSites {
   int32_t pb, nmx, nmy, jj, kk, nmemb, self;
   __device__ __forceinline__ MembSites(const TissueDev& T, int32_t i)
-      : pb(T.pbase), nmx(T.nmx), nmy(T.nmy), jj((i - T.pbase) % T.nmx), kk((i - T.pbase) / T.nmx),
-        nmemb(T.nmemb), self(i) {}
+      : MembSites(T, i, (i - T.pbase) % T.nmx, (i - T.pbase) / T.nmx) {}
+  __device__ __forceinline__ MembSites(const TissueDev& T, int32_t i, int32_t jj_, int32_t kk_)
+      : pb(T.pbase), nmx(T.nmx), nmy(T.nmy), jj(jj_), kk(kk_), nmemb(T.nmemb), self(i) {}
   // column jj+dj, row kk+dk with periodic wrap; the same wiring as _memb_init
   // (cellmanager.cpp:114-158)
   __device__ __forceinline__ int32_t square(const DevState& S, int dj, int dk) const {
@@ -214,28 +224,27 @@ struct MembSites {
   }
 };
 
-// The spring of membrane particle i's link to q (_MEMB_interaction, :529-547,
-// applied once by the higher index): DT coef separation, seen from i.
+// The spring of membrane particle i's link to q at pq (_MEMB_interaction,
+// :529-547, applied once by the higher index): DT coef separation, seen from
+// i.
 template <typename R>
 __device__ __forceinline__ Vec3<R> link_term(const DevState& S, const SiteOffsets<R>& off,
-                                             const double4& p, const TissueDev& T,
-                                             const Laws<R>& L, R dt, int32_t i, int32_t q) {
+                                             const TissueDev& T, const Laws<R>& L, R dt, int32_t i,
+                                             int32_t q, const typename SiteOffsets<R>::Pos& pq) {
   const bool hi = i > q;
-  R dx, dy, dz, rs, d2;
+  const R rs = xadd(off.p.w, pq.w);
+  R dx, dy, dz, d2;
   if constexpr (sizeof(R) == 4) {
     // mixed path: the FP32 copies, as for the bending stencil; the
     // minimum-image FP32 difference is antisymmetric, so both ends of a
     // link see opposite forces
-    const Vec3<float> o = off(q);
+    const Vec3<float> o = off.from(pq);
     dx = -o.x;
     dy = -o.y;
     dz = -o.z;
-    rs = xadd(off.pf.w, S.posf_cur[q].w);
     d2 = xdot(dx, dy, dz, dx, dy, dz);
   } else {
-    const double4 pq = S.pos_cur[q];
-    pair_sep(p, pq, hi, T, dx, dy, dz);
-    rs = xadd(p.w, pq.w);
+    pair_sep(off.p, pq, hi, T, dx, dy, dz);
     d2 = dist_sq_exact(dx, dy, dz);
   }
   bool bad;
@@ -255,7 +264,7 @@ __device__ __forceinline__ double3 memb_force(const DevState& S, int32_t i) {
   const R dt = R(T.P.dt);
   const MembSites M(T, i);
   const double4 p = S.pos_cur[i];
-  const SiteOffsets<R> off(S, i, p, T);
+  const SiteOffsets<R> off(S, SiteOffsets<R>::own(S, i, p), T);
   const bool tri = T.lattice == kLatticeTriangular;
   Vec3<R> f{R(0), R(0), R(0)};
   if (tri) {
@@ -293,7 +302,8 @@ __device__ __forceinline__ double3 memb_force(const DevState& S, int32_t i) {
   const R s = R(T.P.dt * T.P.kbend);
   double ax = double(xmul(s, f.x)), ay = double(xmul(s, f.y)), az = double(xmul(s, f.z));
   for (int k = 0; k < T.nadj; ++k) {
-    const Vec3<R> w = link_term<R>(S, off, p, T, L, dt, i, M.link(S, tri, k));
+    const int32_t q = M.link(S, tri, k);
+    const Vec3<R> w = link_term<R>(S, off, T, L, dt, i, q, off.at(q));
     ax = xadd(ax, double(w.x));
     ay = xadd(ay, double(w.y));
     az = xadd(az, double(w.z));
@@ -319,6 +329,7 @@ struct Particle {
   // The mixed path gathers candidates' FP32 copies and forms separations in
   // FP32; the FP64 path gathers the FP64 positions.
   static constexpr bool kFloatPos = sizeof(R) == 4;
+  using Real = R;
   using Pos = typename std::conditional<kFloatPos, float4, double4>::type;
   const DevState& S;
   const int32_t i;
@@ -355,8 +366,12 @@ struct Particle {
   // a_: the particle's attribute word, p_: its current position
   __device__ __forceinline__ Particle(const DevState& S_, int32_t i_, uint32_t a_,
                                      const double4& p_)
+      : Particle(S_, i_, a_, own(p_), S_.tissues[attr_tissue(a_)]) {}
+  // T_: the particle's tissue, wherever its constants are at hand
+  __device__ __forceinline__ Particle(const DevState& S_, int32_t i_, uint32_t a_, const Pos& own_,
+                                     const TissueDev& T_)
       : S(S_), i(i_), a(a_), t(attr_tissue(a)), st(attr_state(a)),
-        T(S_.tissues[t]), L(T.laws<R>()), p(own(p_)),
+        T(T_), L(T.laws<R>()), p(own_),
         lt2(T.P.lj_thresh * T.P.lj_thresh), dt(R(T.P.dt)) {
     if (!kSimple && st != ST_MEMB) {
       pair_i = __ldg(&S.pair[i]);
@@ -521,8 +536,8 @@ struct Particle {
   }
 
   // p: the position; b: that of the tissue's last candidate rebuild; f: the
-  // membrane sums (membrane particles only)
-  __device__ __forceinline__ void finish(const double4& p, const float4& b, const double4& f) {
+  // membrane sums (membrane particles only). Returns the new position.
+  __device__ __forceinline__ double4 finish(const double4& p, const float4& b, const double4& f) {
     report_bad();
     if (st == ST_MEMB) {
       ax += f.x;
@@ -547,7 +562,7 @@ struct Particle {
       }
     }
     // pos_copy + the single wrap of cell_pos_periodic_fix
-    const double lx = T.lx, ly = T.ly, hlx = T.hlx, hly = T.hly;
+    const double lx = T.lx, ly = T.ly;
     double nx = p.x + ax, ny = p.y + ay;
     const double nz = p.z + az;
     if (nx > lx) nx -= lx;
@@ -566,6 +581,7 @@ struct Particle {
       S.gate[1 + t] = 1;
       S.gate[0] = 1;
     }
+    return make_double4(nx, ny, nz, p.w);
   }
 };
 

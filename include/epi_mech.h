@@ -216,7 +216,8 @@ int epi_rebuild_count(epi_ctx* ctx, int64_t* count);
 /* Kernels of the step sequence (rebuild, membrane prepass, dermis, step, and
  * the graph's condition and loop kernels) executed on the device since the
  * context was created, counted by the kernels themselves; kernels a graph's
- * conditional node skipped are not counted. */
+ * conditional node skipped are not counted. Small batches run their steps in
+ * one resident kernel, whose phases count as the kernels they stand for. */
 int epi_launch_count(epi_ctx* ctx, int64_t* count);
 /* Per-kernel timing: runs nsteps (not graph-captured) recording CUDA events
  * around each kernel class on the context stream. ms receives the summed
