@@ -60,97 +60,112 @@ __device__ __forceinline__ LawD operator+(const LawD& a, const LawD& b) {
   return LawD{a.c + b.c, a.dc_dr2 + b.dc_dr2, a.c_spring + b.c_spring, a.c_eps + b.c_eps};
 }
 
+// A pair's distance with its reciprocals, from one corrected rsqrt: the laws
+// and their derivatives divide by r and r2 up to six times, and an FP64
+// division is a chain of a dozen operations.
+struct Dist {
+  double r2, r, i, i2;  // r2, r, 1 / r, 1 / r2
+};
+__device__ __forceinline__ Dist dist_d(double r2) {
+  const double i = rsqrt(r2);
+  return Dist{r2, dist_of(r2, i), i, inv_sq(r2, i)};
+}
+
 // ljmain (:103-111): c = eps4 u (u - 1) / r2 with u = rs^6 / r2^3.
-__device__ __forceinline__ LawD ljmain_d(const Laws<double>& L, double r2, double rs) {
-  const double rs2 = rs * rs;
-  const double u = rs2 * rs2 * rs2 / (r2 * r2 * r2);
-  const double c = L.eps4 * u * (u - 1.0) / r2;
-  const double dc = -L.eps4 * u * (7.0 * u - 4.0) / (r2 * r2);
+__device__ __forceinline__ LawD ljmain_d(const Laws<double>& L, const Dist& d, double rs2) {
+  const double q = rs2 * d.i2;
+  const double u = q * q * q;
+  const double c = L.eps4 * u * (u - 1.0) * d.i2;
+  const double dc = -L.eps4 * u * (7.0 * u - 4.0) * (d.i2 * d.i2);
   return LawD{c, dc, 0.0, c};
 }
 
 // adhesion (:113-124) with spring constant k.
-__device__ __forceinline__ LawD adhesion_d(const Laws<double>& L, double r2, double rs,
+__device__ __forceinline__ LawD adhesion_d(const Laws<double>& L, const Dist& d, double rs,
                                            double k) {
-  const double r = sqrt(r2);
-  const double y = r / rs - 1.0;
+  const double irs = 1.0 / rs;
+  const double y = d.r * irs - 1.0;
   if (y + 1.0 > L.lj_thresh) return LawD{0.0, 0.0, 0.0, 0.0};
-  const double h = 1.0 - y * y / L.ljt1sq;
-  const double c = -(k / r) * y * h;
+  const double w = y * y * L.inv_ljt1sq;
+  const double h = 1.0 - w;
+  const double c = -(k * d.i) * y * h;
   // dc/dr = k y h / r^2 - (k / r) (1 - 3 y^2 / a^2) / rs
-  const double dcdr = k * y * h / r2 - (k / r) * (1.0 - 3.0 * y * y / L.ljt1sq) / rs;
-  return LawD{c, dcdr / (2.0 * r), c, 0.0};
+  const double dcdr = k * y * h * d.i2 - (k * d.i) * (1.0 - 3.0 * w) * irs;
+  return LawD{c, 0.5 * dcdr * d.i, c, 0.0};
 }
 
 // CI_al_air_de_to_al_air_de_fix_mu (:141-152).
-__device__ __forceinline__ LawD aad_d(const Laws<double>& L, double r2, double rs,
+__device__ __forceinline__ LawD aad_d(const Laws<double>& L, const Dist& d, double rs,
                                       bool both_old) {
-  if (r2 < rs * rs) return ljmain_d(L, r2, rs);
-  return adhesion_d(L, r2, rs, both_old ? L.k_total : L.k_desmosome);
+  if (d.r2 < rs * rs) return ljmain_d(L, d, rs * rs);
+  return adhesion_d(L, d, rs, both_old ? L.k_total : L.k_desmosome);
 }
 
 // CI_fix_mu_to_fix_mu (:154-162).
-__device__ __forceinline__ LawD fixmu_d(const Laws<double>& L, double r2, double rs) {
-  if (r2 < rs * rs) return ljmain_d(L, r2, rs);
-  return adhesion_d(L, r2, rs, L.k_desmosome);
+__device__ __forceinline__ LawD fixmu_d(const Laws<double>& L, const Dist& d, double rs) {
+  if (d.r2 < rs * rs) return ljmain_d(L, d, rs * rs);
+  return adhesion_d(L, d, rs, L.k_desmosome);
 }
 
 // CI_mu_to_memb (:164-172) with the MUSUME's spring_force_to_memb.
-__device__ __forceinline__ LawD mu_memb_d(const Laws<double>& L, double r2, double rs,
+__device__ __forceinline__ LawD mu_memb_d(const Laws<double>& L, const Dist& d, double rs,
                                           uint32_t sfm) {
-  if (r2 < rs * rs) return ljmain_d(L, r2, rs);
-  return adhesion_d(L, r2, rs, sfm_value(sfm, L));
+  if (d.r2 < rs * rs) return ljmain_d(L, d, rs * rs);
+  return adhesion_d(L, d, rs, sfm_value(sfm, L));
 }
 
-// CI_fix_to_memb (:174-183): c = -(kspring / r) (r / rs - 1) = kspring (1/r - 1/rs).
-__device__ __forceinline__ LawD fix_memb_d(const Laws<double>& L, double r2, double rs) {
-  if (r2 < rs * rs) return ljmain_d(L, r2, rs);
-  const double r = sqrt(r2);
-  const double c = -(L.kspring / r) * (r / rs - 1.0);
-  return LawD{c, -L.kspring / (2.0 * r2 * r), c, 0.0};
+// A spring c = -(k / r) (r / a - 1) = k (1/r - 1/a).
+__device__ __forceinline__ LawD spring_d(const Dist& d, double a, double k) {
+  const double c = -(k * d.i) * (d.r / a - 1.0);
+  return LawD{c, -0.5 * k * d.i * d.i2, c, 0.0};
+}
+
+// CI_fix_to_memb (:174-183).
+__device__ __forceinline__ LawD fix_memb_d(const Laws<double>& L, const Dist& d, double rs) {
+  if (d.r2 < rs * rs) return ljmain_d(L, d, rs * rs);
+  return spring_d(d, rs, L.kspring);
 }
 
 // CI_der_to_der (:129-139), dd = r + delta_R, u = (rs / dd)^6, h = u (u - 1):
 // eps4 h / (r dd) + para_ljp2 while dd < rs, para_ljp2 inside the radius
 // sum, eps4 h / r^2 + para_ljp2 beyond; dh/dr = -6 u (2 u - 1) / dd.
-__device__ __forceinline__ LawD der_der_d(const Laws<double>& L, double r2, double rs) {
-  const double r = sqrt(r2);
-  const double dd = r + L.delta_r;
-  if (!(dd < rs) && r2 < rs * rs) return LawD{L.para_ljp2, 0.0, 0.0, 0.0};
-  const double rs2 = rs * rs, dd2 = dd * dd;
-  const double u = rs2 * rs2 * rs2 / (dd2 * dd2 * dd2);
+__device__ __forceinline__ LawD der_der_d(const Laws<double>& L, const Dist& d, double rs) {
+  const double dd = d.r + L.delta_r;
+  if (!(dd < rs) && d.r2 < rs * rs) return LawD{L.para_ljp2, 0.0, 0.0, 0.0};
+  const double rs2 = rs * rs, idd = 1.0 / dd;
+  const double v = rs2 * (idd * idd);
+  const double u = v * v * v;
   const double h = u * (u - 1.0);
-  const double dh = -6.0 * u * (2.0 * u - 1.0) / dd;
+  const double dh = -6.0 * u * (2.0 * u - 1.0) * idd;
   double ce, dce;
   if (dd < rs) {
-    const double q = r * dd;
-    ce = L.eps4 * h / q;
-    dce = L.eps4 * (dh / q - h * (dd + r) / (q * q));
+    const double iq = d.i * idd;
+    ce = L.eps4 * h * iq;
+    dce = L.eps4 * (dh * iq - h * (dd + d.r) * (iq * iq));
   } else {
-    ce = L.eps4 * h / r2;
-    dce = L.eps4 * (dh / r2 - 2.0 * h / (r2 * r));
+    ce = L.eps4 * h * d.i2;
+    dce = L.eps4 * (dh * d.i2 - 2.0 * h * (d.i2 * d.i));
   }
-  return LawD{ce + L.para_ljp2, dce / (2.0 * r), 0.0, ce};
+  return LawD{ce + L.para_ljp2, 0.5 * dce * d.i, 0.0, ce};
 }
 
 // CI_pair (:281-285): c = -Kdiv (r - rest) / r, rest the higher index's
 // spr_nat_len.
-__device__ __forceinline__ LawD pair_d(const Laws<double>& L, double r2, double rest) {
-  const double r = sqrt(r2);
-  const double c = -(L.kspring_division * (r - rest)) / r;
-  return LawD{c, -L.kspring_division * rest / (2.0 * r2 * r), c, 0.0};
+__device__ __forceinline__ LawD pair_d(const Laws<double>& L, const Dist& d, double rest) {
+  const double c = -(L.kspring_division * (d.r - rest)) * d.i;
+  return LawD{c, -0.5 * L.kspring_division * rest * (d.i2 * d.i), c, 0.0};
 }
 
 // The law `law` (law_of) as a LawD.
-__device__ __forceinline__ LawD law_d(int law, const Laws<double>& L, double r2, double rs,
+__device__ __forceinline__ LawD law_d(int law, const Laws<double>& L, const Dist& d, double rs,
                                       bool both_old, uint32_t sfm) {
   switch (law) {
-    case L_OTHER: return ljmain_d(L, r2, rs);
-    case L_DER_DER: return der_der_d(L, r2, rs);
-    case L_AAD: return aad_d(L, r2, rs, both_old);
-    case L_FIXMU: return fixmu_d(L, r2, rs);
-    case L_FIX_MEMB: return fix_memb_d(L, r2, rs);
-    case L_MU_MEMB: return mu_memb_d(L, r2, rs, sfm);
+    case L_OTHER: return ljmain_d(L, d, rs * rs);
+    case L_DER_DER: return der_der_d(L, d, rs);
+    case L_AAD: return aad_d(L, d, rs, both_old);
+    case L_FIXMU: return fixmu_d(L, d, rs);
+    case L_FIX_MEMB: return fix_memb_d(L, d, rs);
+    case L_MU_MEMB: return mu_memb_d(L, d, rs, sfm);
     default: return LawD{0.0, 0.0, 0.0, 0.0};
   }
 }
@@ -173,27 +188,22 @@ __device__ __forceinline__ LawD memb_memb_d(const Laws<double>& L, double r2, do
   const double P = L.p_memb;
   const double rs2 = rs * rs;
   const double cr2 = rs2 * P * P;
-  if (r2 < cr2) {
-    const double u = cr2 * cr2 * cr2 / (r2 * r2 * r2);
-    const double c = L.eps4 * u * (u - 1.0) / r2;
-    return LawD{c, -L.eps4 * u * (7.0 * u - 4.0) / (r2 * r2), 0.0, c};
-  }
-  const double r = sqrt(r2);
-  if (r2 < rs2) {
-    const double c = -(L.der_der_const / r) * (r / (rs * P) - 1.0);
-    return LawD{c, -L.der_der_const / (2.0 * r2 * r), c, 0.0};
-  }
+  const Dist d = dist_d(r2);
+  if (r2 < cr2) return ljmain_d(L, d, cr2);
+  if (r2 < rs2) return spring_d(d, rs * P, L.der_der_const);
   const double lam = (1.0 + P) * rs;
-  const double v = lam - r;
+  const double v = lam - d.r;
   const double cr = rs * P;
-  const double cr2v = cr * cr / (v * v);
+  const double iv = 1.0 / v;
+  const double cr2v = cr * iv * (cr * iv);
   const double u = cr2v * cr2v * cr2v;
-  const double c_spring = -(L.der_der_const / rs) * ((1.0 - P) / P);
-  const double vr = v * r;
-  const double c_eps = -L.eps4 * u * (u - 1.0) / vr;
+  const double c_spring = -L.memb_far / rs;
+  const double ivr = iv * d.i;
+  const double c_eps = -L.eps4 * u * (u - 1.0) * ivr;
   // d/dr of u (u - 1) / (v r), with du/dr = 6 u / v and d(v r)/dr = v - r
-  const double dh = 6.0 * u * (2.0 * u - 1.0) / (v * vr) - u * (u - 1.0) * (v - r) / (vr * vr);
-  return LawD{c_spring + c_eps, -L.eps4 * dh / (2.0 * r), c_spring, c_eps};
+  const double dh =
+      6.0 * u * (2.0 * u - 1.0) * (iv * ivr) - u * (u - 1.0) * (v - d.r) * (ivr * ivr);
+  return LawD{c_spring + c_eps, -0.5 * L.eps4 * dh * d.i, c_spring, c_eps};
 }
 
 // _memb_bend_diff_factor (:349-360) and its derivative.
@@ -206,20 +216,20 @@ __device__ __forceinline__ double bf_d(double c) {
   return -2.0 / (e * e * e);
 }
 
-// Unit vector of b - a with its length.
+// Unit vector of b - a with the inverse of its length.
 struct U3 {
   D3 v;
-  double len;
+  double inv;
 };
 __device__ __forceinline__ U3 unit3(D3 a, D3 b) {
   const D3 w = b - a;
-  const double len = sqrt(dot(w, w));
-  return U3{(1.0 / len) * w, len};
+  const double inv = rsqrt(dot(w, w));
+  return U3{inv * w, inv};
 }
 // Adjoint of w = b - a from the adjoints of the unit vector (ub) and of the
 // length (lb): w_bar = (ub - (ub . u) u) / len + lb u; b += w_bar, a -= w_bar.
 __device__ __forceinline__ void unit3_back(const U3& u, D3 ub, double lb, D3& abar, D3& bbar) {
-  const D3 w = (1.0 / u.len) * (ub - dot(ub, u.v) * u.v) + lb * u.v;
+  const D3 w = u.inv * (ub - dot(ub, u.v) * u.v) + lb * u.v;
   bbar += w;
   abar -= w;
 }
@@ -227,6 +237,9 @@ __device__ __forceinline__ void unit3_back(const U3& u, D3 ub, double lb, D3& ab
 // Stencil slots of the bending term of particle k, as lattice offsets:
 // k, r, rr, l, ll, u, uu, b, bb, r of bb, rr of bb.
 constexpr int kSlots = 11;
+// The row half of BCALC names k, r, rr, l, ll (slots 0-4), the column half
+// the rest and k again (slot kSelf2): a thread each.
+constexpr int kSelf2 = 11;
 // Triangular lattice: k, its neighbour in direction i (slot 1 + i), and the
 // second-ring site c_i = memb[(i+1)%6]->memb[i] (slot 7 + i).
 constexpr int kTriSlots = 13;
@@ -246,12 +259,12 @@ struct HalfBar {
   D3 n, a, l, m;
   double D, E, w;
 };
-__device__ __forceinline__ double half_back(D3 yb, D3 n, D3 a, D3 l, D3 m, double D, double E,
+// iD, iE: 1 / D, 1 / E.
+__device__ __forceinline__ double half_back(D3 yb, D3 n, D3 a, D3 l, D3 m, double iD, double iE,
                                             double w, HalfBar& hb) {
   const double p = dot(n, a), q = dot(l, n);
   const double gp = bf(p), gq = bf(q), gw = bf(w);
   const double yn = dot(yb, n), ya = dot(yb, a), yl = dot(yb, l), ym = dot(yb, m);
-  const double iD = 1.0 / D, iE = 1.0 / E;
   const double val = -gp * (ya - p * yn) * iD + gq * ((yn - q * yl) * iE - (yl - q * yn) * iD) +
                      gw * (ym - w * yl) * iE;
   const double pb = (-bf_d(p) * (ya - p * yn) + gp * yn) * iD;
@@ -277,8 +290,8 @@ __device__ __forceinline__ double tri1_back(D3 y, D3 a, D3 b, D3 c, D3& abar, D3
                                             D3& cbar) {
   const D3 rb = d3(-b.x, -b.y, -b.z), ab = a - b, cb = c - b;
   const D3 N1 = cross(rb, ab), N2 = cross(ab, cb);
-  const double l1 = sqrt(dot(N1, N1)), l2 = sqrt(dot(N2, N2));
-  const D3 n1 = (1.0 / l1) * N1, n2 = (1.0 / l2) * N2;
+  const double i1 = rsqrt(dot(N1, N1)), i2 = rsqrt(dot(N2, N2));
+  const D3 n1 = i1 * N1, n2 = i2 * N2;
   const double d = dot(n1, n2);
   const D3 v = n2 - d * n1;
   const D3 t = cross(ab, v);
@@ -291,8 +304,8 @@ __device__ __forceinline__ double tri1_back(D3 y, D3 a, D3 b, D3 c, D3& abar, D3
   dbar -= dot(vbar, n1);
   n1bar += dbar * n2;
   n2bar += dbar * n1;
-  const D3 N1bar = (1.0 / l1) * (n1bar - dot(n1bar, n1) * n1);
-  const D3 N2bar = (1.0 / l2) * (n2bar - dot(n2bar, n2) * n2);
+  const D3 N1bar = i1 * (n1bar - dot(n1bar, n1) * n1);
+  const D3 N2bar = i2 * (n2bar - dot(n2bar, n2) * n2);
   const D3 rbbar = cross(ab, N1bar);
   abbar += cross(N1bar, rb);
   abbar += cross(cb, N2bar);
@@ -313,8 +326,8 @@ __device__ __forceinline__ double tri2_back(D3 y, D3 a, D3 b, D3 cc, D3& abar, D
   const D3 rc = d3(-cc.x, -cc.y, -cc.z), rb = d3(-b.x, -b.y, -b.z);
   const D3 bc = b - cc, ab = a - b;
   const D3 N1 = cross(rc, bc), N2 = cross(rb, ab);
-  const double l1 = sqrt(dot(N1, N1)), l2 = sqrt(dot(N2, N2));
-  const D3 n1 = (1.0 / l1) * N1, n2 = (1.0 / l2) * N2;
+  const double i1 = rsqrt(dot(N1, N1)), i2 = rsqrt(dot(N2, N2));
+  const D3 n1 = i1 * N1, n2 = i2 * N2;
   const double d = dot(n1, n2);
   const D3 v1 = n2 - d * n1, v2 = n1 - d * n2;
   const D3 t = cross(bc, v1) + cross(ab, v2);
@@ -329,8 +342,8 @@ __device__ __forceinline__ double tri2_back(D3 y, D3 a, D3 b, D3 cc, D3& abar, D
   dbar -= dot(v1bar, n1) + dot(v2bar, n2);
   n1bar += dbar * n2;
   n2bar += dbar * n1;
-  const D3 N1bar = (1.0 / l1) * (n1bar - dot(n1bar, n1) * n1);
-  const D3 N2bar = (1.0 / l2) * (n2bar - dot(n2bar, n2) * n2);
+  const D3 N1bar = i1 * (n1bar - dot(n1bar, n1) * n1);
+  const D3 N2bar = i2 * (n2bar - dot(n2bar, n2) * n2);
   const D3 rcbar = cross(bc, N1bar);
   bcbar += cross(N1bar, rc);
   const D3 rbbar = cross(ab, N2bar);
@@ -344,248 +357,268 @@ __device__ __forceinline__ double tri2_back(D3 y, D3 a, D3 b, D3 cc, D3& abar, D
   return g * yt;
 }
 
-// Membrane particles: bending, lattice-spring and wall adjoints. Writes the
-// bending products for the stencil sites to bend[e * kBendStride + slot],
-// the lattice + wall product at the particle itself to madj[e], and the
-// parameter partials to gmemb[e].
-__global__ void __launch_bounds__(256) k_adj_memb(DevState S, const double4* __restrict__ lam,
-                                                  double4* __restrict__ bend,
-                                                  double4* __restrict__ madj,
-                                                  double4* __restrict__ gmemb) {
-  GRID_STRIDE(e, 0, S.nprep_memb) {
+// The bending adjoint of every membrane particle: its products for the sites
+// of its stencil to bend[e * kBendStride + slot], its parameter partial in the
+// .w of slot 0 (and kSelf2). kLanes threads per particle. Square: the row
+// half of BCALC by the first, the column half by the second. Triangular
+// (kLanes = 8): terms k of both kinds by lane k < 6; a neighbour's products
+// come from the lanes whose terms name it. Bound by the latency of one
+// thread's chain, which is why it is cut: one thread per particle took 21 us
+// on 4,096 membrane particles, on 16 of the SMs.
+template <int kLanes>
+__global__ void __launch_bounds__(64) k_adj_bend(DevState S, const double4* lam,
+                                                 double4* bend) {
+  pdl_entry();
+  const int sub = (int)threadIdx.x & (kLanes - 1);
+  const int64_t stride = (int64_t)gridDim.x * blockDim.x / kLanes;
+  for (int64_t e0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+       e0 - (threadIdx.x & 31) / kLanes < S.nprep_memb; e0 += stride) {
+    // the lanes of a warp run in step; those past the end write nothing
+    const bool in = e0 < S.nprep_memb;
+    const int64_t e = in ? e0 : S.nprep_memb - 1;
     const int32_t i = S.prep[e];
     const TissueDev& T = S.tissues[attr_tissue(S.attr[i])];
-    const Laws<double>& L = T.lawd;
-    const double dt = T.P.dt;
     const int32_t pb = T.pbase, NMX = T.nmx, NMY = T.nmy;
     const int32_t j = i - pb, jj = j % NMX, kk = j / NMX;
-    auto site = [&](int dj, int dk) {
+    const double4 p = S.pos_cur[i];
+    const D3 yb = (T.P.dt * T.P.kbend) * xyz(lam[i]);
+    double4* out = bend + e * kBendStride;
+    auto put = [&](int slot, D3 v, double w) {
+      if (in) out[slot] = make_double4(v.x, v.y, v.z, w);
+    };
+    auto offset = [&](int32_t q) {
+      const Vec3<double> v = offset_of<double>(S.pos_cur[q], p, T);
+      return d3(v.x, v.y, v.z);
+    };
+    const bool tri = T.lattice == kLatticeTriangular;
+    if constexpr (kLanes == 8) {
+      // every lane takes part in the exchange
+      D3 ob[4] = {};  // of this lane's terms: a, b, c of kind 2, ring
+      double g = 0.0;
+      if (tri && sub < 6) {
+        auto site = [&](TriSite t) { return offset(pb + t.row * NMX + t.col); };
+        auto turn = [](int k) { return k >= 6 ? k - 6 : k; };
+        const TriSite s0{jj, kk};
+        const D3 a = site(tri_step(s0, sub, NMX, NMY));
+        const TriSite sb = tri_step(s0, turn(sub + 1), NMX, NMY);
+        const D3 b = site(sb), c = site(tri_step(s0, turn(sub + 2), NMX, NMY));
+        const D3 r = site(tri_step(sb, sub, NMX, NMY));
+        g = tri1_back(yb, a, b, r, ob[0], ob[1], ob[3]);
+        g += tri2_back(yb, a, b, c, ob[0], ob[1], ob[2]);
+      }
+      // neighbour k: a of term k, b of term k - 1, c of term k - 2
+      auto from = [&](D3 v, int k) {
+        const int l = sub >= k ? sub - k : sub - k + 6;
+        return d3(__shfl_sync(0xffffffffu, v.x, l, 8), __shfl_sync(0xffffffffu, v.y, l, 8),
+                  __shfl_sync(0xffffffffu, v.z, l, 8));
+      };
+      const D3 nb = ob[0] + from(ob[1], 1) + from(ob[2], 2);
+      D3 self = sub < 6 ? nb + ob[3] : d3(0.0, 0.0, 0.0);
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) {
+        self += d3(__shfl_xor_sync(0xffffffffu, self.x, o, 8),
+                   __shfl_xor_sync(0xffffffffu, self.y, o, 8),
+                   __shfl_xor_sync(0xffffffffu, self.z, o, 8));
+        g += __shfl_xor_sync(0xffffffffu, g, o, 8);
+      }
+      if (tri) {
+        if (sub < 6) {
+          put(1 + sub, nb, 0.0);
+          put(7 + sub, ob[3], 0.0);
+        }
+        if (sub == 0) put(0, d3(-self.x, -self.y, -self.z), g);
+        continue;
+      }
+    }
+    if (sub > 1) continue;
+    auto at = [&](int dj, int dk) {
       int32_t c = jj + dj, w = kk + dk;
       c += c < 0 ? NMX : 0;
       c -= c >= NMX ? NMX : 0;
       w += w < 0 ? NMY : 0;
       w -= w >= NMY ? NMY : 0;
-      return pb + w * NMX + c;
+      return offset(pb + w * NMX + c);
     };
-    const double4 p = S.pos_cur[i];
-    const D3 li = xyz(lam[i]);
-    double g_spring = 0.0, g_eps = 0.0, g_bend = 0.0;
-    // --- bending: forward recompute of the stencil, then its adjoint
-    const double sb = dt * T.P.kbend;
-    const D3 yb = sb * li;
-    if (T.lattice == kLatticeTriangular) {
-      const int32_t nm = T.nmemb;
-      D3 o[kTriSlots], ob[kTriSlots];
-      o[0] = d3(0.0, 0.0, 0.0);
-#pragma unroll
-      for (int k = 0; k < 6; ++k) {
-        const Vec3<double> v = offset_of<double>(S.pos_cur[pb + tri_link(j, k, NMX, nm)], p, T);
-        o[1 + k] = d3(v.x, v.y, v.z);
-        const int32_t c2 = tri_link(tri_link(j, (k + 1) % 6, NMX, nm), k, NMX, nm);
-        const Vec3<double> w = offset_of<double>(S.pos_cur[pb + c2], p, T);
-        o[7 + k] = d3(w.x, w.y, w.z);
-      }
-#pragma unroll
-      for (int s = 0; s < kTriSlots; ++s) ob[s] = d3(0.0, 0.0, 0.0);
-      for (int k = 0; k < 6; ++k) {
-        const int b = 1 + (k + 1) % 6;
-        g_bend += tri1_back(yb, o[1 + k], o[b], o[7 + k], ob[1 + k], ob[b], ob[7 + k]);
-      }
-      for (int k = 0; k < 6; ++k) {
-        const int b = 1 + (k + 1) % 6, c = 1 + (k + 2) % 6;
-        g_bend += tri2_back(yb, o[1 + k], o[b], o[c], ob[1 + k], ob[b], ob[c]);
-      }
-      D3 self = d3(0.0, 0.0, 0.0);
-#pragma unroll
-      for (int s = 1; s < kTriSlots; ++s) {
-        self -= ob[s];
-        bend[(int64_t)e * kBendStride + s] = make_double4(ob[s].x, ob[s].y, ob[s].z, 0.0);
-      }
-      bend[(int64_t)e * kBendStride] = make_double4(self.x, self.y, self.z, 0.0);
+    // the half's line of sites: next, after next, previous, before previous;
+    // the column half also the row two below
+    const bool col = sub == 1;
+    D3 o1 = at(col ? 0 : 1, col ? 1 : 0), o2 = at(col ? 0 : 2, col ? 2 : 0);
+    D3 o3 = at(col ? 0 : -1, col ? -1 : 0), o4 = at(col ? 0 : -2, col ? -2 : 0);
+    const D3 o0 = d3(0.0, 0.0, 0.0);
+    const U3 nv = unit3(o0, o1), nvr = unit3(o1, o2), nvl = unit3(o3, o0), nvll = unit3(o4, o3);
+    D3 b0 = o0, b1 = o0, b2 = o0, b3 = o0, b4 = o0, b9 = o0, b10 = o0;
+    HalfBar h;
+    double g;
+    if (!col) {
+      g = half_back(yb, nv.v, nvr.v, nvl.v, nvll.v, nv.inv, nvl.inv, dot(nvll.v, nvl.v), h);
+      h.m += h.w * nvl.v;  // w = nvll . nvl
+      h.l += h.w * nvll.v;
     } else {
-      D3 o[kSlots];
-      o[0] = d3(0.0, 0.0, 0.0);
-#pragma unroll
-      for (int s = 1; s < kSlots; ++s) {
-        const Vec3<double> v = offset_of<double>(S.pos_cur[site(kSlotDj[s], kSlotDk[s])], p, T);
-        o[s] = d3(v.x, v.y, v.z);
-      }
-      const U3 nv = unit3(o[0], o[1]), nvr = unit3(o[1], o[2]);
-      const U3 nvl = unit3(o[3], o[0]), nvll = unit3(o[4], o[3]);
-      const U3 mv = unit3(o[0], o[5]), mvu = unit3(o[5], o[6]);
-      const U3 mvb = unit3(o[7], o[0]), mvbb = unit3(o[8], o[7]);
-      const U3 nvbb = unit3(o[8], o[9]), nvbbr = unit3(o[9], o[10]);
-      HalfBar hn, hm;
-      const double ipnll = dot(nvll.v, nvl.v);
-      const double ipmbb = dot(nvbb.v, nvbbr.v);  // memb_bb's ipn (:380)
-      const double fn = half_back(yb, nv.v, nvr.v, nvl.v, nvll.v, nv.len, nvl.len, ipnll, hn);
-      const double fm = half_back(yb, mv.v, mvu.v, mvb.v, mvbb.v, mv.len, mvb.len, ipmbb, hm);
-      g_bend = fn + fm;  // lambda . (dt kbend BCALC): d/ds_bend of the bending term
-      D3 ob[kSlots];
-#pragma unroll
-      for (int s = 0; s < kSlots; ++s) ob[s] = d3(0.0, 0.0, 0.0);
-      // ipnll = nvll . nvl
-      hn.m += hn.w * nvl.v;
-      hn.l += hn.w * nvll.v;
-      unit3_back(nv, hn.n, hn.D, ob[0], ob[1]);
-      unit3_back(nvr, hn.a, 0.0, ob[1], ob[2]);
-      unit3_back(nvl, hn.l, hn.E, ob[3], ob[0]);
-      unit3_back(nvll, hn.m, 0.0, ob[4], ob[3]);
-      unit3_back(mv, hm.n, hm.D, ob[0], ob[5]);
-      unit3_back(mvu, hm.a, 0.0, ob[5], ob[6]);
-      unit3_back(mvb, hm.l, hm.E, ob[7], ob[0]);
-      unit3_back(mvbb, hm.m, 0.0, ob[8], ob[7]);
-      // ipmbb = nvbb . nvbbr
-      unit3_back(nvbb, hm.w * nvbbr.v, 0.0, ob[8], ob[9]);
-      unit3_back(nvbbr, hm.w * nvbb.v, 0.0, ob[9], ob[10]);
-      // o[s] = x_site - x_k: the particle itself receives minus every offset's
-      // adjoint (o[0] is the constant zero)
-      D3 self = d3(0.0, 0.0, 0.0);
-#pragma unroll
-      for (int s = 1; s < kSlots; ++s) {
-        self -= ob[s];
-        bend[(int64_t)e * kBendStride + s] = make_double4(ob[s].x, ob[s].y, ob[s].z, 0.0);
-      }
-      bend[(int64_t)e * kBendStride] = make_double4(self.x, self.y, self.z, 0.0);
+      const D3 o9 = at(1, -2), o10 = at(2, -2);
+      const U3 nvbb = unit3(o4, o9), nvbbr = unit3(o9, o10);
+      // w is memb_bb's ipn (:380)
+      g = half_back(yb, nv.v, nvr.v, nvl.v, nvll.v, nv.inv, nvl.inv, dot(nvbb.v, nvbbr.v), h);
+      unit3_back(nvbb, h.w * nvbbr.v, 0.0, b4, b9);
+      unit3_back(nvbbr, h.w * nvbb.v, 0.0, b9, b10);
     }
-    // --- lattice springs (each pair from both sides: gather)
-    D3 mu = d3(0.0, 0.0, 0.0);
-    for (int k = 0; k < T.nadj; ++k) {
-      const int32_t q = pb + lattice_link(T, j, k);
-      const double4 pq = S.pos_cur[q];
-      double dx, dy, dz;
-      pair_sep(p, pq, i > q, T, dx, dy, dz);
-      const D3 d = d3(dx, dy, dz);
-      const LawD w = memb_memb_d(L, dist_sq_exact(dx, dy, dz), p.w + pq.w);
-      const D3 dl = li - xyz(lam[q]);
-      mu += dt * (w.c * dl + (2.0 * w.dc_dr2 * dot(d, dl)) * d);
-      const double ld = dot(li, d);
-      g_spring += dt * w.c_spring * ld;
-      g_eps += dt * w.c_eps * ld;
+    unit3_back(nv, h.n, h.D, b0, b1);
+    unit3_back(nvr, h.a, 0.0, b1, b2);
+    unit3_back(nvl, h.l, h.E, b3, b0);
+    unit3_back(nvll, h.m, 0.0, b4, b3);
+    // offsets are x_site - x_k: the particle itself receives minus every
+    // offset's adjoint (o0 is the constant zero)
+    const D3 self = b1 + b2 + b3 + b4 + b9 + b10;
+    put(col ? kSelf2 : 0, d3(-self.x, -self.y, -self.z), g);
+    put(col ? 5 : 1, b1, 0.0);
+    put(col ? 6 : 2, b2, 0.0);
+    put(col ? 7 : 3, b3, 0.0);
+    put(col ? 8 : 4, b4, 0.0);
+    if (col) {
+      put(9, b9, 0.0);
+      put(10, b10, 0.0);
     }
-    // --- wall
-    if (p.z < p.w) wall_back(L, dt, p.z, p.w, li.z, mu, g_eps);
-    madj[e] = make_double4(mu.x, mu.y, mu.z, 0.0);
-    gmemb[e] = make_double4(g_spring, g_eps, g_bend, 0.0);
   }
 }
 
-// Every particle: pair adjoint over the exact connections at X_t, plus the
-// membrane terms, into lam_out; parameter partials into gpart.
-__global__ void __launch_bounds__(256) k_adj_pairs(DevState S, const double4* __restrict__ lam,
-                                                   double4* __restrict__ lam_out,
-                                                   const double4* __restrict__ bend,
-                                                   const double4* __restrict__ madj,
-                                                   const double4* __restrict__ gmemb,
-                                                   double4* __restrict__ gpart) {
+// Every particle: the pair adjoint over the exact connections at X_t, and for
+// membrane particles the lattice springs, the wall and the bending products
+// that name them, into lam_out; its parameter partials are added to gpart
+// (summed per tissue once, after the last step). kLanes lanes per particle
+// share candidates, springs and products and add up in a fixed tree, so a row
+// costs one or two evaluations in a row instead of ten: 36,864 particles 54 us
+// with one thread per particle, 23 with eight lanes. (What the previous kernel
+// of the chain wrote is read with ordinary loads, not through restricted
+// pointers: the two kernels' lifetimes overlap.)
+template <int kLanes>
+__global__ void __launch_bounds__(128) k_adj_pairs(DevState S, const double4* lam,
+                                                   double4* lam_out,
+                                                   const double4* bend,
+                                                   double4* gpart) {
+  pdl_entry();
   const int64_t N = S.n_total;
-  GRID_STRIDE(i, 0, N) {
-    const uint32_t a = S.attr[i];
-    const TissueDev& T = S.tissues[attr_tissue(a)];
-    const Laws<double>& L = T.lawd;
-    const double dt = T.P.dt;
-    const double lt2 = T.P.lj_thresh * T.P.lj_thresh;
-    const double4 p = S.pos_cur[i];
-    const D3 li = xyz(lam[i]);
-    D3 mu = li;
-    double g_spring = 0.0, g_eps = 0.0, g_bend = 0.0;
-    const uint32_t st = attr_state(a);
-    int32_t pair_i = -1, dermis_i = -1;
+  const int sub = (int)threadIdx.x & (kLanes - 1);
+  const int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) / kLanes;
+  const int64_t i = i0 < N ? i0 : N - 1;
+  const uint32_t a = S.attr[i];
+  const TissueDev& T = S.tissues[attr_tissue(a)];
+  const Laws<double>& L = T.lawd;
+  const double dt = T.P.dt;
+  const double lt2 = T.P.lj_thresh * T.P.lj_thresh;
+  const double4 p = S.pos_cur[i];
+  const D3 li = xyz(lam[i]);
+  D3 mu = d3(0.0, 0.0, 0.0);
+  double g_spring = 0.0, g_eps = 0.0, g_bend = 0.0;
+  const uint32_t st = attr_state(a);
+  int32_t pair_i = -1, dermis_i = -1;
+  if (st != ST_MEMB) {
+    pair_i = S.pair[i];
+    if (st == ST_FIX || st == ST_MUSUME) dermis_i = S.dermis[i];
+  }
+  auto add = [&](const LawD& w, const D3& d, int32_t q) {
+    const D3 dl = li - xyz(lam[q]);
+    mu += dt * (w.c * dl + (2.0 * w.dc_dr2 * dot(d, dl)) * d);
+    const double ld = dot(li, d);
+    g_spring += dt * w.c_spring * ld;
+    g_eps += dt * w.c_eps * ld;
+  };
+  const int32_t nc = cand_count(S, i);
+  for (int32_t k = sub; k < nc; k += kLanes) {
+    const int32_t q = T.pbase + (int32_t)cand_entry(S, i, k + 1);
+    const double4 pq = S.pos_cur[q];
+    const double dx = pdiff_h(p.x, pq.x, T.lx, T.hlx), dy = pdiff_h(p.y, pq.y, T.ly, T.hly);
+    const double dz = p.z - pq.z;
+    const double r2 = dist_sq_exact(dx, dy, dz);
+    const double rs = __dadd_rn(p.w, pq.w);
+    if (!(r2 <= __dmul_rn(__dmul_rn(lt2, rs), rs))) continue;  // connect_proc :115-119
+    const uint32_t aq = S.attr[q];
+    const uint32_t sq = attr_state(aq);
+    const bool both_old = attr_old(a) && attr_old(aq);
+    const Dist dd = dist_d(r2);
+    // the laws i applies while iterating q and q applies while iterating i
+    LawD w{0.0, 0.0, 0.0, 0.0};
     if (st != ST_MEMB) {
-      pair_i = S.pair[i];
-      if (st == ST_FIX || st == ST_MUSUME) dermis_i = S.dermis[i];
+      const int law = law_of(st, (int32_t)i, pair_i, dermis_i, sq, q);
+      if (law != L_NONE) w = w + law_d(law, L, dd, rs, both_old, attr_sfm(a));
     }
-    const int32_t nc = cand_count(S, i);
-    for (int32_t k = 0; k < nc; ++k) {
-      const int32_t q = T.pbase + (int32_t)cand_entry(S, i, k + 1);
-      const double4 pq = S.pos_cur[q];
-      const double dx = pdiff_h(p.x, pq.x, T.lx, T.hlx), dy = pdiff_h(p.y, pq.y, T.ly, T.hly);
-      const double dz = p.z - pq.z;
-      const double r2 = dist_sq_exact(dx, dy, dz);
-      const double rs = __dadd_rn(p.w, pq.w);
-      if (!(r2 <= __dmul_rn(__dmul_rn(lt2, rs), rs))) continue;  // connect_proc :115-119
-      const uint32_t aq = S.attr[q];
-      const uint32_t sq = attr_state(aq);
-      const bool both_old = attr_old(a) && attr_old(aq);
-      // the laws i applies while iterating q and q applies while iterating i
-      LawD w{0.0, 0.0, 0.0, 0.0};
-      if (st != ST_MEMB) {
-        const int law = law_of(st, (int32_t)i, pair_i, dermis_i, sq, q);
-        if (law != L_NONE) w = w + law_d(law, L, r2, rs, both_old, attr_sfm(a));
+    if (sq != ST_MEMB) {
+      int32_t pair_q = -1, dermis_q = -1;
+      if (sq == ST_FIX || sq == ST_MUSUME) {
+        pair_q = S.pair[q];
+        dermis_q = S.dermis[q];
       }
-      if (sq != ST_MEMB) {
-        int32_t pair_q = -1, dermis_q = -1;
-        if (sq == ST_FIX || sq == ST_MUSUME) {
-          pair_q = S.pair[q];
-          dermis_q = S.dermis[q];
-        }
-        const int law = law_of(sq, q, pair_q, dermis_q, st, (int32_t)i);
-        if (law != L_NONE) w = w + law_d(law, L, r2, rs, both_old, attr_sfm(aq));
-      }
-      const D3 d = d3(dx, dy, dz);
-      const D3 dl = li - xyz(lam[q]);
-      mu += dt * (w.c * dl + (2.0 * w.dc_dr2 * dot(d, dl)) * d);
-      const double ld = dot(li, d);
-      g_spring += dt * w.c_spring * ld;
-      g_eps += dt * w.c_eps * ld;
+      const int law = law_of(sq, q, pair_q, dermis_q, st, (int32_t)i);
+      if (law != L_NONE) w = w + law_d(law, L, dd, rs, both_old, attr_sfm(aq));
     }
-    // _pair_interaction (:637-641): the spring to the partner, from the
-    // higher index's rest length, in the separation of pair_sep
-    if (pair_i >= 0) {
-      const int32_t q = pair_i;
+    add(w, d3(dx, dy, dz), q);
+  }
+  // _pair_interaction (:637-641): the spring to the partner, from the
+  // higher index's rest length, in the separation of pair_sep
+  if (pair_i >= 0 && sub == 0) {
+    const int32_t q = pair_i;
+    const double4 pq = S.pos_cur[q];
+    double dx, dy, dz;
+    pair_sep(p, pq, i > q, T, dx, dy, dz);
+    add(pair_d(L, dist_d(dist_sq_exact(dx, dy, dz)), S.spr[i > q ? i : q]), d3(dx, dy, dz), q);
+  }
+  if ((st == ST_DER || st == ST_MEMB) && p.z < p.w && sub == kLanes - 1)
+    wall_back(L, dt, p.z, p.w, li.z, mu, g_eps);
+  if (st == ST_MEMB) {
+    const int32_t j = (int32_t)i - T.pbase;
+    const int32_t NMX = T.nmx, NMY = T.nmy, jj = j % NMX, kk = j / NMX;
+    const bool tri = T.lattice == kLatticeTriangular;
+    // lattice springs (each pair from both sides: gather)
+    for (int k = sub; k < T.nadj; k += kLanes) {
+      const int32_t q = T.pbase + lattice_link(T, j, k);
       const double4 pq = S.pos_cur[q];
       double dx, dy, dz;
       pair_sep(p, pq, i > q, T, dx, dy, dz);
-      const D3 d = d3(dx, dy, dz);
-      const LawD w = pair_d(L, dist_sq_exact(dx, dy, dz), S.spr[i > q ? i : q]);
-      const D3 dl = li - xyz(lam[q]);
-      mu += dt * (w.c * dl + (2.0 * w.dc_dr2 * dot(d, dl)) * d);
-      g_spring += dt * w.c_spring * dot(li, d);
+      add(memb_memb_d(L, dist_sq_exact(dx, dy, dz), p.w + pq.w), d3(dx, dy, dz), q);
     }
-    if (st == ST_DER && p.z < p.w) wall_back(L, dt, p.z, p.w, li.z, mu, g_eps);
-    if (st == ST_MEMB) {
-      const int32_t j = (int32_t)i - T.pbase;
-      const int32_t e = T.mbase + j;
-      const int32_t NMX = T.nmx, NMY = T.nmy, jj = j % NMX, kk = j / NMX;
-      mu += xyz(madj[e]);
-      const double4 gm = gmemb[e];
-      g_spring += gm.x;
-      g_eps += gm.y;
-      g_bend += gm.z;
-      if (T.lattice == kLatticeTriangular) {
-        // slot 1 + d names this site for its neighbour in the opposite
-        // direction (d + 3) % 6; slot 7 + k (the site two links away, along
-        // (k + 1) % 6 then k) for the particle reached back along the
-        // opposite directions, (k + 3) % 6 then (k + 4) % 6
-        const int32_t nm = T.nmemb;
-        mu += xyz(bend[(int64_t)(T.mbase + j) * kBendStride]);
-#pragma unroll
-        for (int d = 0; d < 6; ++d) {
-          const int32_t src = tri_link(j, (d + 3) % 6, NMX, nm);
-          mu += xyz(bend[(int64_t)(T.mbase + src) * kBendStride + 1 + d]);
+    // bending products naming this site. Square: slot s of the particle at
+    // (jj - dj_s, kk - dk_s), and the second self slot. Triangular: slot 1 + d
+    // names this site for its neighbour in the opposite direction (d + 3) %
+    // 6; slot 7 + k (the site two links away, along (k + 1) % 6 then k) for
+    // the particle reached back along the opposite directions, (k + 3) % 6
+    // then (k + 4) % 6.
+    const int ns = tri ? kTriSlots : kSlots + 1;
+    for (int s = sub; s < ns; s += kLanes) {
+      int32_t src = j;
+      if (tri) {
+        const TriSite s0{jj, kk};
+        if (s > 0) {
+          const TriSite t =
+              s < 7 ? tri_step(s0, (s + 2) % 6, NMX, NMY)
+                    : tri_step(tri_step(s0, (s - 4) % 6, NMX, NMY), (s - 3) % 6, NMX, NMY);
+          src = t.row * NMX + t.col;
         }
-#pragma unroll
-        for (int k = 0; k < 6; ++k) {
-          const int32_t src = tri_link(tri_link(j, (k + 3) % 6, NMX, nm), (k + 4) % 6, NMX, nm);
-          mu += xyz(bend[(int64_t)(T.mbase + src) * kBendStride + 7 + k]);
-        }
-      } else {
-        // bending products naming this site: slot s of the particle at
-        // (jj - dj_s, kk - dk_s)
-#pragma unroll
-        for (int s = 0; s < kSlots; ++s) {
-          int32_t c = jj - kSlotDj[s], w = kk - kSlotDk[s];
-          c += c < 0 ? NMX : 0;
-          c -= c >= NMX ? NMX : 0;
-          w += w < 0 ? NMY : 0;
-          w -= w >= NMY ? NMY : 0;
-          mu += xyz(bend[(int64_t)(T.mbase + w * NMX + c) * kBendStride + s]);
-        }
+      } else if (s < kSlots) {
+        int32_t c = jj - kSlotDj[s], w = kk - kSlotDk[s];
+        c += c < 0 ? NMX : 0;
+        c -= c >= NMX ? NMX : 0;
+        w += w < 0 ? NMY : 0;
+        w -= w >= NMY ? NMY : 0;
+        src = w * NMX + c;
       }
+      const double4 b = bend[(int64_t)(T.mbase + src) * kBendStride + s];
+      mu += xyz(b);
+      if (src == j && (s == 0 || s == kSelf2)) g_bend += b.w;
     }
-    lam_out[i] = make_double4(mu.x, mu.y, mu.z, 0.0);
-    gpart[i] = make_double4(g_spring, g_eps, g_bend, 0.0);
   }
+#pragma unroll
+  for (int o = kLanes / 2; o > 0; o >>= 1) {
+    mu += d3(__shfl_xor_sync(0xffffffffu, mu.x, o), __shfl_xor_sync(0xffffffffu, mu.y, o),
+             __shfl_xor_sync(0xffffffffu, mu.z, o));
+    g_spring += __shfl_xor_sync(0xffffffffu, g_spring, o);
+    g_eps += __shfl_xor_sync(0xffffffffu, g_eps, o);
+    g_bend += __shfl_xor_sync(0xffffffffu, g_bend, o);
+  }
+  if (sub != 0 || i0 >= N) return;
+  lam_out[i] = make_double4(li.x + mu.x, li.y + mu.y, li.z + mu.z, 0.0);
+  double4 g = gpart[i];
+  g.x += g_spring;
+  g.y += g_eps;
+  g.z += g_bend;
+  gpart[i] = g;
 }
 
 // lambda at the last step: dL/dX_T of L_t = inv_cnt[t] sum |X_T - X*|^2 over
@@ -662,7 +695,25 @@ __global__ void k_gate_check(DevState S) {
   }
 }
 
+// *moved = 1 when a particle of any of the m position sets in hist is beyond
+// the reach of the candidate rows (moved_too_far from their rebuild).
+__global__ void k_hist_check(DevState S, const double4* __restrict__ hist, int64_t m,
+                             int32_t* moved) {
+  GRID_STRIDE(e, 0, m * S.n_total) {
+    const int64_t i = e % S.n_total;
+    const double4 p = hist[e];
+    if (moved_too_far(S.skin, S.tissues[attr_tissue(S.attr[i])], p.x, p.y, p.z, S.bpos[i]))
+      *moved = 1;
+  }
+}
+
 }  // namespace
+
+void launch_hist_check(const DevState& S, const double4* hist, int32_t m, int32_t* moved,
+                       const LaunchCfg& lc, cudaStream_t s) {
+  if (S.n_total > 0 && m > 0)
+    k_hist_check<<<stride_blocks(S.n_total * m, lc.block, lc), lc.block, 0, s>>>(S, hist, m, moved);
+}
 
 void launch_gate_check(const DevState& S, const LaunchCfg& lc, cudaStream_t s) {
   if (S.n_total > 0)
@@ -677,14 +728,28 @@ void launch_adjoint_seed(const DevState& S, const double* target, int32_t cells_
         S, target, cells_only, inv_cnt, lam, gpart);
 }
 
-void launch_adjoint_step(const DevState& S, const AdjointBuffers& B, const LaunchCfg& lc,
+// Lanes per particle in k_adj_pairs: as many as keep a batch within a wave or
+// two of the blocks the GPU holds (36,864 particles, whole 200-step gradient:
+// 10.5 ms with four lanes, 11.3 with eight; 11,040 particles 8.9 and 8.6).
+constexpr int64_t kEightLanes = 16384, kFourLanes = 262144;
+
+template <int kLanes>
+void launch_adj_pairs(const DevState& S, const AdjointBuffers& B, cudaStream_t s) {
+  launch_pdl(k_adj_pairs<kLanes>, blocks_for(S.n_total * kLanes, 128), 128, s, S, B.lam_in,
+             B.lam_out, B.bend, B.gpart);
+}
+
+void launch_adjoint_step(const DevState& S, const AdjointBuffers& B, bool tri, const LaunchCfg& lc,
                          cudaStream_t s) {
-  if (S.nprep_memb > 0)
-    k_adj_memb<<<stride_blocks(S.nprep_memb, 256, lc), 256, 0, s>>>(S, B.lam_in, B.bend, B.madj,
-                                                                     B.gmemb);
-  if (S.n_total > 0)
-    k_adj_pairs<<<blocks_for(S.n_total, 256), 256, 0, s>>>(S, B.lam_in, B.lam_out, B.bend, B.madj,
-                                                           B.gmemb, B.gpart);
+  const int64_t nm = S.nprep_memb;
+  if (nm > 0 && tri)
+    launch_pdl(k_adj_bend<8>, stride_blocks(nm * 8, 64, lc), 64, s, S, B.lam_in, B.bend);
+  else if (nm > 0)
+    launch_pdl(k_adj_bend<2>, stride_blocks(nm * 2, 64, lc), 64, s, S, B.lam_in, B.bend);
+  if (S.n_total <= 0) return;
+  if (S.n_total <= kEightLanes) launch_adj_pairs<8>(S, B, s);
+  else if (S.n_total <= kFourLanes) launch_adj_pairs<4>(S, B, s);
+  else launch_adj_pairs<2>(S, B, s);
 }
 
 void launch_tissue_sum(const DevState& S, const double4* gpart, double* acc, const LaunchCfg& lc,

@@ -145,6 +145,8 @@ struct epi_ctx {
   unsigned long long* launches = nullptr;  // step-sequence kernels executed
   int32_t* res_sync = nullptr;   // grid barrier words of the resident kernel
   int coop = 0;                  // the device takes cooperative launches
+  unsigned char* adj_mem = nullptr;  // epi_adjoint's block (AdjointArena)
+  size_t adj_bytes = 0;
   ScanScratch scan{};
   // graphs: one per buffer parity, each replaying two steps
   cudaGraphExec_t graph[2] = {nullptr, nullptr};
@@ -223,6 +225,9 @@ void free_export(epi_ctx* c) {
 }
 
 void free_buffers(epi_ctx* c) {
+  if (c->adj_mem) cudaFree(c->adj_mem);
+  c->adj_mem = nullptr;
+  c->adj_bytes = 0;
   destroy_graphs(c);
   free_field(c);
   free_export(c);
@@ -729,6 +734,41 @@ struct ScopedDeviceMemory {
     return rc;
   }
 };
+
+// The adjoint's device memory: one block per context, kept between calls up
+// to kKeep bytes (and until the context's buffers go), handed out in pieces.
+class AdjointArena {
+ public:
+  explicit AdjointArena(epi_ctx* c) : c_(c) {}
+  ~AdjointArena() {
+    if (c_->adj_bytes > kKeep) release(c_);
+  }
+  int reserve(size_t bytes) {
+    if (c_->adj_bytes < bytes) {
+      release(c_);
+      const int rc = dev_alloc(&c_->adj_mem, bytes);
+      if (rc != EPI_OK) return rc;
+      c_->adj_bytes = bytes;
+    }
+    return EPI_OK;
+  }
+  template <typename T>
+  void take(T** p, size_t count) {
+    *p = reinterpret_cast<T*>(c_->adj_mem + used_);
+    used_ += (sizeof(T) * count + 255) & ~(size_t)255;
+  }
+  static void release(epi_ctx* c) {
+    if (c->adj_mem) cudaFree(c->adj_mem);
+    c->adj_mem = nullptr;
+    c->adj_bytes = 0;
+  }
+
+ private:
+  static constexpr size_t kKeep = (size_t)512 << 20;
+  epi_ctx* c_;
+  size_t used_ = 0;
+};
+
 }  // namespace
 
 extern "C" {
@@ -1156,16 +1196,29 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
   const int32_t nseg = (nsteps + K - 1) / K;
   const size_t hist_len = (size_t)std::max(1, std::min(K, nsteps));
   cudaStream_t s = c->stream;
-  ScopedDeviceMemory mem;
-  double4 *lam0, *lam1, *bend, *madj, *gmemb, *gpart, *ckpt, *hist, *xT;
+  // One block of device memory, kept for the next call while it is small: a
+  // dozen allocations and releases per call took milliseconds and varied.
+  double4 *lam0, *lam1, *bend, *gpart, *ckpt, *hist, *xT;
   double *acc, *target, *inv_cnt;
+  int32_t* moved;
   const size_t nm = (size_t)std::max(c->nprep_memb, 1);
-  if ((rc = mem.get(&lam0, n)) || (rc = mem.get(&lam1, n)) || (rc = mem.get(&gpart, n)) ||
-      (rc = mem.get(&bend, 13 * nm)) || (rc = mem.get(&madj, nm)) || (rc = mem.get(&gmemb, nm)) ||
-      (rc = mem.get(&ckpt, n * (size_t)std::max(nseg, 1))) || (rc = mem.get(&hist, n * hist_len)) ||
-      (rc = mem.get(&xT, n)) || (rc = mem.get(&acc, 4 * (size_t)nt)) ||
-      (rc = mem.get(&target, 3 * n)) || (rc = mem.get(&inv_cnt, (size_t)nt)))
+  AdjointArena mem(c);
+  if ((rc = mem.reserve(sizeof(double4) * (n * (4 + (size_t)std::max(nseg, 1) + hist_len) + 13 * nm) +
+                        sizeof(double) * (5 * (size_t)nt + 3 * n) + 16 * 256)))
     return rc;
+  mem.take(&lam0, n);
+  mem.take(&lam1, n);
+  mem.take(&gpart, n);
+  mem.take(&xT, n);
+  mem.take(&bend, 13 * nm);
+  mem.take(&ckpt, n * (size_t)std::max(nseg, 1));
+  mem.take(&hist, n * hist_len);
+  mem.take(&acc, 4 * (size_t)nt);
+  mem.take(&inv_cnt, (size_t)nt);
+  mem.take(&target, 3 * n);
+  mem.take(&moved, 1);
+  bool tri = false;
+  for (const TissueDev& T : c->tissues_h) tri |= T.lattice == kLatticeTriangular;
   const size_t pbytes = sizeof(double4) * n;
   EPI_CUDA(cudaMemcpyAsync(target, loss->target_x, 8 * n, cudaMemcpyHostToDevice, s));
   EPI_CUDA(cudaMemcpyAsync(target + n, loss->target_y, 8 * n, cudaMemcpyHostToDevice, s));
@@ -1178,47 +1231,75 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
   EPI_CUDA(cudaMemcpyAsync(inv_cnt, inv.data(), 8 * (size_t)nt, cudaMemcpyHostToDevice, s));
   EPI_CUDA(cudaMemsetAsync(acc, 0, 32 * (size_t)nt, s));
   // forward, keeping a checkpoint every K steps
-  for (int32_t t = 0; t < nsteps; ++t) {
-    if (t % K == 0)
-      EPI_CUDA(cudaMemcpyAsync(ckpt + (size_t)(t / K) * n, c->pos[c->cur], pbytes,
-                               cudaMemcpyDeviceToDevice, s));
-    enqueue_step(c, c->cur, nullptr);
+  for (int32_t t = 0; t < nsteps; t += K) {
+    EPI_CUDA(cudaMemcpyAsync(ckpt + (size_t)(t / K) * n, c->pos[c->cur], pbytes,
+                             cudaMemcpyDeviceToDevice, s));
+    if ((rc = enqueue_steps(c, std::min(K, nsteps - t)))) return rc;
   }
   c->lists_fresh = false;
   if ((rc = check_status(c))) return rc;
   EPI_CUDA(cudaMemcpyAsync(xT, c->pos[c->cur], pbytes, cudaMemcpyDeviceToDevice, s));
   launch_adjoint_seed(make_state(c, c->cur), target, loss->cells_only, inv_cnt, lam0,
                       gpart, c->lc, s);
-  launch_tissue_sum(make_state(c, c->cur), gpart, acc, c->lc, s);
   double4* lam[2] = {lam0, lam1};
   int a = 0;
+  ResidentPlan plan;
+  const bool small = resident(c, &plan);
   for (int32_t seg = nseg - 1; seg >= 0; --seg) {
-    const int32_t t0 = seg * K, t1 = std::min(t0 + K, nsteps);
-    // recompute X_t0 .. X_{t1-1} from the checkpoint
-    EPI_CUDA(cudaMemcpyAsync(c->pos[c->cur], ckpt + (size_t)seg * n, pbytes,
-                             cudaMemcpyDeviceToDevice, s));
-    c->posf_stale = true;
-    launch_gate_check(make_state(c, c->cur), c->lc, s);
-    for (int32_t t = t0; t < t1; ++t) {
-      EPI_CUDA(cudaMemcpyAsync(hist + (size_t)(t - t0) * n, c->pos[c->cur], pbytes,
+    const int32_t t0 = seg * K, t1 = std::min(t0 + K, nsteps), len = t1 - t0;
+    // recompute X_t0 .. X_{t1-1} from the checkpoint into hist
+    if (small) {
+      EPI_CUDA(cudaMemcpyAsync(hist, ckpt + (size_t)seg * n, pbytes, cudaMemcpyDeviceToDevice, s));
+      DevState Sh = make_state(c, c->cur);
+      Sh.pos_cur = hist;
+      launch_gate_check(Sh, c->lc, s);
+      if (len > 1) {
+        if (c->cfg.precision == EPI_PREC_MIXED) launch_posf(Sh, c->lc, s);
+        ResidentCfg rcfg{};
+        rcfg.sync = c->res_sync;
+        rcfg.hist = hist;
+        EPI_CUDA(launch_resident(Sh, plan, c->tissues_h[0], len - 1, c->cfg.precision, rcfg, c->lc, s));
+      }
+    } else {
+      EPI_CUDA(cudaMemcpyAsync(c->pos[c->cur], ckpt + (size_t)seg * n, pbytes,
                                cudaMemcpyDeviceToDevice, s));
-      if (t + 1 < t1) enqueue_step(c, c->cur, nullptr);
+      c->posf_stale = true;
+      launch_gate_check(make_state(c, c->cur), c->lc, s);
+      for (int32_t t = 0; t < len; ++t) {
+        EPI_CUDA(cudaMemcpyAsync(hist + (size_t)t * n, c->pos[c->cur], pbytes,
+                                 cudaMemcpyDeviceToDevice, s));
+        if (t + 1 < len) enqueue_step(c, c->cur, nullptr);
+      }
     }
+    // Candidates built at the middle of the segment mostly reach its ends, so
+    // one check stands for a check and the rebuild's kernels at every step.
+    DevState Sm = make_state(c, c->cur);
+    Sm.pos_cur = hist + (size_t)(len / 2) * n;
+    launch_set_gates(Sm, nt, s);
+    launch_rebuild(Sm, whole(c), c->scan, c->lc, s, nullptr);
+    int32_t far = 0;
+    EPI_CUDA(cudaMemsetAsync(moved, 0, sizeof(int32_t), s));
+    launch_hist_check(Sm, hist, len, moved, c->lc, s);
+    EPI_CUDA(cudaMemcpyAsync(&far, moved, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
+    if ((rc = check_status(c))) return rc;
     // and differentiate them in reverse
-    for (int32_t t = t1 - 1; t >= t0; --t) {
+    for (int32_t t = len - 1; t >= 0; --t) {
       DevState St = make_state(c, c->cur);
-      St.pos_cur = hist + (size_t)(t - t0) * n;
-      launch_gate_check(St, c->lc, s);
-      launch_rebuild(St, whole(c), c->scan, c->lc, s, nullptr);
+      St.pos_cur = hist + (size_t)t * n;
+      if (far) {
+        launch_gate_check(St, c->lc, s);
+        launch_rebuild(St, whole(c), c->scan, c->lc, s, nullptr);
+      }
       // the dermis of FIX / MUSUME cells at X_t selects their membrane law
       launch_dermis(St, c->nprep_memb, c->nprep, c->lc, s, nullptr);
-      const AdjointBuffers B{lam[a], lam[a ^ 1], bend, madj, gmemb, gpart};
-      launch_adjoint_step(St, B, c->lc, s);
-      launch_tissue_sum(St, gpart, acc, c->lc, s);
+      const AdjointBuffers B{lam[a], lam[a ^ 1], bend, gpart};
+      launch_adjoint_step(St, B, tri, c->lc, s);
       a ^= 1;
     }
     if ((rc = check_status(c))) return rc;
   }
+  // the parameter partials and loss terms of all steps, per tissue
+  launch_tissue_sum(make_state(c, c->cur), gpart, acc, c->lc, s);
   // the context ends at X_T; its candidates are rebuilt before the next step
   EPI_CUDA(cudaMemcpyAsync(c->pos[c->cur], xT, pbytes, cudaMemcpyDeviceToDevice, s));
   c->posf_stale = true;

@@ -150,10 +150,12 @@ struct AdjointBuffers {
   const double4* lam_in;  // dL/dX_{t+1}
   double4* lam_out;       // dL/dX_t
   double4* bend;          // 13 bending-product slots per membrane particle
-  double4* madj;          // lattice + wall product per membrane particle
-  double4* gmemb;         // membrane parameter partials
   double4* gpart;         // per-particle parameter partials (spring, eps, bend, loss)
 };
+// *moved = 1 when the candidate rows do not reach far enough for one of the m
+// position sets in hist.
+void launch_hist_check(const DevState& S, const double4* hist, int32_t m, int32_t* moved,
+                       const LaunchCfg& lc, cudaStream_t s);
 // Sets the gate of every tissue with a particle farther than skin/2 from
 // its last rebuild position.
 void launch_gate_check(const DevState& S, const LaunchCfg& lc, cudaStream_t s);
@@ -164,7 +166,9 @@ void launch_adjoint_seed(const DevState& S, const double* target, int32_t cells_
                          const LaunchCfg& lc, cudaStream_t s);
 // One backward step at positions S.pos_cur (lists: exact predicate over the
 // current candidates, which must be valid for S.pos_cur).
-void launch_adjoint_step(const DevState& S, const AdjointBuffers& B, const LaunchCfg& lc,
+// Adds the step's parameter partials to B.gpart. tri: some tissue's membrane
+// is triangular.
+void launch_adjoint_step(const DevState& S, const AdjointBuffers& B, bool tri, const LaunchCfg& lc,
                          cudaStream_t s);
 // acc[4 t + c] += per-tissue sums of gpart (fixed order: deterministic).
 void launch_tissue_sum(const DevState& S, const double4* gpart, double* acc, const LaunchCfg& lc,
