@@ -144,6 +144,7 @@ struct epi_ctx {
   int32_t* loop_left = nullptr;  // passes left in the step graph's device loop
   unsigned long long* launches = nullptr;  // step-sequence kernels executed
   int32_t* res_sync = nullptr;   // grid barrier words of the resident kernel
+  uint32_t res_run = 0;          // its runs so far (which barrier word is next)
   int coop = 0;                  // the device takes cooperative launches
   unsigned char* adj_mem = nullptr;  // epi_adjoint's block (AdjointArena)
   size_t adj_bytes = 0;
@@ -162,7 +163,6 @@ struct epi_ctx {
   double* ext[2] = {nullptr, nullptr};
   int ext_cur = 0;
   double* zzmax = nullptr;
-  int32_t* izb = nullptr;
   // export buffers of epi_get_connections / epi_get_dermis, kept between
   // calls (the drop-in exports every step) and grown on demand
   int32_t* x_rowlen = nullptr;   // n
@@ -205,11 +205,11 @@ void destroy_graphs(epi_ctx* c) {
 }
 
 void free_field(epi_ctx* c) {
-  void* ptrs[] = {c->fd, c->cmap1, c->cmap2, c->ext[0], c->ext[1], c->zzmax, c->izb};
+  void* ptrs[] = {c->fd, c->cmap1, c->cmap2, c->ext[0], c->ext[1], c->zzmax};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   c->fd = nullptr; c->cmap1 = nullptr; c->cmap2 = nullptr;
-  c->ext[0] = c->ext[1] = nullptr; c->zzmax = nullptr; c->izb = nullptr;
+  c->ext[0] = c->ext[1] = nullptr; c->zzmax = nullptr;
   c->field_on = false;
   c->nvox = 0;
   c->fd_h.clear();
@@ -385,6 +385,7 @@ int enqueue_resident(epi_ctx* c, const ResidentPlan& P, int32_t nsteps, bool gra
   ensure_posf(c);
   ResidentCfg rc{};
   rc.sync = c->res_sync;
+  c->status_h->flags = 0;
   const int own = (c->nprep_memb > 0 ? 1 : 0) + (c->nprep > c->nprep_memb ? 1 : 0) + 1;
   const bool skips = graph && conditional_rebuild(c);
   rc.per_step = own + (skips ? 1 : 6);
@@ -393,6 +394,8 @@ int enqueue_resident(epi_ctx* c, const ResidentPlan& P, int32_t nsteps, bool gra
   // bounded runs: a kernel of a thousand steps lasts a few milliseconds
   for (int32_t done = 0; done < nsteps;) {
     const int32_t k = std::min(nsteps - done, 1024);
+    rc.run = c->res_run++;
+    rc.post = done + k == nsteps ? c->status_h : nullptr;
     EPI_CUDA(launch_resident(make_state(c, c->cur), P, c->tissues_h[0], k, c->cfg.precision, rc,
                              c->lc, c->stream));
     c->cur ^= k & 1;
@@ -524,14 +527,21 @@ void enqueue_materialize(epi_ctx* c) {
 }
 
 // Waits for the stream and converts any sticky kernel error to a status.
-int check_status(epi_ctx* c) {
-  EPI_CUDA(cudaMemcpyAsync(c->status_h, c->status, sizeof(DevStatus), cudaMemcpyDeviceToHost,
-                           c->stream));
-  EPI_CUDA(cudaStreamSynchronize(c->stream));
+// posted: the last work queued was a resident run, which puts the status into
+// host memory itself (one whose barrier gave up does not).
+int check_status(epi_ctx* c, bool posted = false) {
+  if (posted) EPI_CUDA(cudaStreamSynchronize(c->stream));
+  if (!posted || !(((volatile DevStatus*)c->status_h)->flags & kStatusPosted)) {
+    EPI_CUDA(cudaMemcpyAsync(c->status_h, c->status, sizeof(DevStatus), cudaMemcpyDeviceToHost,
+                             c->stream));
+    EPI_CUDA(cudaStreamSynchronize(c->stream));
+  }
   EPI_CUDA(cudaGetLastError());
   if (c->status_h->code != 0) {
     c->last = *c->status_h;
+    c->last.flags &= ~kStatusPosted;
     EPI_CUDA(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
+    EPI_CUDA(cudaMemsetAsync(c->res_sync, 0, 4 * sizeof(int32_t), c->stream));
     EPI_CUDA(cudaStreamSynchronize(c->stream));
     return c->last.code;
   }
@@ -541,10 +551,12 @@ int check_status(epi_ctx* c) {
 // nsteps steps replayed from the two-step graph of the current parity
 // (both parities' graphs captured on first use), plus one eager step for
 // an odd count.
-int enqueue_graph_steps(epi_ctx* c, int32_t nsteps) {
+// *posted: see check_status.
+int enqueue_graph_steps(epi_ctx* c, int32_t nsteps, bool* posted = nullptr) {
   ResidentPlan P;
   if (nsteps > 0 && resident(c, &P)) {
     c->lists_fresh = false;
+    if (posted) *posted = true;
     return enqueue_resident(c, P, nsteps, true);
   }
   ensure_posf(c);  // never inside the captured graph
@@ -565,10 +577,13 @@ int enqueue_graph_steps(epi_ctx* c, int32_t nsteps) {
 }
 
 // nsteps steps without a graph.
-int enqueue_steps(epi_ctx* c, int32_t nsteps) {
+int enqueue_steps(epi_ctx* c, int32_t nsteps, bool* posted = nullptr) {
   if (nsteps > 0) c->lists_fresh = false;
   ResidentPlan P;
-  if (nsteps > 0 && resident(c, &P)) return enqueue_resident(c, P, nsteps, false);
+  if (nsteps > 0 && resident(c, &P)) {
+    if (posted) *posted = true;
+    return enqueue_resident(c, P, nsteps, false);
+  }
   for (int32_t k = 0; k < nsteps; ++k) enqueue_step(c, c->cur, nullptr);
   return EPI_OK;
 }
@@ -874,7 +889,8 @@ int epi_create(epi_ctx** out, const epi_config* cfg) {
   if (rc == EPI_OK) rc = dev_alloc(&ctx->rebuilds, 1);
   if (rc == EPI_OK) rc = dev_alloc(&ctx->loop_left, 1);
   if (rc == EPI_OK) rc = dev_alloc(&ctx->launches, 1);
-  if (rc == EPI_OK) rc = dev_alloc(&ctx->res_sync, 2);
+  if (rc == EPI_OK) rc = dev_alloc(&ctx->res_sync, 4);
+  if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->res_sync, 0, 4 * sizeof(int32_t)));
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->launches, 0, sizeof(unsigned long long)));
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->rebuilds, 0, sizeof(unsigned long long)));
   if (rc != EPI_OK) {
@@ -956,9 +972,9 @@ int epi_upload(epi_ctx* c, int32_t ntissues, const epi_tissue_view* tv, const ep
   const bool keep_field = c->field_on && c->ntissues == ntissues;
   if (keep_field && !reuse) {
     kept.fd = c->fd; kept.cmap1 = c->cmap1; kept.cmap2 = c->cmap2;
-    kept.ext[0] = c->ext[0]; kept.ext[1] = c->ext[1]; kept.zzmax = c->zzmax; kept.izb = c->izb;
+    kept.ext[0] = c->ext[0]; kept.ext[1] = c->ext[1]; kept.zzmax = c->zzmax;
     c->fd = nullptr; c->cmap1 = nullptr; c->cmap2 = nullptr;
-    c->ext[0] = c->ext[1] = nullptr; c->zzmax = nullptr; c->izb = nullptr;
+    c->ext[0] = c->ext[1] = nullptr; c->zzmax = nullptr;
   } else if (!keep_field) {
     free_field(c);
   }
@@ -969,9 +985,9 @@ int epi_upload(epi_ctx* c, int32_t ntissues, const epi_tissue_view* tv, const ep
   c->lists_fresh = false;
   if (keep_field && !reuse) {
     c->fd = kept.fd; c->cmap1 = kept.cmap1; c->cmap2 = kept.cmap2;
-    c->ext[0] = kept.ext[0]; c->ext[1] = kept.ext[1]; c->zzmax = kept.zzmax; c->izb = kept.izb;
+    c->ext[0] = kept.ext[0]; c->ext[1] = kept.ext[1]; c->zzmax = kept.zzmax;
     kept.fd = nullptr; kept.cmap1 = nullptr; kept.cmap2 = nullptr;
-    kept.ext[0] = kept.ext[1] = nullptr; kept.zzmax = nullptr; kept.izb = nullptr;
+    kept.ext[0] = kept.ext[1] = nullptr; kept.zzmax = nullptr;
     c->field_on = true;
     c->fnx = fnx; c->fny = fny; c->fnz = fnz; c->ext_cur = fcur; c->nvox = fnvox;
     c->fd_h = ffd;
@@ -1257,6 +1273,7 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
         if (c->cfg.precision == EPI_PREC_MIXED) launch_posf(Sh, c->lc, s);
         ResidentCfg rcfg{};
         rcfg.sync = c->res_sync;
+        rcfg.run = c->res_run++;
         rcfg.hist = hist;
         EPI_CUDA(launch_resident(Sh, plan, c->tissues_h[0], len - 1, c->cfg.precision, rcfg, c->lc, s));
       }
@@ -1341,8 +1358,7 @@ int epi_field_init(epi_ctx* c, int32_t nx, int32_t ny, int32_t nz) {
   c->nvox = per * nt;
   if ((rc = dev_alloc(&c->fd, nt)) || (rc = dev_alloc(&c->cmap1, c->nvox)) ||
       (rc = dev_alloc(&c->cmap2, c->nvox)) || (rc = dev_alloc(&c->ext[0], c->nvox)) ||
-      (rc = dev_alloc(&c->ext[1], c->nvox)) || (rc = dev_alloc(&c->zzmax, nt)) ||
-      (rc = dev_alloc(&c->izb, nt))) {
+      (rc = dev_alloc(&c->ext[1], c->nvox)) || (rc = dev_alloc(&c->zzmax, nt))) {
     free_field(c);
     return rc;
   }
@@ -1357,7 +1373,6 @@ int epi_field_init(epi_ctx* c, int32_t nx, int32_t ny, int32_t nz) {
   EPI_CUDA(cudaMemsetAsync(c->cmap1, 0, sizeof(int32_t) * c->nvox, s));
   EPI_CUDA(cudaMemsetAsync(c->cmap2, 0, c->nvox, s));
   EPI_CUDA(cudaMemsetAsync(c->zzmax, 0, sizeof(double) * nt, s));
-  EPI_CUDA(cudaMemsetAsync(c->izb, 0, sizeof(int32_t) * nt, s));
   return check_status(c);
   EPI_GUARD_END
 }
@@ -1377,12 +1392,9 @@ int epi_field_step(epi_ctx* c, int32_t nsteps) {
     FS.cur = c->ext[c->ext_cur];
     FS.nxt = c->ext[c->ext_cur ^ 1];
     FS.zzmax = c->zzmax;
-    FS.izb = c->izb;
     FS.nvox = c->nvox;
     FS.agek = c->agek;
-    int32_t wmax = 1;
-    for (const FieldDev& F : c->fd_h) wmax = std::max(wmax, 4 * std::max(F.irx, F.iry) + 1);
-    launch_field_step(make_state(c, c->cur), FS, wmax, c->lc, c->stream);
+    launch_field_step(make_state(c, c->cur), FS, c->lc, c->stream);
     c->ext_cur ^= 1;  // ext_stim.swap()
   }
   return check_status(c);
@@ -1451,8 +1463,9 @@ int epi_interact_commit(epi_ctx* c) {
   Nvtx nvtx_range("epi_interact_commit");
   int rc = set_device(c);
   if (rc) return rc;
-  if ((rc = enqueue_steps(c, 1))) return rc;
-  return check_status(c);
+  bool posted = false;
+  if ((rc = enqueue_steps(c, 1, &posted))) return rc;
+  return check_status(c, posted);
   EPI_GUARD_END
 }
 
@@ -1463,8 +1476,9 @@ int epi_step(epi_ctx* c, int32_t nsteps) {
   Nvtx nvtx_range("epi_step");
   int rc = set_device(c);
   if (rc) return rc;
-  if ((rc = enqueue_steps(c, nsteps))) return rc;
-  return check_status(c);
+  bool posted = false;
+  if ((rc = enqueue_steps(c, nsteps, &posted))) return rc;
+  return check_status(c, posted);
   EPI_GUARD_END
 }
 
@@ -1475,8 +1489,9 @@ int epi_step_graph(epi_ctx* c, int32_t nsteps) {
   Nvtx nvtx_range("epi_step_graph");
   int rc = set_device(c);
   if (rc) return rc;
-  if ((rc = enqueue_graph_steps(c, nsteps))) return rc;
-  return check_status(c);
+  bool posted = false;
+  if ((rc = enqueue_graph_steps(c, nsteps, &posted))) return rc;
+  return check_status(c, posted);
   EPI_GUARD_END
 }
 

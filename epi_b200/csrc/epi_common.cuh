@@ -72,6 +72,8 @@ struct DevStatus {
   double v;       // offending value
 };
 
+constexpr int32_t kStatusPosted = 1 << 30;  // among flags: put there by a kernel
+
 struct DevState {
   const TissueDev* tissues;
   double4* pos_cur;

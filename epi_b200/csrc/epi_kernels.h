@@ -69,7 +69,10 @@ void launch_step(const DevState& S, const Range& r, int precision, const LaunchC
 // The same for nsteps steps of a small batch in one cooperative kernel
 // (epi_resident.cu), candidate rebuilds included.
 struct ResidentCfg {
-  int32_t* sync;      // two device words: the barrier's count and its abort flag
+  int32_t* sync;      // device words: two barrier counts, used by runs in turn
+  uint32_t run;       // (each run clears the next one's), and the abort flag
+  DevStatus* post;    // pinned host memory the status goes to at the end, with
+                      // kStatusPosted among the flags; or null
   int32_t per_step, per_pair, per_rebuild;  // kernels of the sequence each step, each
                       // second step and each rebuilding step stands for
   double4* hist;      // null: S's two position buffers in turn; else step k reads
@@ -133,7 +136,6 @@ struct FieldState {
   const double* cur;   // external stimulus, current
   double* nxt;         // external stimulus, next
   double* zzmax;       // per tissue
-  int32_t* izb;        // per tissue: grid planes below the diffusion's z bound
   int64_t nvox;        // grid points over all tissues
   const double* agek;  // per particle
 };
@@ -141,9 +143,8 @@ struct FieldState {
 void field_params(FieldDev& F, double lx, double ly, double lz, int32_t nx, int32_t ny,
                   int32_t nz);
 // zzmax, cell maps, external-stimulus update into FS.nxt (the caller swaps).
-// wmax: the widest stamp window over the batch's tissues, 2 (2 irx) + 1.
-void launch_field_step(const DevState& S, const FieldState& FS, int32_t wmax,
-                       const LaunchCfg& lc, cudaStream_t s);
+void launch_field_step(const DevState& S, const FieldState& FS, const LaunchCfg& lc,
+                       cudaStream_t s);
 
 // ---- reverse-mode adjoint (FP64), membrane + ALIVE / DEAD / AIR tissues ----
 struct AdjointBuffers {

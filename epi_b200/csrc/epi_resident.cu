@@ -47,7 +47,9 @@ struct ResidentArgs {
   int32_t dealt;            // tiles of particles are dealt round the blocks
   int32_t thread_from;      // candidate search: a thread per particle from here on
   unsigned* bar;            // barrier arrivals (zero at launch)
-  int32_t* abort;           // set when a barrier wait gave up (zero at launch)
+  unsigned* other;          // the next run's (zeroed here)
+  int32_t* abort;           // set when a barrier wait gave up
+  DevStatus* post;          // non-null: pinned host memory the status is put in
   int32_t per_step, per_pair, per_rebuild;  // launches counted (see epi_launch_count)
   double4* hist;            // non-null: step k's positions go to hist + k n_total
 };
@@ -254,6 +256,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   // once: the slots' attributes, positions and membrane list, and the
   // constants of the block's first tissues
   if (tid == 0) {
+    if (blockIdx.x == 0) *A.other = 0u;
     s_nm = 0;
     s_t0 = !A.dealt && particle(0) < n ? (int32_t)attr_tissue(S0.attr[particle(0)]) : 0;
   }
@@ -290,6 +293,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   // slots [c0, c1) hold the pair tasks listed in K.task
   int c0 = 0, c1 = 0;
   bool fresh = true;  // rows and rebuild positions are to be read
+  bool done = false;
   for (int32_t step = 0; step < A.nsteps; ++step) {
     counted += A.per_step + ((step & 1) ? A.per_pair : 0);
     if (flagged) {
@@ -492,8 +496,23 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
     S.posf_cur = S.posf_nxt;
     S.posf_nxt = tf;
     if (!B.sync(S0.gate, &flagged)) break;
+    done = step + 1 == A.nsteps;
   }
-  if (blockIdx.x == 0 && tid == 0 && S0.launches) atomicAdd(S0.launches, counted);
+  if (blockIdx.x == 0 && tid == 0) {
+    if (S0.launches) atomicAdd(S0.launches, counted);
+    // past the last barrier every block has raised what it had to: the host
+    // finds the status after its wait for the stream, without a copy
+    if (A.post && done) {
+      const volatile DevStatus* from = S0.status;
+      volatile DevStatus* to = A.post;
+      to->code = from->code;
+      to->a = from->a;
+      to->b = from->b;
+      to->v = from->v;
+      to->flags = from->flags | kStatusPosted;
+      __threadfence_system();
+    }
+  }
 }
 
 // Kernel of a batch's form.
@@ -566,13 +585,14 @@ cudaError_t launch_resident(const DevState& S, const ResidentPlan& P, const Tiss
   A.terms = P.terms;
   A.dealt = P.dealt;
   A.thread_from = lc.search_switch;
-  A.bar = reinterpret_cast<unsigned*>(rc.sync);
-  A.abort = rc.sync + 1;
+  A.bar = reinterpret_cast<unsigned*>(rc.sync) + (rc.run & 1);
+  A.other = reinterpret_cast<unsigned*>(rc.sync) + (~rc.run & 1);
+  A.abort = rc.sync + 2;
+  A.post = rc.post;
   A.per_step = rc.per_step;
   A.per_pair = rc.per_pair;
   A.per_rebuild = rc.per_rebuild;
   A.hist = rc.hist;
-  if ((e = cudaMemsetAsync(rc.sync, 0, 2 * sizeof(int32_t), s)) != cudaSuccess) return e;
   DevState S1 = S;
   TissueDev T0 = first;
   void* args[] = {&S1, &A, &T0};
