@@ -263,14 +263,19 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   __syncthreads();
   for (int s = tid; s < slots; s += NT) {
     const int32_t i = particle(s);
+    K.off[s] = 0;
     if (i >= n) continue;
     const uint32_t a = S0.attr[i];
     const double4 p = S.pos_cur[i];
+    const int32_t nc = cand_count(S, i);
+    const float4 b = S.bpos[i];
     K.attr[s] = a;
     K.pos[s] = p;
+    K.off[s] = nc;
+    K.bpos[s] = b;
     if constexpr (Slots<R>::kOwn) K.own[s] = Part::own(p);
     if (attr_state(a) == ST_MEMB) {
-      const TissueDev& T = S0.tissues[attr_tissue(a)];
+      const TissueDev& T = kOne ? T0 : S0.tissues[attr_tissue(a)];
       const int32_t j = i - T.pbase, at = atomicAdd(&s_nm, 1);
       K.list[at] = s;
       K.jk[at] = j % T.nmx | (j / T.nmx) << 16;
@@ -292,25 +297,31 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   };
   // slots [c0, c1) hold the pair tasks listed in K.task
   int c0 = 0, c1 = 0;
-  bool fresh = true;  // rows and rebuild positions are to be read
+  bool fresh = true, rebuilt = false;  // rows are to be listed, to be read first
   bool done = false;
   for (int32_t step = 0; step < A.nsteps; ++step) {
     counted += A.per_step + ((step & 1) ? A.per_pair : 0);
     if (flagged) {
       counted += A.per_rebuild;
       if (!resident_rebuild<NT>(S0, S.pos_cur, A.thread_from, B)) break;
-      fresh = true;
+      fresh = rebuilt = true;
     }
     if (fresh) {
       fresh = false;
+      // first task of each slot, from the row lengths (in K.off after the
+      // set-up, read again after a rebuild)
       int32_t carry = 0;
       for (int base = 0; base < slots; base += NT) {
         const int s = base + tid;
-        const int32_t i = s < slots ? particle(s) : n;
         int32_t nc = 0;
-        if (i < n) {
-          nc = cand_count(S, i);
-          K.bpos[s] = S.bpos[i];
+        if (s < slots) {
+          const int32_t i = particle(s);
+          if (!rebuilt) {
+            nc = K.off[s];  // written by this thread
+          } else if (i < n) {
+            nc = cand_count(S, i);
+            K.bpos[s] = S.bpos[i];
+          }
         }
         int32_t total;
         const int32_t before = block_excl_scan_n<NT>(nc, &total);
@@ -510,7 +521,6 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
       to->b = from->b;
       to->v = from->v;
       to->flags = from->flags | kStatusPosted;
-      __threadfence_system();
     }
   }
 }
