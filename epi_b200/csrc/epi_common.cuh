@@ -287,7 +287,7 @@ template <typename R>
 struct Laws {
   R eps4, p_memb, der_der_const, k_total, k_desmosome, kspring, kspring_d, delta_r, para_ljp2,
       kspring_division, lj_thresh, ljt1sq;
-  R ljt1;        // LJ_THRESH - 1
+  R ljt1;        // largest m with 1 + m, rounded, not above lj_thresh
   R inv_ljt1sq;  // 1 / (LJ_THRESH - 1)^2
   R memb_far;    // der_der_const (1 - p_memb) / p_memb
   static constexpr bool kF32 = sizeof(R) == 4;
@@ -354,16 +354,15 @@ struct Laws {
   // The same law in FP32 without a branch: both sides from one reciprocal
   // square root, then a select, so lanes of a warp on either side of
   // is_near do not run both paths one after the other. Two MUFU operations
-  // in all (the reciprocal of rs is the other).
-  __device__ __forceinline__ float aad_fused(float d2, float rs, bool both_old) const {
+  // in all (the reciprocal of rs is the other). inv: 1 / ljt1sq (rcp_approx).
+  __device__ __forceinline__ float aad_fused(float d2, float rs, bool both_old, float inv) const {
     const float inv_d = rsqrtf(d2);
     const float inv_d2 = xmul(inv_d, inv_d);
     const float r2 = xmul(rs, rs);
-    const float u = pow3(xmul(r2, inv_d2));
-    const float c_lj = xmul(xfma(u, u, -u), xmul(eps4, inv_d2));
+    const float c_lj = xmul(lj_factor(pow3(xmul(r2, inv_d2))), inv_d2);
     const float m1 = xfma(xmul(d2, inv_d), rcp_approx(rs), -1.f);
     const float k = both_old ? k_total : k_desmosome;
-    const float h = xfma(-xmul(m1, m1), inv_ljt1sq, 1.f);
+    const float h = xfma(-xmul(m1, m1), inv, 1.f);
     const float c_ad = m1 > ljt1 ? 0.f : xmul(xmul(xmul(-k, inv_d), m1), h);
     return d2 < r2 ? c_lj : c_ad;
   }
@@ -455,6 +454,14 @@ __host__ __device__ inline Laws<R> make_laws(const Params& P) {
   L.lj_thresh = R(P.lj_thresh);
   L.ljt1sq = R((P.lj_thresh - 1.0) * (P.lj_thresh - 1.0));
   L.ljt1 = R(P.lj_thresh - 1.0);
+  if (sizeof(R) == 4) {
+    const float lt = float(P.lj_thresh);
+    const double half = (double(lt) + double(nextafterf(lt, INFINITY))) * 0.5 - 1.0;
+    float m = float(half);
+    if (double(m) > half) m = nextafterf(m, -INFINITY);
+    if (m + 1.f > lt) m = nextafterf(m, -INFINITY);  // a tie that rounds up
+    L.ljt1 = R(m);
+  }
   L.inv_ljt1sq = R(1.0 / ((P.lj_thresh - 1.0) * (P.lj_thresh - 1.0)));
   L.memb_far = R(P.der_der_const * ((1.0 - P.p_memb) / P.p_memb));
   return L;

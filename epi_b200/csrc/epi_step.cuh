@@ -114,13 +114,16 @@ template <typename R>
 struct Unit {
   Vec3<R> v;
   R inv;
+  Vec3<R> w;  // b - a
+  R scale;    // v = scale w
 };
 template <typename R>
 __device__ __forceinline__ Unit<R> unit_ab(const Vec3<R>& a, const Vec3<R>& b) {
   const Vec3<R> w = v3_sub(b, a);
   const R s = v3_dot(w, w);
   const R inv = lrsqrt(s);
-  return Unit<R>{v3_scale(inv, w), sizeof(R) == 4 ? ldiv(R(1), xmul(s, inv)) : inv};
+  return Unit<R>{v3_scale(inv, w), sizeof(R) == 4 ? ldiv(R(1), xmul(s, inv)) : inv, w,
+                 inv};
 }
 
 // The bending force of a membrane particle is a sum of terms g t, taken in a
@@ -142,10 +145,12 @@ __device__ __forceinline__ void bend_add(Vec3<R>& f, const BendTerm<R>& b) {
 //   kind 0   F ((a - c b) / |B| - (b - c a) / |A|)      the links on either side
 //   kind 1  -F (b - c a) / |A|                          the particle's own link, the next
 //   kind 2   F (a - c b) / |B|                          the link before, the one before that
-// taken in the order 0, 1, 2 of the row, then 1, 0, 2 of the column
-// (square_kind).
+//   kind 3   the same, a formed within the difference
+// taken in the order 0, 1, 2 of the row, then 1, 0, 3 of the column
+// (square_kind). The roundings (kind 3's too, and the order of the cross
+// products below) are those of the plain expressions as nvcc contracts them.
 constexpr int kSquareTerms = 6;
-__device__ __forceinline__ int square_kind(int e) { return e < 3 ? e : (e == 3 ? 1 : (e == 4 ? 0 : 2)); }
+__device__ __forceinline__ int square_kind(int e) { return e < 3 ? e : (e == 3 ? 1 : (e == 4 ? 0 : 3)); }
 template <typename R>
 __device__ __forceinline__ BendTerm<R> square_term(int kind, const Unit<R>& A, const Unit<R>& B,
                                                    R c) {
@@ -156,6 +161,10 @@ __device__ __forceinline__ BendTerm<R> square_term(int kind, const Unit<R>& A, c
     return BendTerm<R>{v3_axpy(B.inv, P, v3_neg(q)), F};
   }
   if (kind == 1) return BendTerm<R>{v3_scale(-F, Q), A.inv};
+  if (kind == 3) {
+    const Vec3<R> cb = v3_scale(c, B.v);
+    return BendTerm<R>{v3_scale(F, v3_axpy(A.scale, A.w, v3_neg(cb))), B.inv};
+  }
   return BendTerm<R>{v3_scale(F, P), B.inv};
 }
 
@@ -172,7 +181,7 @@ template <typename R>
 __device__ __forceinline__ BendTerm<R> tri_term1(const Vec3<R>& a, const Vec3<R>& b,
                                                  const Vec3<R>& c) {
   const Vec3<R> ab = v3_sub(a, b);
-  const Vec3<R> n1 = v3_unit(v3_cross(v3_neg(b), ab));
+  const Vec3<R> n1 = v3_unit(v3_cross(ab, b));  // -b x ab
   const Vec3<R> n2 = v3_unit(v3_cross(ab, v3_sub(c, b)));
   const R d = v3_dot(n1, n2);
   return BendTerm<R>{v3_cross(ab, v3_axpy(-d, n1, n2)), bend_factor(d)};  // ab x tri_rho(n1, n2)
@@ -181,8 +190,8 @@ template <typename R>
 __device__ __forceinline__ BendTerm<R> tri_term2(const Vec3<R>& a, const Vec3<R>& b,
                                                  const Vec3<R>& c) {
   const Vec3<R> bc = v3_sub(b, c), ab = v3_sub(a, b);
-  const Vec3<R> n1 = v3_unit(v3_cross(v3_neg(c), bc));
-  const Vec3<R> n2 = v3_unit(v3_cross(v3_neg(b), ab));
+  const Vec3<R> n1 = v3_unit(v3_cross(bc, c));  // -c x bc
+  const Vec3<R> n2 = v3_unit(v3_cross(ab, b));  // -b x ab
   const R d = v3_dot(n1, n2);
   const Vec3<R> t1 = v3_cross(bc, v3_axpy(-d, n1, n2));  // bc x tri_rho(n1, n2)
   const Vec3<R> t2 = v3_cross(ab, v3_axpy(-d, n2, n1));  // ab x tri_rho(n2, n1)
@@ -297,7 +306,7 @@ __device__ __forceinline__ double3 memb_force(const DevState& S, int32_t i) {
     bend_add(f, square_term(0, mv, mvb, v3_dot(mv.v, mvb.v)));
     // the reference reads memb_bb's ipn (:380)
     const R c = v3_dot(unit_ab(bb, bbr).v, unit_ab(bbr, bbrr).v);
-    bend_add(f, square_term(2, mvbb, mvb, c));
+    bend_add(f, square_term(3, mvbb, mvb, c));
   }
   const R s = R(T.P.dt * T.P.kbend);
   double ax = double(xmul(s, f.x)), ay = double(xmul(s, f.y)), az = double(xmul(s, f.z));
@@ -344,6 +353,7 @@ struct Particle {
   Pos p;
   const double lt2;  // LJ_THRESH * LJ_THRESH, folded as the reference does
   const R dt;
+  R inv_ljt1sq;  // for aad_fused
   int32_t pair_i = -1, dermis_i = -1;
   double ax = 0.0, ay = 0.0, az = 0.0;
   // the first too-strong interaction of this particle (|coef| > 1000): kept
@@ -373,6 +383,7 @@ struct Particle {
       : S(S_), i(i_), a(a_), t(attr_tissue(a)), st(attr_state(a)),
         T(T_), L(T.laws<R>()), p(own_),
         lt2(T.P.lj_thresh * T.P.lj_thresh), dt(R(T.P.dt)) {
+    if constexpr (kFloatPos && kSimple) inv_ljt1sq = rcp_approx(L.ljt1sq);
     if (!kSimple && st != ST_MEMB) {
       pair_i = __ldg(&S.pair[i]);
       if (st == ST_FIX || st == ST_MUSUME) dermis_i = S.dermis[i];
@@ -463,7 +474,7 @@ struct Particle {
     bool conn = !(s.over > T.ftol);
     if (conn && s.over >= -T.ftol) conn = connected_fp64(q);
     const bool both_old = kOld && attr_old(a) && attr_old(__ldg(&S.attr[q]));
-    float coef = L.aad_fused(s.d2, s.rs, both_old);
+    float coef = L.aad_fused(s.d2, s.rs, both_old, inv_ljt1sq);
     coef = conn ? coef : 0.f;
     note_bad(coef, q, 0);
     const float sdt = xmul(-dt, coef);
