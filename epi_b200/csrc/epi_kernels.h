@@ -81,7 +81,7 @@ struct ResidentCfg {
 // How a batch is laid out over the blocks; false: the batch is beyond what
 // the resident kernel takes (particles, or shared memory per block).
 struct ResidentPlan {
-  int32_t slots, grid, membs, tasks, terms, dealt, smem;
+  int32_t slots, grid, membs, turn, tasks, terms, group, smem;
 };
 // beyond this the kernel sequence fills the GPU and is the faster one (both
 // 17 us per step at 147,456 particles)

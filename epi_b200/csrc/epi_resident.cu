@@ -21,8 +21,9 @@
 // (0.4 us), and the evaluation, summing and committing chains. A step costs
 // 4.9 us for 768 particles (FP64; 21 in the graph), 6.9 for 36,864 (13.5),
 // 11.7 for 92,160 (16.1), and meets the sequence at 147,456 (17 both); FP64
-// forces 9.9 for 36,864 (18.1). Batches: 5 tissues of 57,984 particles 11.6
-// (19.4), 16 all-states tissues 21 (99).
+// forces 9.9 for 36,864 (18.1). Batches: 9 tissues of 106,112 particles 18.0
+// (20.6), 64 small ones of 49,152 17.5 (20.5); with every cell state and FP64
+// forces 16 tissues of 17,360 particles 20 (97), 64 53 (104), 118 97 (117).
 #include "epi_kernels.h"
 
 #include <algorithm>
@@ -34,17 +35,17 @@
 namespace epi {
 namespace {
 
-constexpr int kTile = 8;
-constexpr int kResidentMaxLog = 4;  // consecutive particles dealt to a block at a time
+constexpr int kTile = 8;  // consecutive particles dealt to a block at a time
 
 // Positions the run works on: step k reads pos(k), writes pos(k + 1).
 struct ResidentArgs {
   int32_t nsteps;
   int32_t slots;            // particles per block
   int32_t membs;            // membrane particles a block may hold
+  int32_t turn;             // of which it holds the terms at a time
   int32_t tasks;            // pair terms a block holds at a time
   int32_t terms;            // bending threads per membrane particle
-  int32_t dealt;            // tiles of particles are dealt round the blocks
+  int32_t group;            // blocks that deal their range's tiles of particles among them
   int32_t thread_from;      // candidate search: a thread per particle from here on
   unsigned* bar;            // barrier arrivals (zero at launch)
   unsigned* other;          // the next run's (zeroed here)
@@ -124,7 +125,7 @@ __device__ __noinline__ bool resident_rebuild(const DevState& S0, double4* pos, 
 }
 
 constexpr int kLinks = kMembAdjTri + 1;  // springs of a membrane particle, and its wall
-constexpr int kTissues = 8;  // tissues of a block whose constants it keeps
+constexpr int kTissues = 8;  // tissues of a group whose constants its blocks keep
 
 // What a block keeps of its particles (slots) in shared memory between steps:
 // an L2 load costs 700 cycles and more here, and after a barrier L1 holds
@@ -138,8 +139,8 @@ struct Slots {
   Pos* own;         // the same as the forces see them (FP64 path: pos itself)
   float4* bpos;     // positions at the last candidate rebuild
   R* term;          // pair terms x | y | z (tasks each)
-  R* bend;          // bending terms t, g: 4 x terms per membrane slot
-  R* link;          // spring terms and the wall: 3 x kLinks per membrane slot
+  R* bend;          // bending terms t, g: 4 x terms per membrane slot of a turn
+  R* link;          // spring terms and the wall: 3 x kLinks of the same
   uint32_t* attr;
   int32_t* off;     // slots + 1: first pair task of each slot
   int32_t* at;      // membrane slot: its place in list
@@ -149,13 +150,14 @@ struct Slots {
   static constexpr bool kOwn = sizeof(R) == 4;
   // terms: bending threads per membrane particle (kTriTerms, or with square
   // lattices only kSquareTerms + 2)
-  static __host__ __device__ constexpr size_t bytes(int slots, int membs, int tasks, int terms) {
+  static __host__ __device__ constexpr size_t bytes(int slots, int membs, int turn, int tasks,
+                                                    int terms) {
     return (size_t)slots * (sizeof(double4) + 24 + (kOwn ? sizeof(float4) : 0) + sizeof(float4) + 8) +
            (size_t)membs * 24 +
-           sizeof(R) * 3 * tasks + sizeof(R) * (4 * terms + 3 * kLinks) * membs +
+           sizeof(R) * 3 * tasks + sizeof(R) * (4 * terms + 3 * kLinks) * turn +
            4 * (slots + 4 + 2 * membs + tasks);
   }
-  __device__ Slots(unsigned char* m, int slots, int membs, int tasks, int terms) {
+  __device__ Slots(unsigned char* m, int slots, int membs, int turn, int tasks, int terms) {
     pos = reinterpret_cast<double4*>(m);
     bpos = reinterpret_cast<float4*>(pos + slots);
     unsigned char* rest = reinterpret_cast<unsigned char*>(bpos + slots);
@@ -168,8 +170,8 @@ struct Slots {
     sum = reinterpret_cast<double*>(rest);
     msum = sum + 3 * slots;
     bend = reinterpret_cast<R*>(msum + 3 * membs);
-    link = bend + 4 * terms * membs;
-    term = link + 3 * kLinks * membs;
+    link = bend + 4 * terms * turn;
+    term = link + 3 * kLinks * turn;
     attr = reinterpret_cast<uint32_t*>(term + 3 * tasks);
     off = reinterpret_cast<int32_t*>(attr + slots);
     at = off + slots + 1;
@@ -225,11 +227,11 @@ __device__ __forceinline__ BendTerm<R> bend_task(const DevState& S, int32_t i,
 
 // NT threads per block, one block per SM (more threads would halve their
 // registers: at 64 a thread spilled 45 words a step, and a reload misses L1
-// after a barrier: 9.2 us per step on 36,864 particles against 7.0). Block
-// b's particles (slots): of up to kTissues tissues, tiles of kTile particles
-// dealt round the blocks, so every block gets its share of the membrane; of
-// more, consecutive ones, so a block meets few tissues. The constants of its
-// tissues are in shared memory, those of a single one (kOne) arguments.
+// after a barrier: 9.2 us per step on 36,864 particles against 7.0). A group
+// of blocks holds consecutive particles of about kTissues tissues, whose
+// constants each block has in shared memory (those of a single one, kOne, are
+// arguments), and deals them round in tiles of kTile particles, so that every
+// block gets its share of the membrane and of the long rows.
 template <typename R, bool kSimple, bool kOld, bool kOne, int NT, int kMin>
 __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ DevState S0,
                                                        const __grid_constant__ ResidentArgs A,
@@ -240,7 +242,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   __shared__ __align__(16) unsigned char s_tissue[kTissues][sizeof(TissueDev)];
   __shared__ int32_t s_nm, s_t0;
   const int slots = A.slots;
-  const Slots<R> K(smem, slots, A.membs, A.tasks, A.terms);
+  const Slots<R> K(smem, slots, A.membs, A.turn, A.tasks, A.terms);
   const int32_t n = (int32_t)S0.n_total;
   const int tid = (int)threadIdx.x;
   DevState S = S0;
@@ -249,16 +251,18 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   GridBarrier B{A.bar, A.abort, S0.status, 0u};
   unsigned long long counted = 0;
   int32_t flagged = *(volatile const int32_t*)S0.gate;
+  // this block's group: its first particle, its blocks, the block's place
+  const int32_t lead = kOne ? 0 : (int32_t)blockIdx.x / A.group * A.group;
+  const int32_t deal = kOne ? (int32_t)gridDim.x : min(A.group, (int32_t)gridDim.x - lead);
   auto particle = [&](int slot) {
-    return kOne || A.dealt ? (slot / kTile * (int32_t)gridDim.x + (int32_t)blockIdx.x) * kTile + slot % kTile
-                : (int32_t)blockIdx.x * slots + slot;
+    return lead * slots + (slot / kTile * deal + (int32_t)blockIdx.x - lead) * kTile + slot % kTile;
   };
   // once: the slots' attributes, positions and membrane list, and the
   // constants of the block's first tissues
   if (tid == 0) {
     if (blockIdx.x == 0) *A.other = 0u;
     s_nm = 0;
-    s_t0 = !A.dealt && particle(0) < n ? (int32_t)attr_tissue(S0.attr[particle(0)]) : 0;
+    s_t0 = !kOne && lead * slots < n ? (int32_t)attr_tissue(S0.attr[lead * slots]) : 0;
   }
   __syncthreads();
   for (int s = tid; s < slots; s += NT) {
@@ -339,11 +343,14 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
         dermis_cell(S, S.prep[e], tid & 31);
       if (!B.sync(nullptr, nullptr)) break;
     }
-    for (int from = 0; from < slots; from = c1) {
-      // the slots from `from` on whose pair tasks fit; listed once per
-      // rebuild when all do
-      if (c0 != from || c1 == from) {
-        __syncthreads();
+    // in turns: pair terms of the slots from `from` on, membrane terms of the
+    // membrane slots from `m0` on, as many as fit (kSimple: all of them)
+    const int held = min(s_nm, A.membs);  // (the same: the host counted them)
+    int from = 0, m0 = 0;
+    do {
+      const bool pairs = kSimple || from < slots;
+      // the slots whose pair tasks fit; listed once per rebuild when all do
+      if (pairs && (c0 != from || c1 == from)) {
         c0 = from;
         int lo = from + 1, hi = slots;
         while (lo < hi) {
@@ -369,7 +376,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
         __syncthreads();
       }
       // every term of these slots: a thread each
-      const int32_t t0 = K.off[c0], np = K.off[c1] - t0;
+      const int32_t t0 = K.off[c0], np = pairs ? K.off[c1] - t0 : 0;
       R *tx = K.term, *ty = tx + A.tasks, *tz = ty + A.tasks;
       const Pos* src;
       if constexpr (Part::kFloatPos) src = S.posf_cur;
@@ -400,23 +407,24 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
           }
         }
       }
-      if (from == 0) {
+      const int nm = kSimple && from > 0 ? 0 : min(held - m0, A.turn);
+      if (nm > 0) {
         // the membrane: bending terms, then lattice springs, A.terms and
         // kLinks threads per particle, from the first warp on that took
         // no or one pair task less
-        const int nm = s_nm, nb32 = (nm * A.terms + 31) & ~31, nl = nm * kLinks;
+        const int nb32 = (nm * A.terms + 31) & ~31, nl = nm * kLinks;
         for (int t = (tid + NT - (np & ~31) % NT) % NT; t < nb32 + nl; t += NT) {
           const bool spring = t >= nb32;
           const int r = spring ? t - nb32 : t;
           const int m = r / (spring ? kLinks : A.terms);
           const int e = r - m * (spring ? kLinks : A.terms);
           const bool in = m < nm;
-          const int slot = in ? K.list[m] : 0;
+          const int slot = in ? K.list[m0 + m] : 0;
           const int32_t i = particle(slot);
           const TissueDev& T = tissue(K.attr[slot]);
           const bool tri = T.lattice == kLatticeTriangular;
           const SiteOffsets<R> off(S, K.own[slot], T);
-          const int32_t jk = in ? K.jk[m] : 0;
+          const int32_t jk = in ? K.jk[m0 + m] : 0;
           const MembSites M(T, i, jk & 0xffff, jk >> 16);
           if (spring) {
             if (!in) continue;
@@ -447,7 +455,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
       __syncthreads();
       // sums in the order of the thread-per-particle kernels, a thread per
       // component: the slots' pair terms, then the membrane's
-      const int ns = c1 - c0, nm = from == 0 ? s_nm : 0;
+      const int ns = pairs ? c1 - c0 : 0;
       for (int r = tid; r < 3 * (ns + nm); r += NT) {
         if (r < 3 * ns) {
           const int s = c0 + r / 3, c = r % 3;
@@ -458,7 +466,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
           for (int t = K.off[s] - t0; t < end; ++t) sum = xadd(sum, double(v[t]));
           K.sum[3 * s + c] = sum;
         } else {
-          const int m = (r - 3 * ns) / 3, c = (r - 3 * ns) % 3, slot = K.list[m];
+          const int m = (r - 3 * ns) / 3, c = (r - 3 * ns) % 3, slot = K.list[m0 + m];
           const TissueDev& T = tissue(K.attr[slot]);
           const int nb = T.lattice == kLatticeTriangular ? kTriTerms : kSquareTerms;
           const R* b = K.bend + 4 * A.terms * m;
@@ -471,29 +479,31 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
           for (int e = 0; e < T.nadj; ++e) sum = xadd(sum, double(l[3 * e]));
           // (adding no wall, +0, changes nothing: the sum is not -0)
           if (c == 2) sum = xadd(sum, double(l[3 * kMembAdjTri - 2]));
-          K.msum[3 * m + c] = sum;
+          K.msum[3 * (m0 + m) + c] = sum;
         }
       }
       __syncthreads();
-      // the commit, a thread per particle
-      for (int s = c0 + tid; s < c1; s += NT) {
-        const int32_t i = particle(s);
-        if (i >= n) continue;
-        const uint32_t a = K.attr[s];
-        const double4 p = K.pos[s];
-        Part P(S, i, a, K.own[s], tissue(a));
-        P.ax = K.sum[3 * s];
-        P.ay = K.sum[3 * s + 1];
-        P.az = K.sum[3 * s + 2];
-        double4 f = make_double4(0.0, 0.0, 0.0, 0.0);
-        if (attr_state(a) == ST_MEMB) {
-          const double* v = K.msum + 3 * K.at[s];
-          f = make_double4(v[0], v[1], v[2], 0.0);
-        }
-        const double4 q = P.finish(p, K.bpos[s], f);
-        K.pos[s] = q;
-        if constexpr (Slots<R>::kOwn) K.own[s] = Part::own(q);
+      if (pairs) from = c1;
+      if (!kSimple) m0 += nm;
+    } while (from < slots || (!kSimple && m0 < held));
+    // the commit, a thread per particle
+    for (int s = tid; s < slots; s += NT) {
+      const int32_t i = particle(s);
+      if (i >= n) continue;
+      const uint32_t a = K.attr[s];
+      const double4 p = K.pos[s];
+      Part P(S, i, a, K.own[s], tissue(a));
+      P.ax = K.sum[3 * s];
+      P.ay = K.sum[3 * s + 1];
+      P.az = K.sum[3 * s + 2];
+      double4 f = make_double4(0.0, 0.0, 0.0, 0.0);
+      if (attr_state(a) == ST_MEMB) {
+        const double* v = K.msum + 3 * K.at[s];
+        f = make_double4(v[0], v[1], v[2], 0.0);
       }
+      const double4 q = P.finish(p, K.bpos[s], f);
+      K.pos[s] = q;
+      if constexpr (Slots<R>::kOwn) K.own[s] = Part::own(q);
     }
     if (A.hist) {
       S.pos_cur = S.pos_nxt;
@@ -540,6 +550,15 @@ constexpr int kLeastSlots = 16;
 // density, a part of them for batches of every cell state, whose membrane rows
 // are short and cell rows long (the rest of a step's follow in turns)
 constexpr int kLeastTasks = 8, kLeastTasksGeneral = 3;
+// membrane particles per block: a step takes about 10 us and 0.07 more for
+// each (112: 17.5 us, 168: 21.9, 224: 26.2, mixed precision), the sequence 20
+// to 22 at the same sizes. (Batches of every cell state are not limited: 240
+// of FP64 29 us, the sequence 99.)
+constexpr int kMostMembs = 144;
+// Turns that the membrane terms of such a batch may take: at 64 tissues (472
+// membrane particles per block, FP64) two, 53 us a step; at 118 seven, 97;
+// the sequence 104 and 117.
+constexpr int kMostTurns = 8;
 
 }  // namespace
 
@@ -551,25 +570,44 @@ bool resident_plan(const TissueDev* T, int32_t ntissues, int64_t n, int precisio
   const int64_t share = ((n + lc.num_sms - 1) / lc.num_sms + kTile - 1) / kTile * kTile;
   P.slots = (int32_t)std::max<int64_t>(share, kLeastSlots);
   P.grid = (int32_t)((n + P.slots - 1) / P.slots);
-  P.dealt = ntissues <= kTissues ? 1 : 0;
+  // the largest group whose particles are of kTissues tissues at most: more
+  // tissues than that hold all of the ones between their first and last
+  int64_t range = (int64_t)P.grid * P.slots;
+  for (int32_t t = kTissues; t < ntissues; ++t)
+    range = std::min<int64_t>(range, T[t].pbase - T[t - kTissues + 1].pbase + 1);
+  P.group = (int32_t)std::max<int64_t>(range / P.slots, 1);
+  // membrane particles of a block, group by group: the tiles that a tissue's
+  // membrane touches, dealt round
   bool tri = false;
-  int64_t membs = 0;
+  int64_t membs = 0, most = 0, of = 0;
   for (int32_t t = 0; t < ntissues; ++t) {
     tri |= T[t].lattice == kLatticeTriangular;
-    // tiles the tissue's membrane touches, dealt round the blocks
-    const int64_t tiles = (T[t].pbase + T[t].nmemb + kTile - 1) / kTile - T[t].pbase / kTile;
-    membs += (tiles + P.grid - 1) / P.grid * kTile;
+    if (!T[t].nmemb) continue;
+    const int64_t per = (int64_t)P.group * P.slots, end = T[t].pbase + T[t].nmemb;
+    for (int64_t g = T[t].pbase / per; g <= (end - 1) / per; ++g) {
+      if (g != of) membs = 0;
+      of = g;
+      const int64_t deal = std::min<int64_t>(P.group, P.grid - g * P.group);
+      const int64_t lo = std::max<int64_t>(T[t].pbase, g * per), hi = std::min(end, (g + 1) * per);
+      const int64_t tiles = (hi + kTile - 1) / kTile - lo / kTile;
+      membs += (tiles + deal - 1) / deal * kTile;
+      most = std::max(most, membs);
+    }
   }
-  P.membs = (int32_t)std::min<int64_t>(P.slots, P.dealt ? membs : P.slots);
+  P.membs = (int32_t)std::min<int64_t>(P.slots, most);
+  if (lc.simple && P.membs > kMostMembs) return false;
   P.terms = tri ? kTriTerms : kSquareTerms + 2;
+  P.turn = P.membs;
   auto bytes = [&](int tasks) {
-    return precision == 1 ? Slots<float>::bytes(P.slots, P.membs, tasks, P.terms)
-                          : Slots<double>::bytes(P.slots, P.membs, tasks, P.terms);
+    return precision == 1 ? Slots<float>::bytes(P.slots, P.membs, P.turn, tasks, P.terms)
+                          : Slots<double>::bytes(P.slots, P.membs, P.turn, tasks, P.terms);
   };
   // room for the pair terms of all slots at 24 partners each, as far as it
   // goes, and for the longest row
   const int least =
       std::max(P.slots * (lc.simple ? kLeastTasks : kLeastTasksGeneral), max_cand);
+  for (int turns = 2; !lc.simple && turns <= kMostTurns && bytes(least) > kSmemPerBlock; ++turns)
+    P.turn = (P.membs + turns - 1) / turns;
   P.tasks = std::max(P.slots * 24, max_cand);
   while (P.tasks > least && bytes(P.tasks) > kSmemPerBlock) P.tasks -= std::min(64, P.tasks - least);
   P.smem = (int32_t)bytes(P.tasks);
@@ -591,9 +629,10 @@ cudaError_t launch_resident(const DevState& S, const ResidentPlan& P, const Tiss
   A.nsteps = nsteps;
   A.slots = P.slots;
   A.membs = P.membs;
+  A.turn = P.turn;
   A.tasks = P.tasks;
   A.terms = P.terms;
-  A.dealt = P.dealt;
+  A.group = P.group;
   A.thread_from = lc.search_switch;
   A.bar = reinterpret_cast<unsigned*>(rc.sync) + (rc.run & 1);
   A.other = reinterpret_cast<unsigned*>(rc.sync) + (~rc.run & 1);

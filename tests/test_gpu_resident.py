@@ -5,8 +5,8 @@ Both evaluate the same operations in the same order, so positions must agree
 bit for bit, with candidate rebuilds along the way (a small skin forces
 many). Forms: the smallest grid, sizes around the tiles a block is dealt,
 both lattices, every cell state (long rows, several turns of a block's pair
-terms), up to eight tissues dealt tile by tile and more laid out in order,
-old cells, runs longer than one launch, one step per call.
+terms, then of its membrane terms as well), up to eight tissues dealt tile by
+tile over all blocks and more over groups of blocks, old cells, runs longer than one launch, one step per call.
 """
 import numpy as np
 import pytest
@@ -36,10 +36,12 @@ def cases():
         "wide": ([small(64, 4, 6)], 30, {}),
         "eight": ([small(12 + k, 2, k) for k in range(8)], 30, {}),
         "eleven": ([small(12 + k, 2, k) for k in range(11)], 30, {}),
+        "sixty": ([small(10 + k % 5, 1 + k % 3, k) for k in range(60)], 20, {}),
         "lattices": ([small(16, 2, 1), T.tri_layered_tissue(17, 20, 3, 2)], 30, {}),
         "all states": ([T.mixed_state_tissue(3)], 30, ALL),
         "all states tri": ([T.mixed_state_tissue(4, T.TRIANGULAR), small(16, 2, 7)], 30, ALL),
         "all states x 12": ([T.mixed_state_tissue(k) for k in range(12)], 20, ALL),
+        "all states x 70": ([T.mixed_state_tissue(k, k % 2) for k in range(70)], 6, ALL),
         "all states x 40": ([T.mixed_state_tissue(k) for k in range(40)], 6, ALL),
         "long": ([small(12, 2, 8)], 1100, {}),
     }
