@@ -1,12 +1,14 @@
 // Mechanics kernels for sm_100a.
 //
 // One step of the reference (epi5_MT/proc.cpp:22-32 without state renewal)
-// runs as
+// runs as the sequence below (small batches: as phases of one resident kernel,
+// epi_resident.cu)
 //   [rebuild]  Verlet candidate rebuild of the tissues that need one
 //              (bin -> scan -> scatter -> per-bin sort -> candidate search);
 //              every kernel of it exits at once when no tissue does
-//   k_prepass  membrane bending scratch (_memb_bend_calc1) and the dermis of
-//              FIX / MUSUME cells (find_dermis)
+//   k_memb_force  bending, lattice springs and wall of the membrane
+//              (_memb_bend_calc1..3, tri_memb_bend, _MEMB_interaction)
+//   k_dermis   the dermis of FIX / MUSUME cells (find_dermis)
 //   k_step     connect_proc's exact predicate over the candidates, every
 //              force of cell_interaction, pos_copy and the periodic wrap,
 //              fused; flags tissues whose particles moved more than skin/2
@@ -154,8 +156,8 @@ __global__ void k_gate_set_all(DevState S, int32_t ntissues) {
 
 // ---------------------------------------------------------------------------
 // find_dermis for the FIX / MUSUME cells in prep[f0, f1), from the current
-// positions, one warp per cell: 64 all-states tissues (640 such cells) 68 us
-// with a thread per cell.
+// positions, one warp per cell: 64 all-states tissues (640 such cells) took
+// 68 us with a thread per cell, 128 take 8.
 // ---------------------------------------------------------------------------
 __global__ void k_dermis(DevState S, int32_t f0, int32_t f1) {
   pdl_entry();
@@ -268,7 +270,8 @@ __device__ __forceinline__ void gather_candidates(const DevState& S, Part& P, co
 // spill, four blocks per SM. On 6.56M particles (512 tissues): 0.333 ms with
 // three blocks and four gathers and all inputs loaded first, 0.329 ms with
 // the late loads, 0.291 ms with four blocks and two gathers (0.309 with one,
-// 0.308 with three, 0.326 with four; five blocks 0.326 to 0.338 with spills).
+// 0.308 with three, 0.326 with four; five blocks 0.326 to 0.338 with spills);
+// 0.294 ms with the laws' roundings of the plain expressions.
 // FP64 forces, 96 tissues: three blocks with one gather 91 us, with two 97;
 // two blocks without spills 110.
 // Streaming loads that do not allocate in L1 (the particle's own inputs,
