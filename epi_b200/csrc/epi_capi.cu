@@ -143,7 +143,7 @@ struct epi_ctx {
   unsigned long long* rebuilds = nullptr;
   int32_t* loop_left = nullptr;  // passes left in the step graph's device loop
   unsigned long long* launches = nullptr;  // step-sequence kernels executed
-  int32_t* res_sync = nullptr;   // grid barrier words of the resident kernel
+  int32_t* res_sync = nullptr;   // words of the resident kernel (ResidentCfg::sync)
   uint32_t res_run = 0;          // its runs so far (which barrier word is next)
   int coop = 0;                  // the device takes cooperative launches
   unsigned char* adj_mem = nullptr;  // epi_adjoint's block (AdjointArena)
@@ -276,6 +276,7 @@ DevState make_state(epi_ctx* c, int cur) {
   S.skey = c->skey;
   S.spos = c->spos;
   S.gate = c->gate;
+  S.flag = c->gate;
   S.rl_count = c->rl;
   S.rl_list = c->rl ? c->rl + 1 : nullptr;
   S.rl_ppre = c->rl ? c->rl + 1 + c->ntissues : nullptr;
@@ -541,7 +542,7 @@ int check_status(epi_ctx* c, bool posted = false) {
     c->last = *c->status_h;
     c->last.flags &= ~kStatusPosted;
     EPI_CUDA(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
-    EPI_CUDA(cudaMemsetAsync(c->res_sync, 0, 4 * sizeof(int32_t), c->stream));
+    EPI_CUDA(cudaMemsetAsync(c->res_sync, 0, kResidentWords * sizeof(int32_t), c->stream));
     EPI_CUDA(cudaStreamSynchronize(c->stream));
     return c->last.code;
   }
@@ -889,8 +890,8 @@ int epi_create(epi_ctx** out, const epi_config* cfg) {
   if (rc == EPI_OK) rc = dev_alloc(&ctx->rebuilds, 1);
   if (rc == EPI_OK) rc = dev_alloc(&ctx->loop_left, 1);
   if (rc == EPI_OK) rc = dev_alloc(&ctx->launches, 1);
-  if (rc == EPI_OK) rc = dev_alloc(&ctx->res_sync, 4);
-  if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->res_sync, 0, 4 * sizeof(int32_t)));
+  if (rc == EPI_OK) rc = dev_alloc(&ctx->res_sync, kResidentWords);
+  if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->res_sync, 0, kResidentWords * sizeof(int32_t)));
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->launches, 0, sizeof(unsigned long long)));
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->rebuilds, 0, sizeof(unsigned long long)));
   if (rc != EPI_OK) {

@@ -101,6 +101,7 @@ struct DevState {
   uint32_t* skey;   // sorted particles: global index | (is_memb << 31)
   float4* spos;     // sorted copy of the positions at rebuild; w: +-LJ_THRESH * radius
   int32_t* gate;    // [0]: some tissue needs a rebuild, [1 + t]: tissue t does
+  int32_t* flag;    // where a step's commit notes the former: gate, in a resident run its own word
   int32_t* rl_count;  // rebuild work list: number of gated tissues
   int32_t* rl_list;   // their ids
   int32_t* rl_ppre;   // prefix sums of their particle counts (count + 1 entries)

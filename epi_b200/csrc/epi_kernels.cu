@@ -102,7 +102,7 @@ __global__ void k_scan_final(const int32_t* __restrict__ in, int32_t* __restrict
 __global__ void k_gate_compact(DevState S, int32_t t0, int32_t t1) {
   pdl_entry();
   count_launch(S.launches);
-  gate_compact<kScanThreads>(S, t0, t1, t0 == 0 && t1 == S.ntissues);
+  gate_compact<kScanThreads>(S, t0, t1, S.gate[0] != 0, t0 == 0 && t1 == S.ntissues);
 }
 
 __global__ void k_bin(DevState S) {
@@ -144,7 +144,7 @@ __global__ void k_rebuild_condition(DevState S, int32_t t0, int32_t t1,
                                     cudaGraphConditionalHandle h) {
   pdl_entry();
   count_launch(S.launches);
-  gate_compact<kScanThreads>(S, t0, t1, t0 == 0 && t1 == S.ntissues);
+  gate_compact<kScanThreads>(S, t0, t1, S.gate[0] != 0, t0 == 0 && t1 == S.ntissues);
   __syncthreads();
   if (threadIdx.x == 0) cudaGraphSetConditional(h, S.rl_count[0] > 0 ? 1u : 0u);
 }

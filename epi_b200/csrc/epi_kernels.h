@@ -68,9 +68,11 @@ void launch_step(const DevState& S, const Range& r, int precision, const LaunchC
                  cudaStream_t s, Timer* tm);
 // The same for nsteps steps of a small batch in one cooperative kernel
 // (epi_resident.cu), candidate rebuilds included.
+constexpr int kResidentWords = 5;
 struct ResidentCfg {
   int32_t* sync;      // device words: two barrier counts, used by runs in turn
-  uint32_t run;       // (each run clears the next one's), and the abort flag
+  uint32_t run;       // (each run clears the next one's), the abort flag, and
+                      // the two words of RunFlags
   DevStatus* post;    // pinned host memory the status goes to at the end, with
                       // kStatusPosted among the flags; or null
   int32_t per_step, per_pair, per_rebuild;  // kernels of the sequence each step, each

@@ -93,12 +93,13 @@ __device__ __forceinline__ int32_t ref_bin(const TissueDev& T, double x, double 
 // index back to (tissue, local index) by binary search in the prefix sums.
 // With nothing gated the list is empty and each kernel exits at once.
 // ---------------------------------------------------------------------------
-// Run by one block of NT threads. clear (whole batch): the "some tissue" word
-// is cleared once the list is built; the step sets it again for the next step.
+// Run by one block of NT threads. any: the "some tissue" word. clear (whole
+// batch): gate[0] is cleared once the list is built; the step sets it again
+// for the next step.
 template <int NT>
-__device__ __forceinline__ void gate_compact(const DevState& S, int32_t t0, int32_t t1,
+__device__ __forceinline__ void gate_compact(const DevState& S, int32_t t0, int32_t t1, bool any,
                                              bool clear) {
-  if (S.gate[0] == 0) {
+  if (!any) {
     if (threadIdx.x == 0) {
       S.rl_count[0] = 0;
       S.rl_ppre[0] = 0;
@@ -119,7 +120,7 @@ __device__ __forceinline__ void gate_compact(const DevState& S, int32_t t0, int3
     }
     return;
   }
-  __syncthreads();  // every thread has read gate[0] before it is cleared
+  __syncthreads();  // every thread has read the word before it is cleared
   if (clear && threadIdx.x == 0) S.gate[0] = 0;
   int32_t cc = 0, cp = 0, cb = 0;
   for (int32_t base = t0; base < t1; base += NT) {

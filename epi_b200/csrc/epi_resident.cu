@@ -30,6 +30,7 @@
 
 #include "epi_device.cuh"
 #include "epi_rebuild.cuh"
+#include "epi_run_words.h"
 #include "epi_step.cuh"
 
 namespace epi {
@@ -50,6 +51,7 @@ struct ResidentArgs {
   unsigned* bar;            // barrier arrivals (zero at launch)
   unsigned* other;          // the next run's (zeroed here)
   int32_t* abort;           // set when a barrier wait gave up
+  int32_t* flags;           // RunFlags::words
   DevStatus* post;          // non-null: pinned host memory the status is put in
   int32_t per_step, per_pair, per_rebuild;  // launches counted (see epi_launch_count)
   double4* hist;            // non-null: step k's positions go to hist + k n_total
@@ -65,9 +67,9 @@ struct GridBarrier {
   int32_t* abort;
   DevStatus* status;
   unsigned target;
-  // flag: a word read by thread 0 after the barrier and returned to all
-  // threads of the block (the same value in every block: nothing writes it
-  // between this barrier and the next). False: some block gave up.
+  // word: read by thread 0 after the barrier and returned to all threads of
+  // the block (the same value in every block: see RunFlags). False: some
+  // block gave up.
   __device__ __forceinline__ bool sync(const int32_t* word, int32_t* value) {
     __shared__ int32_t s_word, s_ok;
     __syncthreads();
@@ -101,16 +103,16 @@ struct GridBarrier {
 };
 
 // The candidate rebuild of the flagged tissues, the phases of launch_rebuild
-// between barriers. The flag every block acted on (gate[0]) is cleared only
-// once all blocks are past the first barrier here.
+// between barriers. The word every block acted on, *flag, is cleared once all
+// blocks are past the first barrier here (RunFlags).
 template <int NT>
 __device__ __noinline__ bool resident_rebuild(const DevState& S0, double4* pos, int32_t thread_from,
-                                              GridBarrier& B) {
+                                              int32_t* flag, GridBarrier& B) {
   DevState S = S0;
   S.pos_cur = pos;
-  if (blockIdx.x == 0) gate_compact<NT>(S, 0, S.ntissues, false);
+  if (blockIdx.x == 0) gate_compact<NT>(S, 0, S.ntissues, true, false);
   if (!B.sync(nullptr, nullptr)) return false;
-  if (blockIdx.x == 0 && threadIdx.x == 0) S.gate[0] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *flag = 0;
   rebuild_bin(S);
   if (!B.sync(nullptr, nullptr)) return false;
   rebuild_scan<NT>(S);
@@ -250,7 +252,8 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   if (A.hist) S.pos_nxt = A.hist + n;
   GridBarrier B{A.bar, A.abort, S0.status, 0u};
   unsigned long long counted = 0;
-  int32_t flagged = *(volatile const int32_t*)S0.gate;
+  const RunFlags flags{S0.gate, A.flags};
+  int32_t flagged = *(volatile const int32_t*)flags.read_by(0);
   // this block's group: its first particle, its blocks, the block's place
   const int32_t lead = kOne ? 0 : (int32_t)blockIdx.x / A.group * A.group;
   const int32_t deal = kOne ? (int32_t)gridDim.x : min(A.group, (int32_t)gridDim.x - lead);
@@ -305,9 +308,10 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   bool done = false;
   for (int32_t step = 0; step < A.nsteps; ++step) {
     counted += A.per_step + ((step & 1) ? A.per_pair : 0);
+    S.flag = flags.raised_by(step);
     if (flagged) {
       counted += A.per_rebuild;
-      if (!resident_rebuild<NT>(S0, S.pos_cur, A.thread_from, B)) break;
+      if (!resident_rebuild<NT>(S0, S.pos_cur, A.thread_from, flags.read_by(step), B)) break;
       fresh = rebuilt = true;
     }
     if (fresh) {
@@ -516,10 +520,14 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
     float4* tf = S.posf_cur;
     S.posf_cur = S.posf_nxt;
     S.posf_nxt = tf;
-    if (!B.sync(S0.gate, &flagged)) break;
     done = step + 1 == A.nsteps;
+    if (!B.sync(done ? nullptr : flags.read_by(step + 1), &flagged)) {
+      done = false;
+      break;
+    }
   }
   if (blockIdx.x == 0 && tid == 0) {
+    if (done) flags.hand_on(A.nsteps);
     if (S0.launches) atomicAdd(S0.launches, counted);
     // past the last barrier every block has raised what it had to: the host
     // finds the status after its wait for the stream, without a copy
@@ -637,6 +645,7 @@ cudaError_t launch_resident(const DevState& S, const ResidentPlan& P, const Tiss
   A.bar = reinterpret_cast<unsigned*>(rc.sync) + (rc.run & 1);
   A.other = reinterpret_cast<unsigned*>(rc.sync) + (~rc.run & 1);
   A.abort = rc.sync + 2;
+  A.flags = rc.sync + 3;
   A.post = rc.post;
   A.per_step = rc.per_step;
   A.per_pair = rc.per_pair;

@@ -1,0 +1,39 @@
+// Which device words the blocks of a resident run (epi_resident.cu) read and
+// write between its grid barriers: plain index rules, shared with the host.
+#pragma once
+#include <cstdint>
+
+#ifdef __CUDACC__
+#define EPI_HD __host__ __device__ __forceinline__
+#else
+#define EPI_HD inline
+#endif
+
+namespace epi {
+
+// "Some tissue needs a candidate rebuild" in a run of steps. A step's commit
+// raises it, and after the barrier that ends the step every block reads it
+// and, if it is set, takes part in the rebuild that begins the next step. A
+// fast block may commit the next step while a slow one has yet to read, so
+// the word a step raises is never the one read at its beginning: gate is the
+// word the run starts from (S.gate[0], which no step raises), step k raises
+// words[k & 1]. A set word is cleared by one block within the rebuild it
+// causes, past the rebuild's first barrier: by then every block has read it,
+// and no block commits before the rebuild's last barrier. A word that is not
+// set needs no clearing, so each is zero again when step k + 2 raises it.
+struct RunFlags {
+  int32_t* gate;
+  int32_t* words;  // two, zero between runs
+  EPI_HD int32_t* raised_by(int32_t step) const { return words + (step & 1); }
+  EPI_HD int32_t* read_by(int32_t step) const { return step == 0 ? gate : raised_by(step - 1); }
+  // After the last barrier, by one block (nobody else reads the words any
+  // more): what the last step raised becomes the next run's first flag.
+  EPI_HD void hand_on(int32_t nsteps) const {
+    volatile int32_t* last = read_by(nsteps);
+    if (!*last) return;
+    *last = 0;
+    *(volatile int32_t*)gate = 1;
+  }
+};
+
+}  // namespace epi

@@ -590,7 +590,7 @@ struct Particle {
     // Candidate validity: rebuild the tissue once a particle moved skin/2.
     if (moved_too_far(S.skin, T, nx, ny, nz, b)) {
       S.gate[1 + t] = 1;
-      S.gate[0] = 1;
+      *S.flag = 1;
     }
     return make_double4(nx, ny, nz, p.w);
   }
