@@ -144,7 +144,7 @@ struct epi_ctx {
   int32_t* loop_left = nullptr;  // passes left in the step graph's device loop
   unsigned long long* launches = nullptr;  // step-sequence kernels executed
   int32_t* res_sync = nullptr;   // words of the resident kernel (ResidentCfg::sync)
-  uint32_t res_run = 0;          // its runs so far (which barrier word is next)
+  RunCount res_runs;             // its runs so far
   int coop = 0;                  // the device takes cooperative launches
   unsigned char* adj_mem = nullptr;  // epi_adjoint's block (AdjointArena)
   size_t adj_bytes = 0;
@@ -380,12 +380,18 @@ bool resident(const epi_ctx* c, ResidentPlan* P) {
 
 bool conditional_rebuild(const epi_ctx* c);
 
-// nsteps steps in the resident kernel. graph: what the launch count stands
+// The next *left steps in the resident kernel, if the batch steps there; *left
+// comes back as what remains for the kernel sequence (all or nothing, unless
+// the device stops taking the launches). graph: what the launch count stands
 // for, the replayed graph or the eager sequence (see epi_launch_count).
-int enqueue_resident(epi_ctx* c, const ResidentPlan& P, int32_t nsteps, bool graph) {
+// *posted: see check_status.
+int enqueue_resident(epi_ctx* c, int32_t* left, bool graph, bool* posted) {
+  ResidentPlan P;
+  if (*left <= 0 || !resident(c, &P)) return EPI_OK;
   ensure_posf(c);
   ResidentCfg rc{};
   rc.sync = c->res_sync;
+  rc.runs = &c->res_runs;
   c->status_h->flags = 0;
   const int own = (c->nprep_memb > 0 ? 1 : 0) + (c->nprep > c->nprep_memb ? 1 : 0) + 1;
   const bool skips = graph && conditional_rebuild(c);
@@ -393,15 +399,23 @@ int enqueue_resident(epi_ctx* c, const ResidentPlan& P, int32_t nsteps, bool gra
   rc.per_pair = graph ? 1 : 0;
   rc.per_rebuild = skips ? 5 : 0;
   // bounded runs: a kernel of a thousand steps lasts a few milliseconds
-  for (int32_t done = 0; done < nsteps;) {
-    const int32_t k = std::min(nsteps - done, 1024);
-    rc.run = c->res_run++;
-    rc.post = done + k == nsteps ? c->status_h : nullptr;
-    EPI_CUDA(launch_resident(make_state(c, c->cur), P, c->tissues_h[0], k, c->cfg.precision, rc,
-                             c->lc, c->stream));
+  while (*left > 0) {
+    const int32_t k = std::min(*left, 1024);
+    rc.post = k == *left ? c->status_h : nullptr;
+    const cudaError_t e = launch_resident(make_state(c, c->cur), P, c->tissues_h[0], k,
+                                          c->cfg.precision, rc, c->lc, c->stream);
+    if (e == cudaErrorCooperativeLaunchTooLarge) {
+      // a block per SM at once is more than the SMs at hand hold (a share of
+      // the GPU): the sequence from here on
+      (void)cudaGetLastError();
+      c->coop = 0;
+      return EPI_OK;
+    }
+    EPI_CUDA(e);
     c->cur ^= k & 1;
-    done += k;
+    *left -= k;
   }
+  if (posted) *posted = true;
   return EPI_OK;
 }
 
@@ -554,12 +568,8 @@ int check_status(epi_ctx* c, bool posted = false) {
 // an odd count.
 // *posted: see check_status.
 int enqueue_graph_steps(epi_ctx* c, int32_t nsteps, bool* posted = nullptr) {
-  ResidentPlan P;
-  if (nsteps > 0 && resident(c, &P)) {
-    c->lists_fresh = false;
-    if (posted) *posted = true;
-    return enqueue_resident(c, P, nsteps, true);
-  }
+  if (nsteps > 0) c->lists_fresh = false;
+  if (const int rc = enqueue_resident(c, &nsteps, true, posted)) return rc;
   ensure_posf(c);  // never inside the captured graph
   const int32_t pairs = nsteps / 2;
   if (pairs > 0) {
@@ -573,18 +583,13 @@ int enqueue_graph_steps(epi_ctx* c, int32_t nsteps, bool* posted = nullptr) {
     EPI_CUDA(cudaGraphLaunch(ge, c->stream));
   }
   if (nsteps % 2) enqueue_step(c, c->cur, nullptr);
-  if (nsteps > 0) c->lists_fresh = false;
   return EPI_OK;
 }
 
 // nsteps steps without a graph.
 int enqueue_steps(epi_ctx* c, int32_t nsteps, bool* posted = nullptr) {
   if (nsteps > 0) c->lists_fresh = false;
-  ResidentPlan P;
-  if (nsteps > 0 && resident(c, &P)) {
-    if (posted) *posted = true;
-    return enqueue_resident(c, P, nsteps, false);
-  }
+  if (const int rc = enqueue_resident(c, &nsteps, false, posted)) return rc;
   for (int32_t k = 0; k < nsteps; ++k) enqueue_step(c, c->cur, nullptr);
   return EPI_OK;
 }
@@ -1274,7 +1279,7 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
         if (c->cfg.precision == EPI_PREC_MIXED) launch_posf(Sh, c->lc, s);
         ResidentCfg rcfg{};
         rcfg.sync = c->res_sync;
-        rcfg.run = c->res_run++;
+        rcfg.runs = &c->res_runs;
         rcfg.hist = hist;
         EPI_CUDA(launch_resident(Sh, plan, c->tissues_h[0], len - 1, c->cfg.precision, rcfg, c->lc, s));
       }

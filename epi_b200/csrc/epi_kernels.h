@@ -1,6 +1,7 @@
 // Internal launch interface of the mechanics kernels (not part of the C ABI).
 #pragma once
 #include "epi_common.cuh"
+#include "epi_run_words.h"
 
 namespace epi {
 
@@ -70,9 +71,9 @@ void launch_step(const DevState& S, const Range& r, int precision, const LaunchC
 // (epi_resident.cu), candidate rebuilds included.
 constexpr int kResidentWords = 5;
 struct ResidentCfg {
-  int32_t* sync;      // device words: two barrier counts, used by runs in turn
-  uint32_t run;       // (each run clears the next one's), the abort flag, and
-                      // the two words of RunFlags
+  int32_t* sync;      // device words: two barrier counts (RunCount), the abort
+                      // flag, and the two words of RunFlags
+  RunCount* runs;     // of sync; counts this run once it is launched
   DevStatus* post;    // pinned host memory the status goes to at the end, with
                       // kStatusPosted among the flags; or null
   int32_t per_step, per_pair, per_rebuild;  // kernels of the sequence each step, each

@@ -30,7 +30,6 @@
 
 #include "epi_device.cuh"
 #include "epi_rebuild.cuh"
-#include "epi_run_words.h"
 #include "epi_step.cuh"
 
 namespace epi {
@@ -642,8 +641,8 @@ cudaError_t launch_resident(const DevState& S, const ResidentPlan& P, const Tiss
   A.terms = P.terms;
   A.group = P.group;
   A.thread_from = lc.search_switch;
-  A.bar = reinterpret_cast<unsigned*>(rc.sync) + (rc.run & 1);
-  A.other = reinterpret_cast<unsigned*>(rc.sync) + (~rc.run & 1);
+  A.bar = reinterpret_cast<unsigned*>(rc.sync) + rc.runs->own();
+  A.other = reinterpret_cast<unsigned*>(rc.sync) + rc.runs->next();
   A.abort = rc.sync + 2;
   A.flags = rc.sync + 3;
   A.post = rc.post;
@@ -654,8 +653,10 @@ cudaError_t launch_resident(const DevState& S, const ResidentPlan& P, const Tiss
   DevState S1 = S;
   TissueDev T0 = first;
   void* args[] = {&S1, &A, &T0};
-  return cudaLaunchCooperativeKernel(kernel, dim3((unsigned)P.grid), dim3((unsigned)kThreads), args,
-                                     (size_t)P.smem, s);
+  e = cudaLaunchCooperativeKernel(kernel, dim3((unsigned)P.grid), dim3((unsigned)kThreads), args,
+                                  (size_t)P.smem, s);
+  if (e == cudaSuccess) ++rc.runs->launched;
+  return e;
 }
 
 }  // namespace epi

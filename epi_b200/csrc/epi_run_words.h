@@ -36,4 +36,15 @@ struct RunFlags {
   }
 };
 
+// Barrier counts of runs that follow each other on a stream: two words, both
+// zero at first. A run counts arrivals in its own, which must be zero when it
+// starts, and clears the other for the next run as it starts itself. So the
+// words change over only when a run was launched: after a refused launch the
+// next run still finds the word that the last one cleared.
+struct RunCount {
+  uint32_t launched = 0;
+  EPI_HD int own() const { return (int)(launched & 1u); }
+  EPI_HD int next() const { return own() ^ 1; }
+};
+
 }  // namespace epi

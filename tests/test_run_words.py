@@ -4,8 +4,6 @@ interleaving of their reads, writes and barrier arrivals is walked."""
 import subprocess
 from pathlib import Path
 
-import pytest
-
 CSRC = Path(__file__).resolve().parents[1] / "epi_b200" / "csrc"
 
 
@@ -97,3 +95,30 @@ int main() {
 
 def test_blocks_agree_on_rebuilds_in_every_interleaving(tmp_path):
     subprocess.run([str(build(tmp_path, FLAGS))], check=True, timeout=300)
+
+
+# Runs on a stream: some launches are refused, the others add their arrivals to
+# their own word and clear the next one. Exits 0 when every run finds zero.
+RUNS = r"""
+#include <cstdio>
+#include "epi_run_words.h"
+int main() {
+  for (unsigned refused = 0; refused < 1u << 12; ++refused) {
+    epi::RunCount runs;
+    unsigned word[2] = {0, 0};
+    for (int k = 0; k < 12; ++k) {
+      const int own = runs.own(), next = runs.next();
+      if (own == next || word[own] != 0) return 1;
+      if (refused >> k & 1) continue;
+      ++runs.launched;
+      word[next] = 0;
+      word[own] += 148 * (1 + k);
+    }
+  }
+  return 0;
+}
+"""
+
+
+def test_a_refused_launch_leaves_the_next_run_a_zero_barrier_word(tmp_path):
+    subprocess.run([str(build(tmp_path, RUNS))], check=True, timeout=60)
