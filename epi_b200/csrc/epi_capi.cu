@@ -145,6 +145,7 @@ struct epi_ctx {
   unsigned long long* launches = nullptr;  // step-sequence kernels executed
   int32_t* res_sync = nullptr;   // words of the resident kernel (ResidentCfg::sync)
   RunCount res_runs;             // its runs so far
+  uint32_t res_sized = 0;        // its kernels whose shared memory limit is set
   int coop = 0;                  // the device takes cooperative launches
   unsigned char* adj_mem = nullptr;  // epi_adjoint's block (AdjointArena)
   size_t adj_bytes = 0;
@@ -392,6 +393,7 @@ int enqueue_resident(epi_ctx* c, int32_t* left, bool graph, bool* posted) {
   ResidentCfg rc{};
   rc.sync = c->res_sync;
   rc.runs = &c->res_runs;
+  rc.sized = &c->res_sized;
   c->status_h->flags = 0;
   const int own = (c->nprep_memb > 0 ? 1 : 0) + (c->nprep > c->nprep_memb ? 1 : 0) + 1;
   const bool skips = graph && conditional_rebuild(c);
@@ -1280,6 +1282,7 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
         ResidentCfg rcfg{};
         rcfg.sync = c->res_sync;
         rcfg.runs = &c->res_runs;
+        rcfg.sized = &c->res_sized;
         rcfg.hist = hist;
         EPI_CUDA(launch_resident(Sh, plan, c->tissues_h[0], len - 1, c->cfg.precision, rcfg, c->lc, s));
       }

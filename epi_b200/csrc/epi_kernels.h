@@ -74,6 +74,7 @@ struct ResidentCfg {
   int32_t* sync;      // device words: two barrier counts (RunCount), the abort
                       // flag, and the two words of RunFlags
   RunCount* runs;     // of sync; counts this run once it is launched
+  uint32_t* sized;    // kernels whose shared memory limit the context has set
   DevStatus* post;    // pinned host memory the status goes to at the end, with
                       // kStatusPosted among the flags; or null
   int32_t per_step, per_pair, per_rebuild;  // kernels of the sequence each step, each

@@ -542,16 +542,21 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   }
 }
 
-// Kernel of a batch's form.
+// Kernel of a batch's form, and the form's number (0 to 11).
 constexpr int kThreads = 512;
 template <typename R, bool kOne>
-const void* kernel_of(const LaunchCfg& lc) {
-  if (lc.simple && lc.any_old) return (const void*)k_resident<R, true, true, kOne, kThreads, 1>;
-  if (lc.simple) return (const void*)k_resident<R, true, false, kOne, kThreads, 1>;
+const void* kernel_of(const LaunchCfg& lc, int* form) {
+  const int kind = lc.simple ? (lc.any_old ? 1 : 0) : 2;
+  *form = kind + (kOne ? 3 : 0) + (sizeof(R) == 4 ? 6 : 0);
+  if (kind == 1) return (const void*)k_resident<R, true, true, kOne, kThreads, 1>;
+  if (kind == 0) return (const void*)k_resident<R, true, false, kOne, kThreads, 1>;
   return (const void*)k_resident<R, false, true, kOne, kThreads, 1>;
 }
 
-constexpr size_t kSmemPerBlock = 216 * 1024;  // of 227 KB, less the static parts
+// Of 227 KB, less the static parts. The limit that every kernel is given,
+// whatever a plan needs of it: the attribute belongs to the kernel, not to a
+// context, so contexts in other threads may be between setting and launching.
+constexpr size_t kSmemPerBlock = 216 * 1024;
 constexpr int kLeastSlots = 16;
 // pair terms per slot a block must have room for: all of a step's at unit
 // density, a part of them for batches of every cell state, whose membrane rows
@@ -627,11 +632,17 @@ cudaError_t launch_resident(const DevState& S, const ResidentPlan& P, const Tiss
                             int32_t nsteps, int precision, const ResidentCfg& rc,
                             const LaunchCfg& lc, cudaStream_t s) {
   const bool one = S.ntissues == 1;
-  const void* kernel = precision == 1 ? (one ? kernel_of<float, true>(lc) : kernel_of<float, false>(lc))
-                                      : (one ? kernel_of<double, true>(lc) : kernel_of<double, false>(lc));
-  cudaError_t e =
-      cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, P.smem);
-  if (e != cudaSuccess) return e;
+  int form;
+  const void* kernel =
+      precision == 1 ? (one ? kernel_of<float, true>(lc, &form) : kernel_of<float, false>(lc, &form))
+                     : (one ? kernel_of<double, true>(lc, &form) : kernel_of<double, false>(lc, &form));
+  cudaError_t e = cudaSuccess;
+  if (!(*rc.sized >> form & 1u)) {  // once per context and form: a driver call
+    e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kSmemPerBlock);
+    if (e != cudaSuccess) return e;
+    *rc.sized |= 1u << form;
+  }
   ResidentArgs A;
   A.nsteps = nsteps;
   A.slots = P.slots;
