@@ -146,7 +146,8 @@ struct Slots {
   int32_t* off;     // slots + 1: first pair task of each slot
   int32_t* at;      // membrane slot: its place in list
   int32_t* list;    // slots of membrane particles
-  int32_t* jk;      // their lattice column and row (16 bits each)
+  uint32_t* jk;     // their lattice column and row (16 bits each: a membrane is three
+                    // wide or more, so of kResidentParticles it has under 65,536 rows)
   uint32_t* task;   // pair tasks: partner (global index, 20 bits) | slot << 20
   static constexpr bool kOwn = sizeof(R) == 4;
   // terms: bending threads per membrane particle (kTriTerms, or with square
@@ -177,7 +178,7 @@ struct Slots {
     off = reinterpret_cast<int32_t*>(attr + slots);
     at = off + slots + 1;
     list = at + slots;
-    jk = list + membs;
+    jk = reinterpret_cast<uint32_t*>(list + membs);
     task = reinterpret_cast<uint32_t*>(jk + membs);
   }
 };
@@ -284,7 +285,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
       const TissueDev& T = kOne ? T0 : S0.tissues[attr_tissue(a)];
       const int32_t j = i - T.pbase, at = atomicAdd(&s_nm, 1);
       K.list[at] = s;
-      K.jk[at] = j % T.nmx | (j / T.nmx) << 16;
+      K.jk[at] = (uint32_t)(j % T.nmx) | (uint32_t)(j / T.nmx) << 16;
       K.at[s] = at;
     }
   }
@@ -427,8 +428,8 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
           const TissueDev& T = tissue(K.attr[slot]);
           const bool tri = T.lattice == kLatticeTriangular;
           const SiteOffsets<R> off(S, K.own[slot], T);
-          const int32_t jk = in ? K.jk[m0 + m] : 0;
-          const MembSites M(T, i, jk & 0xffff, jk >> 16);
+          const uint32_t jk = in ? K.jk[m0 + m] : 0u;
+          const MembSites M(T, i, (int32_t)(jk & 0xffffu), (int32_t)(jk >> 16));
           if (spring) {
             if (!in) continue;
             if (e == kMembAdjTri) {  // the wall
@@ -557,6 +558,7 @@ const void* kernel_of(const LaunchCfg& lc, int* form) {
 // whatever a plan needs of it: the attribute belongs to the kernel, not to a
 // context, so contexts in other threads may be between setting and launching.
 constexpr size_t kSmemPerBlock = 216 * 1024;
+static_assert(kResidentParticles / 3 < 65536, "rows of a membrane fit 16 bits");
 constexpr int kLeastSlots = 16;
 // pair terms per slot a block must have room for: all of a step's at unit
 // density, a part of them for batches of every cell state, whose membrane rows
