@@ -260,14 +260,18 @@ __device__ __forceinline__ F2 xfma(F2 a, F2 b, F2 c) {
 // FP64 path: the distance sqrt(d2) and 1 / d2 from i = 1 / sqrt(d2), each
 // corrected to within an ulp, as a square root and a division would give
 // (the laws subtract nearly equal numbers, so it would show). One rsqrt and
-// four multiply-adds stand for a square root and two divisions.
+// four multiply-adds stand for a square root and two divisions. Cells at one
+// place (d2 = 0, i infinite) get what those give, 0 and infinity, so that the
+// coefficient comes out infinite and is reported: the correction alone would
+// make it NaN, which passes the reference's test of its size.
 __device__ __forceinline__ double dist_of(double d2, double i) {
   const double d = xmul(d2, i);
-  return xfma(xmul(0.5, i), xfma(-d, d, d2), d);
+  return d2 > 0.0 ? xfma(xmul(0.5, i), xfma(-d, d, d2), d) : d2;
 }
 __device__ __forceinline__ double inv_sq(double d2, double i) {
   const double v = xmul(i, i);
-  return xfma(v, xfma(-d2, v, 1.0), v);
+  // (v is not negative: infinite or NaN from this high word on)
+  return __double2hiint(v) < 0x7ff00000 ? xfma(v, xfma(-d2, v, 1.0), v) : v;
 }
 
 template <typename R>
