@@ -46,7 +46,7 @@ EXPORTED = [
     "epi_step_per_tissue", "epi_sync", "epi_num_particles", "epi_download_positions",
     "epi_upload_positions", "epi_step_host", "epi_step_host_async", "epi_get_connections", "epi_get_dermis", "epi_error_info",
     "epi_stream", "epi_rebuild_count", "epi_launch_count", "epi_time_kernels", "epi_autotune",
-    "epi_get_config", "epi_set_tuning", "epi_field_init",
+    "epi_get_config", "epi_set_tuning", "epi_set_wait_limit", "epi_field_init",
     "epi_field_step", "epi_field_get", "epi_field_set_ext", "epi_adjoint", "epi_connect_noalloc",
 ]
 
@@ -143,6 +143,7 @@ def lib():
         L.epi_get_config.argtypes = [vp, ctypes.POINTER(ConfigC)]
         L.epi_set_tuning.argtypes = [vp, ctypes.c_double, ctypes.c_int32, ctypes.c_int32,
                                      ctypes.c_int32]
+        L.epi_set_wait_limit.argtypes = [vp, ctypes.c_int32]
         L.epi_field_init.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, ctypes.c_int32]
         L.epi_field_step.argtypes = [vp, ctypes.c_int32]
         L.epi_field_get.argtypes = [vp, ctypes.c_int32, _ip, _up, _dp, _dp]
@@ -397,6 +398,10 @@ class Context:
         """epi_set_tuning: apply a tuning chosen earlier (e.g. cached)."""
         _check(lib().epi_set_tuning(self._h, float(skin), int(variant), int(search_switch),
                                     int(rebuild_gate)), "epi_set_tuning")
+
+    def set_wait_limit(self, polls: int = 0):
+        """epi_set_wait_limit: polls of a wait between blocks before it gives up."""
+        _check(lib().epi_set_wait_limit(self._h, int(polls)), "epi_set_wait_limit")
 
     def autotune(self, trial_steps: int = 64):
         """epi_autotune: returns (skin, variant, ms per step of the best trial)

@@ -70,6 +70,9 @@ constexpr int kHostStepGroups = 4;
 // Rebuilt particles from which the candidate search takes one thread per
 // particle (epi_config.search_switch = 0).
 constexpr int kDefaultSearchSwitch = 48 * 1024;
+// Polls of a wait between blocks before it gives up (epi_set_wait_limit):
+// seconds.
+constexpr int32_t kDefaultPolls = 1 << 23;
 
 // Host-side bookkeeping of one tissue in the batch.
 struct TissueHost {
@@ -147,6 +150,7 @@ struct epi_ctx {
   RunCount res_runs;             // its runs so far
   uint32_t res_sized = 0;        // its kernels whose shared memory limit is set
   int coop = 0;                  // the device takes cooperative launches
+  int32_t polls = kDefaultPolls;  // of a wait in a kernel before it gives up
   unsigned char* adj_mem = nullptr;  // epi_adjoint's block (AdjointArena)
   size_t adj_bytes = 0;
   ScanScratch scan{};
@@ -394,6 +398,7 @@ int enqueue_resident(epi_ctx* c, int32_t* left, bool graph, bool* posted) {
   rc.sync = c->res_sync;
   rc.runs = &c->res_runs;
   rc.sized = &c->res_sized;
+  rc.polls = c->polls;
   c->status_h->flags = 0;
   const int own = (c->nprep_memb > 0 ? 1 : 0) + (c->nprep > c->nprep_memb ? 1 : 0) + 1;
   const bool skips = graph && conditional_rebuild(c);
@@ -557,6 +562,10 @@ int check_status(epi_ctx* c, bool posted = false) {
   if (c->status_h->code != 0) {
     c->last = *c->status_h;
     c->last.flags &= ~kStatusPosted;
+    // Blocks that gave up waiting left in the middle of a step or a rebuild:
+    // positions, bin counts and candidate rows are between two states. Only an
+    // upload starts from here, and one that takes nothing over.
+    if (c->last.flags & (1 << E_TIMEOUT)) c->loaded = false;
     EPI_CUDA(cudaMemsetAsync(c->status, 0, sizeof(DevStatus), c->stream));
     EPI_CUDA(cudaMemsetAsync(c->res_sync, 0, kResidentWords * sizeof(int32_t), c->stream));
     EPI_CUDA(cudaStreamSynchronize(c->stream));
@@ -1283,6 +1292,7 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
         rcfg.sync = c->res_sync;
         rcfg.runs = &c->res_runs;
         rcfg.sized = &c->res_sized;
+        rcfg.polls = c->polls;
         rcfg.hist = hist;
         EPI_CUDA(launch_resident(Sh, plan, c->tissues_h[0], len - 1, c->cfg.precision, rcfg, c->lc, s));
       }
@@ -1554,7 +1564,9 @@ int epi_autotune(epi_ctx* c, int32_t trial_steps, double* skin_out, int32_t* var
     EPI_CUDA(cudaEventRecord(ev[1], s));
     *ms_out = INFINITY;
     // a skin whose candidate rows overflow max_cand fails here: skip it
-    if (check_status(c) != EPI_OK) return EPI_OK;
+    const int failed = check_status(c);
+    if (!c->loaded) return failed;  // a wait gave up: nothing to restore into
+    if (failed != EPI_OK) return EPI_OK;
     float ms = 0;
     EPI_CUDA(cudaEventElapsedTime(&ms, ev[0], ev[1]));
     *ms_out = ms;
@@ -1633,6 +1645,12 @@ int epi_set_tuning(epi_ctx* c, double skin, int32_t variant, int32_t search_swit
   }
   return EPI_OK;
   EPI_GUARD_END
+}
+
+int epi_set_wait_limit(epi_ctx* c, int32_t polls) {
+  if (!c || polls < 0) return EPI_ERR_INVALID_ARG;
+  c->polls = polls > 0 ? polls : kDefaultPolls;
+  return EPI_OK;
 }
 
 int epi_step_per_tissue(epi_ctx* c, int32_t nsteps) {

@@ -75,6 +75,7 @@ struct ResidentCfg {
                       // flag, and the two words of RunFlags
   RunCount* runs;     // of sync; counts this run once it is launched
   uint32_t* sized;    // kernels whose shared memory limit the context has set
+  int32_t polls;      // of a barrier wait before it gives up
   DevStatus* post;    // pinned host memory the status goes to at the end, with
                       // kStatusPosted among the flags; or null
   int32_t per_step, per_pair, per_rebuild;  // kernels of the sequence each step, each

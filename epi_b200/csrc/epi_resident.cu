@@ -51,20 +51,19 @@ struct ResidentArgs {
   unsigned* other;          // the next run's (zeroed here)
   int32_t* abort;           // set when a barrier wait gave up
   int32_t* flags;           // RunFlags::words
+  int32_t polls;            // limit of a barrier wait
   DevStatus* post;          // non-null: pinned host memory the status is put in
   int32_t per_step, per_pair, per_rebuild;  // launches counted (see epi_launch_count)
   double4* hist;            // non-null: step k's positions go to hist + k n_total
 };
 
-// Waits of thread 0 of every block; a wait that is not met in kSpinLimit
-// polls (seconds) gives up: the error is recorded and every block leaves at
-// its next check.
-constexpr int kSpinLimit = 1 << 23;
-
+// Waits of thread 0 of every block; a wait that is not met within the limit
+// gives up: the error is recorded and every block leaves at its next check.
 struct GridBarrier {
   unsigned* bar;
   int32_t* abort;
   DevStatus* status;
+  int32_t limit;  // polls
   unsigned target;
   // word: read by thread 0 after the barrier and returned to all threads of
   // the block (the same value in every block: see RunFlags). False: some
@@ -83,8 +82,8 @@ struct GridBarrier {
       for (;;) {
         asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
         if ((int32_t)(seen - target) >= 0) break;
-        if (++spins >= kSpinLimit || ((spins & 1023) == 0 && *(volatile int32_t*)abort)) {
-          if (spins >= kSpinLimit) {
+        if (++spins >= limit || ((spins & 1023) == 0 && *(volatile int32_t*)abort)) {
+          if (spins >= limit) {
             raise_error(status, E_TIMEOUT, (int32_t)blockIdx.x, -1, (double)seen);
             *(volatile int32_t*)abort = 1;
           }
@@ -250,7 +249,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   DevState S = S0;
   if (A.hist) S.pos_cur = A.hist;
   if (A.hist) S.pos_nxt = A.hist + n;
-  GridBarrier B{A.bar, A.abort, S0.status, 0u};
+  GridBarrier B{A.bar, A.abort, S0.status, A.polls, 0u};
   unsigned long long counted = 0;
   const RunFlags flags{S0.gate, A.flags};
   int32_t flagged = *(volatile const int32_t*)flags.read_by(0);
@@ -658,6 +657,7 @@ cudaError_t launch_resident(const DevState& S, const ResidentPlan& P, const Tiss
   A.other = reinterpret_cast<unsigned*>(rc.sync) + rc.runs->next();
   A.abort = rc.sync + 2;
   A.flags = rc.sync + 3;
+  A.polls = rc.polls;
   A.post = rc.post;
   A.per_step = rc.per_step;
   A.per_pair = rc.per_pair;

@@ -47,7 +47,8 @@ typedef enum epi_status {
   EPI_ERR_COEF_RANGE = 8,       /* |pair coefficient| > 1000: cell_interaction.cpp:51-55 */
   EPI_ERR_MEMB_COEF_RANGE = 9,  /* |membrane coefficient| > 100: cell_interaction.cpp:200-231 */
   EPI_ERR_NONFINITE = 10,       /* a position became NaN or infinite */
-  EPI_ERR_TIMEOUT = 11,         /* a bounded device-side wait gave up */
+  EPI_ERR_TIMEOUT = 11,         /* a bounded device-side wait gave up (epi_set_wait_limit); the
+                                   context must be uploaded to again */
   EPI_ERR_STATE = 12,           /* call out of order (e.g. step before upload) */
   EPI_ERR_UNSUPPORTED = 13,     /* geometry outside what the library implements */
   EPI_ERR_CHECK = 14            /* an index check of the bounds-checked build failed
@@ -169,6 +170,12 @@ int epi_step_graph(epi_ctx* ctx, int32_t nsteps);
 /* Same as epi_step, but one kernel sequence per tissue and no graph: the
  * unbatched launch pattern, kept as the comparison point for batching. */
 int epi_step_per_tissue(epi_ctx* ctx, int32_t nsteps);
+/* The blocks of a small batch's resident kernel wait for each other between
+ * steps. Such a wait is bounded: after this many polls (0 = the default, 2^23,
+ * which takes seconds) it gives up, the call that reports it returns
+ * EPI_ERR_TIMEOUT, and steps return EPI_ERR_STATE until the next epi_upload,
+ * since the run ended between two states. No counterpart in the reference. */
+int epi_set_wait_limit(epi_ctx* ctx, int32_t polls);
 /* Waits for queued work and reports any kernel-side error. */
 int epi_sync(epi_ctx* ctx);
 
