@@ -493,7 +493,7 @@ def main():
     if args.warmup:
         ctx.step(args.warmup, args.mode)
     rebuilds0 = ctx.rebuild_count()
-    launches0 = ctx.launch_count()
+    launches0 = ctx.kernels_run()
     torch.cuda.synchronize()
     barrier()
     torch.cuda.synchronize()
@@ -508,7 +508,7 @@ def main():
     barrier()
     ms = e0.elapsed_time(e1)
     rebuilds_timed = ctx.rebuild_count() - rebuilds0
-    launches_timed = ctx.launch_count() - launches0
+    launches_timed = ctx.kernels_run() - launches0
     if dist is not None:
         t = torch.tensor([ms], device="cuda", dtype=torch.float64)
         dist.all_reduce(t, op=dist.ReduceOp.MAX)

@@ -45,7 +45,7 @@ EXPORTED = [
     "epi_upload", "epi_connect", "epi_interact_commit", "epi_step", "epi_step_graph",
     "epi_step_per_tissue", "epi_sync", "epi_num_particles", "epi_download_positions",
     "epi_upload_positions", "epi_step_host", "epi_step_host_async", "epi_get_connections", "epi_get_dermis", "epi_error_info",
-    "epi_stream", "epi_rebuild_count", "epi_launch_count", "epi_time_kernels", "epi_autotune",
+    "epi_stream", "epi_rebuild_count", "epi_launch_count", "epi_resident_count", "epi_time_kernels", "epi_autotune",
     "epi_get_config", "epi_set_tuning", "epi_set_wait_limit", "epi_field_init",
     "epi_field_step", "epi_field_get", "epi_field_set_ext", "epi_adjoint", "epi_connect_noalloc",
 ]
@@ -135,6 +135,8 @@ def lib():
         L.epi_error_info.argtypes = [vp, _ip, _ip, _ip, _dp]
         L.epi_rebuild_count.argtypes = [vp, ctypes.POINTER(ctypes.c_int64)]
         L.epi_launch_count.argtypes = [vp, ctypes.POINTER(ctypes.c_int64)]
+        L.epi_resident_count.argtypes = [vp, ctypes.POINTER(ctypes.c_int64),
+                                         ctypes.POINTER(ctypes.c_int64)]
         L.epi_stream.argtypes = [vp]
         L.epi_stream.restype = vp
         L.epi_time_kernels.argtypes = [vp, ctypes.c_int32, ctypes.c_int32, _dp, _ip,
@@ -356,6 +358,20 @@ class Context:
         v = ctypes.c_int64()
         _check(lib().epi_launch_count(self._h, ctypes.byref(v)), "epi_launch_count")
         return int(v.value)
+
+    def resident_count(self):
+        """epi_resident_count: (resident kernels run, kernels of the step sequence
+        that launch_count() counts for them)."""
+        runs, stood_for = ctypes.c_int64(), ctypes.c_int64()
+        _check(lib().epi_resident_count(self._h, ctypes.byref(runs), ctypes.byref(stood_for)),
+               "epi_resident_count")
+        return int(runs.value), int(stood_for.value)
+
+    def kernels_run(self) -> int:
+        """Kernels of the step path that ran: launch_count() with a resident run
+        counted as the one kernel it is."""
+        runs, stood_for = self.resident_count()
+        return self.launch_count() - stood_for + runs
 
     def stream_handle(self) -> int:
         return int(lib().epi_stream(self._h) or 0)

@@ -145,7 +145,7 @@ struct epi_ctx {
   size_t upin_bytes = 0;
   unsigned long long* rebuilds = nullptr;
   int32_t* loop_left = nullptr;  // passes left in the step graph's device loop
-  unsigned long long* launches = nullptr;  // step-sequence kernels executed
+  unsigned long long* launches = nullptr;  // see DevState
   int32_t* res_sync = nullptr;   // words of the resident kernel (ResidentCfg::sync)
   RunCount res_runs;             // its runs so far
   uint32_t res_sized = 0;        // its kernels whose shared memory limit is set
@@ -385,26 +385,31 @@ bool resident(const epi_ctx* c, ResidentPlan* P) {
 
 bool conditional_rebuild(const epi_ctx* c);
 
-// The next *left steps in the resident kernel, if the batch steps there; *left
-// comes back as what remains for the kernel sequence (all or nothing, unless
-// the device stops taking the launches). graph: what the launch count stands
-// for, the replayed graph or the eager sequence (see epi_launch_count).
-// *posted: see check_status.
-int enqueue_resident(epi_ctx* c, int32_t* left, bool graph, bool* posted) {
-  ResidentPlan P;
-  if (*left <= 0 || !resident(c, &P)) return EPI_OK;
-  ensure_posf(c);
+// A resident run's words, limits and counts. graph: what the launch count
+// stands for, the replayed graph or the eager sequence (see epi_launch_count).
+ResidentCfg resident_cfg(epi_ctx* c, bool graph) {
   ResidentCfg rc{};
   rc.sync = c->res_sync;
   rc.runs = &c->res_runs;
   rc.sized = &c->res_sized;
   rc.polls = c->polls;
-  c->status_h->flags = 0;
   const int own = (c->nprep_memb > 0 ? 1 : 0) + (c->nprep > c->nprep_memb ? 1 : 0) + 1;
   const bool skips = graph && conditional_rebuild(c);
   rc.per_step = own + (skips ? 1 : 6);
   rc.per_pair = graph ? 1 : 0;
   rc.per_rebuild = skips ? 5 : 0;
+  return rc;
+}
+
+// The next *left steps in the resident kernel, if the batch steps there; *left
+// comes back as what remains for the kernel sequence (all or nothing, unless
+// the device stops taking the launches). *posted: see check_status.
+int enqueue_resident(epi_ctx* c, int32_t* left, bool graph, bool* posted) {
+  ResidentPlan P;
+  if (*left <= 0 || !resident(c, &P)) return EPI_OK;
+  ensure_posf(c);
+  ResidentCfg rc = resident_cfg(c, graph);
+  c->status_h->flags = 0;
   // bounded runs: a kernel of a thousand steps lasts a few milliseconds
   while (*left > 0) {
     const int32_t k = std::min(*left, 1024);
@@ -905,10 +910,10 @@ int epi_create(epi_ctx** out, const epi_config* cfg) {
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->status, 0, sizeof(DevStatus)));
   if (rc == EPI_OK) rc = dev_alloc(&ctx->rebuilds, 1);
   if (rc == EPI_OK) rc = dev_alloc(&ctx->loop_left, 1);
-  if (rc == EPI_OK) rc = dev_alloc(&ctx->launches, 1);
+  if (rc == EPI_OK) rc = dev_alloc(&ctx->launches, 3);
   if (rc == EPI_OK) rc = dev_alloc(&ctx->res_sync, kResidentWords);
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->res_sync, 0, kResidentWords * sizeof(int32_t)));
-  if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->launches, 0, sizeof(unsigned long long)));
+  if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->launches, 0, 3 * sizeof(unsigned long long)));
   if (rc == EPI_OK) rc = cuda_status(cudaMemset(ctx->rebuilds, 0, sizeof(unsigned long long)));
   if (rc != EPI_OK) {
     epi_destroy(ctx);
@@ -1288,11 +1293,7 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
       launch_gate_check(Sh, c->lc, s);
       if (len > 1) {
         if (c->cfg.precision == EPI_PREC_MIXED) launch_posf(Sh, c->lc, s);
-        ResidentCfg rcfg{};
-        rcfg.sync = c->res_sync;
-        rcfg.runs = &c->res_runs;
-        rcfg.sized = &c->res_sized;
-        rcfg.polls = c->polls;
+        ResidentCfg rcfg = resident_cfg(c, false);
         rcfg.hist = hist;
         EPI_CUDA(launch_resident(Sh, plan, c->tissues_h[0], len - 1, c->cfg.precision, rcfg, c->lc, s));
       }
@@ -1985,6 +1986,20 @@ int epi_launch_count(epi_ctx* c, int64_t* count) {
   EPI_CUDA(cudaMemcpyAsync(&v, c->launches, sizeof(v), cudaMemcpyDeviceToHost, c->stream));
   EPI_CUDA(cudaStreamSynchronize(c->stream));
   *count = (int64_t)v;
+  return EPI_OK;
+  EPI_GUARD_END
+}
+
+int epi_resident_count(epi_ctx* c, int64_t* runs, int64_t* stood_for) {
+  if (!c || !runs || !stood_for) return EPI_ERR_INVALID_ARG;
+  EPI_GUARD_BEGIN
+  int rc = set_device(c);
+  if (rc) return rc;
+  unsigned long long v[2] = {0, 0};
+  EPI_CUDA(cudaMemcpyAsync(v, c->launches + 1, sizeof(v), cudaMemcpyDeviceToHost, c->stream));
+  EPI_CUDA(cudaStreamSynchronize(c->stream));
+  *runs = (int64_t)v[0];
+  *stood_for = (int64_t)v[1];
   return EPI_OK;
   EPI_GUARD_END
 }

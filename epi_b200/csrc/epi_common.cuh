@@ -113,7 +113,9 @@ struct DevState {
   int32_t nprep, nprep_memb;
   DevStatus* status;
   unsigned long long* rebuilds;  // tissue candidate rebuilds so far
-  unsigned long long* launches;  // kernels of the step sequence executed so far
+  // [0] kernels of the step sequence executed so far, [1] resident runs,
+  // [2] kernels of the sequence that those stand for (counted in [0] too)
+  unsigned long long* launches;
   int64_t n_total;  // column stride of cand / nbr
   int32_t max_conn, max_cand;
   double skin;

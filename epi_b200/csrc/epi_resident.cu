@@ -53,7 +53,7 @@ struct ResidentArgs {
   int32_t* flags;           // RunFlags::words
   int32_t polls;            // limit of a barrier wait
   DevStatus* post;          // non-null: pinned host memory the status is put in
-  int32_t per_step, per_pair, per_rebuild;  // launches counted (see epi_launch_count)
+  int32_t per_step, per_pair, per_rebuild;  // kernels stood for (see ResidentCfg)
   double4* hist;            // non-null: step k's positions go to hist + k n_total
 };
 
@@ -527,7 +527,11 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
   }
   if (blockIdx.x == 0 && tid == 0) {
     if (done) flags.hand_on(A.nsteps);
-    if (S0.launches) atomicAdd(S0.launches, counted);
+    if (S0.launches) {
+      atomicAdd(S0.launches, counted);
+      atomicAdd(S0.launches + 1, 1ull);
+      atomicAdd(S0.launches + 2, counted);
+    }
     // past the last barrier every block has raised what it had to: the host
     // finds the status after its wait for the stream, without a copy
     if (A.post && done) {

@@ -223,9 +223,14 @@ int epi_rebuild_count(epi_ctx* ctx, int64_t* count);
 /* Kernels of the step sequence (rebuild, membrane prepass, dermis, step, and
  * the graph's condition and loop kernels) executed on the device since the
  * context was created, counted by the kernels themselves; kernels a graph's
- * conditional node skipped are not counted. Small batches run their steps in
- * one resident kernel, whose phases count as the kernels they stand for. */
+ * conditional node skipped are not counted. The phases of a small batch's
+ * resident kernel count as the kernels they stand for: epi_resident_count
+ * tells how many those are. */
 int epi_launch_count(epi_ctx* ctx, int64_t* count);
+/* Resident kernels executed since the context was created, and the kernels of
+ * the step sequence that epi_launch_count counts for them: kernels that ran
+ * are epi_launch_count's number - stood_for + runs. */
+int epi_resident_count(epi_ctx* ctx, int64_t* runs, int64_t* stood_for);
 /* Per-kernel timing: runs nsteps (not graph-captured) recording CUDA events
  * around each kernel class on the context stream. ms receives the summed
  * milliseconds per class, launches the launch count per class, names the

@@ -44,6 +44,7 @@ def test_rows_beyond_15_bits(built, rows, lattice, precision):
         with capi.Context(precision=precision) as ctx:
             ctx.upload([t])
             ctx.step(STEPS, mode)
+            assert ctx.resident_count()[0] == (1 if mode == "eager" else 0)
             got.append(ctx.positions())
     for a, b in zip(*got):
         assert np.array_equal(a, b)
