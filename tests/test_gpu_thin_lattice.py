@@ -39,12 +39,14 @@ def thin(rows, lattice):
                                           (32800, T.TRIANGULAR), (43600, T.SQUARE)])
 def test_rows_beyond_15_bits(built, rows, lattice, precision):
     t = thin(rows, lattice)
+    # 43,600 rows' FP64 terms are beyond a block's shared memory: the sequence
+    fits = rows < 43600 or precision == capi.EPI_PREC_MIXED
     got = []
     for mode in ("eager", "per_tissue"):
         with capi.Context(precision=precision) as ctx:
             ctx.upload([t])
             ctx.step(STEPS, mode)
-            assert ctx.resident_count()[0] == (1 if mode == "eager" else 0)
+            assert ctx.resident_count()[0] == (1 if fits and mode == "eager" else 0)
             got.append(ctx.positions())
     for a, b in zip(*got):
         assert np.array_equal(a, b)
