@@ -473,7 +473,8 @@ def main():
             ctx.step(args.warmup, args.mode)
         from epi_b200.autotune import tuned as autotuned
         tuned = autotuned(ctx, mine, args.tune_steps, device=local, retune=args.retune)
-        tuned["grid"] = ("skin {0.05,0.08,0.1,0.15,0.2,0.3} x step-kernel variant 1..4, "
+        tuned["grid"] = ("skin {0.05,0.08,0.1,0.15,0.2,0.3} x step-kernel variant 1..4 "
+                         "(0, resident, too where the batch is small), "
                          "then rebuild node {conditional, always launched}, "
                          "then search switch {8192,16384,49152,131072}")
     off, _ = ctx.connections()
@@ -706,7 +707,7 @@ def main():
         cfg = {"workload": desc, "tissues": n_tissues_all, "particles": n_all,
                "mean_connections": kbar, "precision": args.precision,
                "skin": cfg_skin(tuned, args),
-               "variant": tuned["variant"] if tuned else (args.variant or 3),
+               "variant": ctx.config()["variant"],
                "search_switch": ctx.config()["search_switch"] or 49152,
                "autotune": tuned,
                "tissues_rebuilt_per_step": rebuilds_timed / max(args.steps, 1),

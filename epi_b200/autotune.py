@@ -7,7 +7,9 @@ shape up in a JSON cache first and applies a stored choice with
 epi_set_tuning, so repeated runs of one workload tune once.
 
 Key: precision, GPU name and SM count, tissue count, and a digest of every
-tissue's (particles, membrane particles, lattice, box).
+tissue's (particles, membrane particles, lattice, box). The "v2" before them:
+choices stored without it were made when a small batch's resident kernel ran
+whatever variant was named, so the variant they hold was not chosen by its time.
 """
 from __future__ import annotations
 
@@ -25,7 +27,7 @@ def shape_key(tissues: Sequence, precision: int, gpu: str) -> str:
     for t in tissues:
         h.update(f"{t.n},{t.nmemb},{getattr(t, 'lattice', 0)},{t.lx:.6g},{t.ly:.6g},"
                  f"{t.lz:.6g};".encode())
-    return f"p{precision}|{gpu}|{len(tissues)}|{h.hexdigest()[:16]}"
+    return f"v2|p{precision}|{gpu}|{len(tissues)}|{h.hexdigest()[:16]}"
 
 
 def gpu_name(device: int = 0) -> str:

@@ -377,10 +377,12 @@ void enqueue_step(epi_ctx* c, int& cur, Timer* tm) {
 }
 
 // Whether the batch steps in one resident kernel (epi_resident.cu) instead of
-// the kernel sequence; the results are the same bits.
+// the kernel sequence; the results are the same bits. A configuration that
+// names a step-kernel form or a rebuild node asks for the sequence.
 bool resident(const epi_ctx* c, ResidentPlan* P) {
-  return c->coop && resident_plan(c->tissues_h.data(), c->ntissues, c->n, c->cfg.precision,
-                                  c->cfg.max_cand, c->lc, P);
+  return c->coop && c->cfg.variant == 0 && c->cfg.rebuild_gate == 0 &&
+         resident_plan(c->tissues_h.data(), c->ntissues, c->n, c->cfg.precision,
+                       c->cfg.max_cand, c->lc, P);
 }
 
 bool conditional_rebuild(const epi_ctx* c);
@@ -1524,7 +1526,7 @@ int epi_autotune(epi_ctx* c, int32_t trial_steps, double* skin_out, int32_t* var
   int rc = set_device(c);
   if (rc) return rc;
   static const double kSkins[] = {0.05, 0.08, 0.1, 0.15, 0.2, 0.3};
-  static const int32_t kVariants[] = {1, 2, 3, 4};
+  static const int32_t kVariants[] = {0, 1, 2, 3, 4};
   constexpr int32_t kWarm = 4;  // the first step after a restore rebuilds every tissue
   const size_t pbytes = sizeof(double4) * (size_t)c->n;
   cudaStream_t s = c->stream;
@@ -1576,9 +1578,15 @@ int epi_autotune(epi_ctx* c, int32_t trial_steps, double* skin_out, int32_t* var
   double best = INFINITY, best_skin = c->cfg.skin;
   int32_t best_variant = c->cfg.variant;
   const int32_t switch0 = c->cfg.search_switch, form0 = c->cfg.rebuild_gate;
+  // A batch that steps resident (variant 0 and no node named) has that as one
+  // more form; in any other 0 is one of 1 to 4.
+  apply(best_skin, 0, switch0, 0);
+  ResidentPlan plan;
+  const bool small = resident(c, &plan);
   for (double skin : kSkins) {
     for (int32_t variant : kVariants) {
-      apply(skin, variant, switch0, form0);
+      if (variant == 0 && !small) continue;
+      apply(skin, variant, switch0, variant == 0 ? 0 : form0);
       double ms;
       if ((rc = trial(&ms))) return rc;
       if (ms < best) {
@@ -1590,9 +1598,11 @@ int epi_autotune(epi_ctx* c, int32_t trial_steps, double* skin_out, int32_t* var
   }
   // then the rebuild in a conditional graph node or not, and the candidate
   // search's switch from a warp to a thread per particle
-  int32_t best_form = form0, best_switch = switch0;
+  const bool sequence = !small || best_variant != 0;  // which has a node
+  int32_t best_form = sequence ? form0 : 0, best_switch = switch0;
   if (std::isfinite(best)) {
     for (int32_t form : {1, 2}) {
+      if (!sequence) break;
       apply(best_skin, best_variant, switch0, form);
       double ms;
       if ((rc = trial(&ms))) return rc;

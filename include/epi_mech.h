@@ -123,7 +123,9 @@ typedef struct epi_config {
                          extra); the reference allows 400 (define.h:80) */
   int32_t max_cand;   /* candidates per particle (>= max_conn) */
   double skin;        /* candidate margin, > 0 (default 0.1) */
-  int32_t variant;    /* step-kernel form: 0 = default (4; FP64: 3); 1, 2 = the
+  int32_t variant;    /* step-kernel form: 0 = default (a small batch in one
+                         resident kernel for a run of steps, see
+                         rebuild_gate; others 4, FP64: 3); 1, 2 = the
                          neighbours' positions copied asynchronously into
                          shared memory, 8 / 15 per thread at once (FP64: 4 /
                          8); 3, 4 = gathered into registers: four at a time
@@ -132,12 +134,16 @@ typedef struct epi_config {
                          arithmetic in every form. */
   int32_t search_switch; /* candidate search: rebuilds of at least this many
                          particles take one thread per particle, smaller ones
-                         one warp per particle; 0 = default (49152) */
+                         a warp or part of one; 0 = default (49152) */
   int32_t rebuild_gate; /* step graph: 0 = default (1 for a single tissue,
                          2 for a batch); 1 = the candidate rebuild's kernels
                          sit in a conditional node that skips them on steps
                          with nothing to rebuild; 2 = they are always launched
-                         (and exit at once when nothing is listed) */
+                         (and exit at once when nothing is listed). The
+                         resident kernel, which holds every SM for up to 1024
+                         steps, is taken with variant and rebuild_gate both 0;
+                         naming either keeps a small batch in the kernel
+                         sequence, between whose kernels other streams run */
   int32_t reserved;   /* must be 0 */
 } epi_config;
 
@@ -240,9 +246,10 @@ int epi_time_kernels(epi_ctx* ctx, int32_t nsteps, int32_t max_classes, double* 
 
 /* Autotuner. Times short graph-replayed trials of the uploaded batch for
  * every candidate skin in {0.05, 0.08, 0.1, 0.15, 0.2, 0.3} and step-kernel
- * variant 1..4 (4 warm-up steps, then trial_steps timed with CUDA events),
- * then, for the fastest pair, the rebuild in a conditional graph node or
- * not, and the candidate search's switch from a warp to a thread per
+ * variant 1..4, for a batch that steps resident 0 as well (4 warm-up steps,
+ * then trial_steps timed with CUDA events), then, for the fastest pair, the
+ * rebuild in a conditional graph node or not (not for the resident kernel,
+ * which has none), and the candidate search's switch from a warp to a thread per
  * particle in {8192, 16384, 49152, 131072} rebuilt particles, and keeps the
  * fastest choice in the context's configuration. Skins whose candidate rows would overflow
  * max_cand are skipped. The simulation state is left as it was (positions

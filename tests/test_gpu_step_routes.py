@@ -34,3 +34,38 @@ def test_a_batch_that_fills_the_gpu_steps_in_the_sequence(built):
     with capi.Context(precision=MIXED) as ctx:
         ctx.upload(ts)
         assert counted(ctx, 2, "eager") == (16, 0, 0)
+
+
+@pytest.mark.parametrize("precision", [FP64, MIXED])
+@pytest.mark.parametrize("named", [dict(variant=v) for v in (1, 2, 3, 4)] +
+                         [dict(rebuild_gate=g) for g in (1, 2)])
+def test_a_named_form_is_the_one_that_runs(built, named, precision):
+    """A variant or a rebuild node in the configuration keeps a small batch in
+    the kernel sequence, eager and graph; the results are the same bits."""
+    ts = [T.mixed_state_tissue(2), T.layered_tissue(16, 2, 1), T.tri_layered_tissue(16, 18, 2, 0)]
+    got = []
+    for cfg in ({}, named):
+        with capi.Context(precision=precision, skin=0.05, max_conn=96, max_cand=192, **cfg) as ctx:
+            ctx.upload(ts)
+            runs = [counted(ctx, 15, mode)[1] for mode in ("eager", "graph")]
+            assert runs == ([0, 0] if cfg else [1, 1])
+            got.append(ctx.positions() + ctx.connections())
+    for a, b in zip(*got):
+        assert np.array_equal(a, b)
+
+
+def test_autotuner_times_the_resident_kernel_as_one_form(built):
+    ts = [T.config1(k) for k in range(2)]
+    with capi.Context(precision=MIXED) as ctx:
+        ctx.upload(ts)
+        runs = ctx.resident_count()[0]
+        _, variant, _ = ctx.autotune(16)
+        # six skins in the run loop, two launches each; the forms of the
+        # sequence (four variants, two nodes) in none of theirs
+        tried = ctx.resident_count()[0] - runs
+        assert tried == 2 * (6 + (4 if variant == 0 else 0))
+        cfg = ctx.config()
+        assert cfg["variant"] == variant
+        if variant == 0:
+            assert cfg["rebuild_gate"] == 0
+        assert counted(ctx, 4, "graph")[1] == (1 if variant == 0 else 0)
