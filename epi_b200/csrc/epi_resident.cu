@@ -199,9 +199,9 @@ __device__ __forceinline__ BendTerm<R> bend_task(const DevState& S, int32_t i,
   if (!live) {
   } else if (tri) {
     const int k = e < 6 ? e : e - 6;
-    site[0] = M.tri(k);
-    site[1] = M.tri(k == 5 ? 0 : k + 1);
-    site[2] = e < 6 ? M.tri_ring(k) : M.tri(k >= 4 ? k - 4 : k + 2);
+    site[0] = M.tri(S, k);
+    site[1] = M.tri(S, k == 5 ? 0 : k + 1);
+    site[2] = e < 6 ? M.tri_ring(S, k) : M.tri(S, k >= 4 ? k - 4 : k + 2);
   } else {
     const bool col = e >= 3 && e < 6;
     const int d = e == 6 ? 0 : (kind == 0 ? -1 : (kind == 1 ? 0 : -2));
@@ -283,6 +283,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
     if (attr_state(a) == ST_MEMB) {
       const TissueDev& T = kOne ? T0 : S0.tissues[attr_tissue(a)];
       const int32_t j = i - T.pbase, at = atomicAdd(&s_nm, 1);
+      if (!EPI_CHECKED(at < A.membs, S0.status, i, at)) continue;
       K.list[at] = s;
       K.jk[at] = (uint32_t)(j % T.nmx) | (uint32_t)(j / T.nmx) << 16;
       K.at[s] = at;

@@ -206,6 +206,10 @@ struct MembSites {
       : MembSites(T, i, (i - T.pbase) % T.nmx, (i - T.pbase) / T.nmx) {}
   __device__ __forceinline__ MembSites(const TissueDev& T, int32_t i, int32_t jj_, int32_t kk_)
       : pb(T.pbase), nmx(T.nmx), nmy(T.nmy), jj(jj_), kk(kk_), nmemb(T.nmemb), self(i) {}
+  __device__ __forceinline__ int32_t site(const DevState& S, int32_t col, int32_t row) const {
+    const int32_t q = pb + row * nmx + col;
+    return EPI_CHECKED(q >= pb && q < pb + nmemb, S.status, self, q) ? q : self;
+  }
   // column jj+dj, row kk+dk with periodic wrap; the same wiring as _memb_init
   // (cellmanager.cpp:114-158)
   __device__ __forceinline__ int32_t square(const DevState& S, int dj, int dk) const {
@@ -214,21 +218,20 @@ struct MembSites {
     c -= c >= nmx ? nmx : 0;
     w += w < 0 ? nmy : 0;
     w -= w >= nmy ? nmy : 0;
-    const int32_t q = pb + w * nmx + c;
-    return EPI_CHECKED(q >= pb && q < pb + nmemb, S.status, self, q) ? q : self;
+    return site(S, c, w);
   }
-  __device__ __forceinline__ int32_t tri(int k) const {
+  __device__ __forceinline__ int32_t tri(const DevState& S, int k) const {
     const TriSite a = tri_step(TriSite{jj, kk}, k, nmx, nmy);
-    return pb + a.row * nmx + a.col;
+    return site(S, a.col, a.row);
   }
-  __device__ __forceinline__ int32_t tri_ring(int k) const {
+  __device__ __forceinline__ int32_t tri_ring(const DevState& S, int k) const {
     const TriSite a =
         tri_step(tri_step(TriSite{jj, kk}, k == 5 ? 0 : k + 1, nmx, nmy), k, nmx, nmy);
-    return pb + a.row * nmx + a.col;
+    return site(S, a.col, a.row);
   }
   // lattice links in connected_cell's order (square: l, r, b, u)
   __device__ __forceinline__ int32_t link(const DevState& S, bool is_tri, int k) const {
-    if (is_tri) return tri(k);
+    if (is_tri) return tri(S, k);
     return square(S, k == 0 ? -1 : (k == 1 ? 1 : 0), k == 2 ? -1 : (k == 3 ? 1 : 0));
   }
 };
@@ -279,9 +282,9 @@ __device__ __forceinline__ double3 memb_force(const DevState& S, int32_t i) {
   if (tri) {
     Vec3<R> n[6], c[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) n[k] = off(M.tri(k));
+    for (int k = 0; k < 6; ++k) n[k] = off(M.tri(S, k));
 #pragma unroll
-    for (int k = 0; k < 6; ++k) c[k] = off(M.tri_ring(k));
+    for (int k = 0; k < 6; ++k) c[k] = off(M.tri_ring(S, k));
 #pragma unroll
     for (int k = 0; k < 6; ++k) bend_add(f, tri_term1(n[k], n[(k + 1) % 6], c[k]));
 #pragma unroll
