@@ -695,15 +695,21 @@ __global__ void k_gate_check(DevState S) {
   }
 }
 
-// *moved = 1 when a particle of any of the m position sets in hist is beyond
-// the reach of the candidate rows (moved_too_far from their rebuild).
+// k_gate_check over the m position sets in hist. With moved, *moved = 1 stands
+// for the flags.
 __global__ void k_hist_check(DevState S, const double4* __restrict__ hist, int64_t m,
                              int32_t* moved) {
   GRID_STRIDE(e, 0, m * S.n_total) {
     const int64_t i = e % S.n_total;
+    const uint32_t t = attr_tissue(S.attr[i]);
     const double4 p = hist[e];
-    if (moved_too_far(S.skin, S.tissues[attr_tissue(S.attr[i])], p.x, p.y, p.z, S.bpos[i]))
+    if (!moved_too_far(S.skin, S.tissues[t], p.x, p.y, p.z, S.bpos[i])) continue;
+    if (moved) {
       *moved = 1;
+    } else {
+      S.gate[1 + t] = 1;
+      S.gate[0] = 1;
+    }
   }
 }
 

@@ -1279,20 +1279,33 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
   c->lists_fresh = false;
   if ((rc = check_status(c))) return rc;
   EPI_CUDA(cudaMemcpyAsync(xT, c->pos[c->cur], pbytes, cudaMemcpyDeviceToDevice, s));
+  // The context ends at X_T, after an error too: the recomputation leaves other
+  // positions, FP32 copies and candidates behind.
+  struct Settle {
+    epi_ctx* c;
+    const double4* xT;
+    ~Settle() {
+      (void)cudaMemcpyAsync(c->pos[c->cur], xT, sizeof(double4) * (size_t)c->n,
+                            cudaMemcpyDeviceToDevice, c->stream);
+      c->posf_stale = true;
+      launch_set_gates(make_state(c, c->cur), c->ntissues, c->stream);
+    }
+  } settle{c, xT};
   launch_adjoint_seed(make_state(c, c->cur), target, loss->cells_only, inv_cnt, lam0,
                       gpart, c->lc, s);
   double4* lam[2] = {lam0, lam1};
   int a = 0;
   ResidentPlan plan;
   const bool small = resident(c, &plan);
-  for (int32_t seg = nseg - 1; seg >= 0; --seg) {
-    const int32_t t0 = seg * K, t1 = std::min(t0 + K, nsteps), len = t1 - t0;
-    // recompute X_t0 .. X_{t1-1} from the checkpoint into hist
+  // recompute X_t0 .. X_{t0+len-1} from the checkpoint into hist. fresh: with
+  // candidates built at X_t0, whatever rows there are
+  auto recompute = [&](int32_t seg, int32_t len, bool fresh) -> int {
     if (small) {
       EPI_CUDA(cudaMemcpyAsync(hist, ckpt + (size_t)seg * n, pbytes, cudaMemcpyDeviceToDevice, s));
       DevState Sh = make_state(c, c->cur);
       Sh.pos_cur = hist;
-      launch_gate_check(Sh, c->lc, s);
+      if (fresh) launch_set_gates(Sh, nt, s);
+      else launch_gate_check(Sh, c->lc, s);
       if (len > 1) {
         if (c->cfg.precision == EPI_PREC_MIXED) launch_posf(Sh, c->lc, s);
         ResidentCfg rcfg = resident_cfg(c, false);
@@ -1303,24 +1316,39 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
       EPI_CUDA(cudaMemcpyAsync(c->pos[c->cur], ckpt + (size_t)seg * n, pbytes,
                                cudaMemcpyDeviceToDevice, s));
       c->posf_stale = true;
-      launch_gate_check(make_state(c, c->cur), c->lc, s);
+      if (fresh) launch_set_gates(make_state(c, c->cur), nt, s);
+      else launch_gate_check(make_state(c, c->cur), c->lc, s);
       for (int32_t t = 0; t < len; ++t) {
         EPI_CUDA(cudaMemcpyAsync(hist + (size_t)t * n, c->pos[c->cur], pbytes,
                                  cudaMemcpyDeviceToDevice, s));
         if (t + 1 < len) enqueue_step(c, c->cur, nullptr);
       }
     }
-    // Candidates built at the middle of the segment mostly reach its ends, so
-    // one check stands for a check and the rebuild's kernels at every step.
+    return EPI_OK;
+  };
+  for (int32_t seg = nseg - 1; seg >= 0; --seg) {
+    const int32_t t0 = seg * K, t1 = std::min(t0 + K, nsteps), len = t1 - t0;
+    if ((rc = recompute(seg, len, false))) return rc;
+    // Where the rows the recomputation ended with do not reach over the whole
+    // segment, rows built at its middle mostly do: one check stands for a
+    // check and the rebuild's kernels at every step.
     DevState Sm = make_state(c, c->cur);
     Sm.pos_cur = hist + (size_t)(len / 2) * n;
-    launch_set_gates(Sm, nt, s);
+    launch_hist_check(Sm, hist, len, nullptr, c->lc, s);
     launch_rebuild(Sm, whole(c), c->scan, c->lc, s, nullptr);
     int32_t far = 0;
     EPI_CUDA(cudaMemsetAsync(moved, 0, sizeof(int32_t), s));
     launch_hist_check(Sm, hist, len, moved, c->lc, s);
     EPI_CUDA(cudaMemcpyAsync(&far, moved, sizeof(int32_t), cudaMemcpyDeviceToHost, s));
-    if ((rc = check_status(c))) return rc;
+    rc = check_status(c);
+    if (rc == EPI_ERR_LIST_OVERFLOW) {
+      // The rows at the middle are longer than max_cand, which the forward
+      // steps' were not: candidates as those built them, checked at each step.
+      if ((rc = recompute(seg, len, true))) return rc;
+      far = 1;
+      rc = check_status(c);
+    }
+    if (rc) return rc;
     // and differentiate them in reverse
     for (int32_t t = len - 1; t >= 0; --t) {
       DevState St = make_state(c, c->cur);
@@ -1339,10 +1367,6 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
   }
   // the parameter partials and loss terms of all steps, per tissue
   launch_tissue_sum(make_state(c, c->cur), gpart, acc, c->lc, s);
-  // the context ends at X_T; its candidates are rebuilt before the next step
-  EPI_CUDA(cudaMemcpyAsync(c->pos[c->cur], xT, pbytes, cudaMemcpyDeviceToDevice, s));
-  c->posf_stale = true;
-  launch_set_gates(make_state(c, c->cur), nt, s);
   std::vector<double> h(4 * (size_t)nt);
   EPI_CUDA(cudaMemcpyAsync(h.data(), acc, 32 * (size_t)nt, cudaMemcpyDeviceToHost, s));
   if ((rc = check_status(c))) return rc;

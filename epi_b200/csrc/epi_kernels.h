@@ -158,8 +158,8 @@ struct AdjointBuffers {
   double4* bend;          // 13 bending-product slots per membrane particle
   double4* gpart;         // per-particle parameter partials (spring, eps, bend, loss)
 };
-// *moved = 1 when the candidate rows do not reach far enough for one of the m
-// position sets in hist.
+// Sets the gate of every tissue whose candidate rows do not reach far enough
+// for one of the m position sets in hist; with moved, *moved = 1 instead.
 void launch_hist_check(const DevState& S, const double4* hist, int32_t m, int32_t* moved,
                        const LaunchCfg& lc, cudaStream_t s);
 // Sets the gate of every tissue with a particle farther than skin/2 from
