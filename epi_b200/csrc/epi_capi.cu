@@ -90,7 +90,7 @@ struct epi_ctx {
   // the membrane sums run on `aux` beside the candidate rebuild (fork / join)
   cudaStream_t aux = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-  LaunchCfg lc{148, 256, 0, 0, 0, kDefaultSearchSwitch};
+  LaunchCfg lc{148, 256, 0, 0, 0, kDefaultSearchSwitch, 0};
   bool loaded = false;
   bool lists_fresh = false;  // nbr / nn / dermis match the current positions
   int32_t ntissues = 0;

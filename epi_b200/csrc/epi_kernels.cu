@@ -639,14 +639,16 @@ void launch_prepass(const DevState& S, int32_t m0, int32_t m1, int32_t f0, int32
 
 // The asynchronous-gather kernel with kS shared-memory slots per thread.
 template <typename R, bool kSimple, bool kOld, bool k16, int kS, int kMinBlocks>
-void launch_step_async(const DevState& S, const Range& r, cudaStream_t s) {
+void launch_step_async(const DevState& S, const Range& r, const LaunchCfg& lc, cudaStream_t s) {
   using Pos = typename std::conditional<sizeof(R) == 4, float4, double4>::type;
   auto kern = k_step_async<R, kSimple, kOld, kMinBlocks, k16, kS>;
   constexpr int smem = kS * kStepThreads * (int)sizeof(Pos);
-  static bool configured = false;
-  if (!configured) {
+  // once per context (and so per device) and form; every context sets the same
+  constexpr int form = (k16 ? 1 : 0) + (kS > 128 / (int)sizeof(Pos) ? 2 : 0) +
+                       4 * (kSimple ? (kOld ? 1 : 0) : 2) + (sizeof(R) == 4 ? 12 : 0);
+  if (!(lc.step_sized >> form & 1u)) {
     cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    configured = true;
+    lc.step_sized |= 1u << form;
   }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3((unsigned)blocks_for(r.p1 - r.p0, kStepThreads));
@@ -671,8 +673,8 @@ void launch_step_w(const DevState& S, const Range& r, const LaunchCfg& lc, cudaS
   const int grid = blocks_for(r.p1 - r.p0, 256);
   constexpr bool kF = sizeof(R) == 4;
   switch (lc.variant) {
-    case 1: launch_step_async<R, kSimple, kOld, k16, kF ? 8 : 4, kF ? 4 : 3>(S, r, s); break;
-    case 2: launch_step_async<R, kSimple, kOld, k16, kF ? 15 : 8, 3>(S, r, s); break;
+    case 1: launch_step_async<R, kSimple, kOld, k16, kF ? 8 : 4, kF ? 4 : 3>(S, r, lc, s); break;
+    case 2: launch_step_async<R, kSimple, kOld, k16, kF ? 15 : 8, 3>(S, r, lc, s); break;
     case 3: launch_pdl(k_step<R, kSimple, kOld, 3, k16>, grid, 256, s, S, r); break;
     default: launch_pdl(k_step<R, kSimple, kOld, kF ? 4 : 2, k16>, grid, 256, s, S, r); break;
   }

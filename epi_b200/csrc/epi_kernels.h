@@ -26,6 +26,7 @@ struct LaunchCfg {
   int any_old;      // some cell is older than THRESH_SP
   int variant;      // step-kernel instantiation (pipeline depth / residency), see epi_config
   int search_switch;  // rebuilt particles from which the search takes a thread per particle
+  mutable uint32_t step_sized;  // step kernels whose shared memory limit is set
 };
 
 // Kernel classes, for per-class timing.
