@@ -261,11 +261,14 @@ __device__ __forceinline__ F2 xfma(F2 a, F2 b, F2 c) {
 
 // FP64 path: the distance sqrt(d2) and 1 / d2 from i = 1 / sqrt(d2), each
 // corrected to within an ulp, as a square root and a division would give
-// (the laws subtract nearly equal numbers, so it would show). One rsqrt and
-// four multiply-adds stand for a square root and two divisions. Cells at one
-// place (d2 = 0, i infinite) get what those give, 0 and infinity, so that the
-// coefficient comes out infinite and is reported: the correction alone would
-// make it NaN, which passes the reference's test of its size.
+// (the laws subtract nearly equal numbers, so it would show): one Newton step
+// on the residual that a fused multiply-add leaves exact (P. W. Markstein,
+// Computation of elementary functions on the IBM RISC System/6000 processor,
+// IBM J. Res. Dev. 34, 1990). One rsqrt and four multiply-adds stand for a
+// square root and two divisions. Cells at one place (d2 = 0, i infinite) get
+// what those give, 0 and infinity, so that the coefficient comes out infinite
+// and is reported: the correction alone would make it NaN, which passes the
+// reference's test of its size.
 __device__ __forceinline__ double dist_of(double d2, double i) {
   const double d = xmul(d2, i);
   return d2 > 0.0 ? xfma(xmul(0.5, i), xfma(-d, d, d2), d) : d2;
