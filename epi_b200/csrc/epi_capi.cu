@@ -379,10 +379,10 @@ void enqueue_step(epi_ctx* c, int& cur, Timer* tm) {
 // Whether the batch steps in one resident kernel (epi_resident.cu) instead of
 // the kernel sequence; the results are the same bits. A configuration that
 // names a step-kernel form or a rebuild node asks for the sequence.
-bool resident(const epi_ctx* c, ResidentPlan* P) {
+bool resident(const epi_ctx* c, int32_t nsteps, ResidentPlan* P) {
   return c->coop && c->cfg.variant == 0 && c->cfg.rebuild_gate == 0 &&
          resident_plan(c->tissues_h.data(), c->ntissues, c->n, c->cfg.precision,
-                       c->cfg.max_cand, c->lc, P);
+                       c->cfg.max_cand, std::max(nsteps, 1), c->lc, P);
 }
 
 bool conditional_rebuild(const epi_ctx* c);
@@ -408,7 +408,7 @@ ResidentCfg resident_cfg(epi_ctx* c, bool graph) {
 // the device stops taking the launches). *posted: see check_status.
 int enqueue_resident(epi_ctx* c, int32_t* left, bool graph, bool* posted) {
   ResidentPlan P;
-  if (*left <= 0 || !resident(c, &P)) return EPI_OK;
+  if (*left <= 0 || !resident(c, *left, &P)) return EPI_OK;
   ensure_posf(c);
   ResidentCfg rc = resident_cfg(c, graph);
   c->status_h->flags = 0;
@@ -1296,7 +1296,7 @@ int epi_adjoint(epi_ctx* c, int32_t nsteps, int32_t K, const epi_loss* loss, dou
   double4* lam[2] = {lam0, lam1};
   int a = 0;
   ResidentPlan plan;
-  const bool small = resident(c, &plan);
+  const bool small = resident(c, (int32_t)hist_len, &plan);
   // recompute X_t0 .. X_{t0+len-1} from the checkpoint into hist. fresh: with
   // candidates built at X_t0, whatever rows there are
   auto recompute = [&](int32_t seg, int32_t len, bool fresh) -> int {
@@ -1606,7 +1606,7 @@ int epi_autotune(epi_ctx* c, int32_t trial_steps, double* skin_out, int32_t* var
   // more form; in any other 0 is one of 1 to 4.
   apply(best_skin, 0, switch0, 0);
   ResidentPlan plan;
-  const bool small = resident(c, &plan);
+  const bool small = resident(c, trial_steps, &plan);
   for (double skin : kSkins) {
     for (int32_t variant : kVariants) {
       if (variant == 0 && !small) continue;

@@ -85,7 +85,8 @@ struct ResidentCfg {
                       // hist + k n, writes hist + (k + 1) n
 };
 // How a batch is laid out over the blocks; false: the batch is beyond what
-// the resident kernel takes (particles, or shared memory per block).
+// the resident kernel takes (particles, or shared memory per block), or the
+// kernel sequence steps it faster in a run of nsteps.
 struct ResidentPlan {
   int32_t slots, grid, membs, turn, tasks, terms, group, smem;
 };
@@ -93,7 +94,7 @@ struct ResidentPlan {
 // 17 us per step at 147,456 particles)
 constexpr int64_t kResidentParticles = 131072;
 bool resident_plan(const TissueDev* tissues_h, int32_t ntissues, int64_t n, int precision,
-                   int max_cand, const LaunchCfg& lc, ResidentPlan* out);
+                   int max_cand, int32_t nsteps, const LaunchCfg& lc, ResidentPlan* out);
 cudaError_t launch_resident(const DevState& S, const ResidentPlan& plan, const TissueDev& first,
                             int32_t nsteps, int precision, const ResidentCfg& rc,
                             const LaunchCfg& lc, cudaStream_t s);

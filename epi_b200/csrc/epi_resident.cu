@@ -568,20 +568,35 @@ constexpr int kLeastSlots = 16;
 // density, a part of them for batches of every cell state, whose membrane rows
 // are short and cell rows long (the rest of a step's follow in turns)
 constexpr int kLeastTasks = 8, kLeastTasksGeneral = 3;
-// membrane particles per block: a step takes about 10 us and 0.07 more for
-// each (112: 17.5 us, 168: 21.9, 224: 26.2, mixed precision), the sequence 20
-// to 22 at the same sizes. (Batches of every cell state are not limited: 240
-// of FP64 29 us, the sequence 99.)
-constexpr int kMostMembs = 144;
-// Turns that the membrane terms of such a batch may take: at 64 tissues (472
-// membrane particles per block, FP64) two, 53 us a step; at 118 seven, 97;
-// the sequence 104 and 117.
+// Where the resident step is the faster one. A block walks its slots and its
+// membrane terms; a step of the sequence costs its launches whatever the batch
+// holds, and with every cell state as long as the longest row takes one
+// thread. So the resident step gains `base` and `row` per candidate of that
+// row, and loses `slot` per slot and `memb` per membrane particle of a block.
+// Nanoseconds, fitted to 8,512 batches of one to 420 tissues with both routes
+// timed (50-step runs); of 1,313 other ones two take the resident route and
+// lose more than 2 % by it (2.4 at most), and of the fitted ones 1 % take the
+// sequence and leave more than 5 %.
+// With 144 membrane particles per block as the only limit, and none in batches
+// of every state, 20 % lost more than 2 %, up to 2.5 times: 28 us a step
+// against 22 for six tissues of 63,116 particles under triangular membranes
+// (mixed), 118 against 99 for 105 small tissues of every state.
+struct Gain {
+  int32_t base, row, slot, memb;
+};
+// What a run saves once: its launches, eight against one (a call of one step
+// near the line: 4 us, between 0 and 12).
+constexpr int32_t kGainRun = 4000;
+constexpr Gain kGain[2][2][2] = {  // [every state][triangular][mixed]
+    {{{15000, 0, 16, 50}, {9800, 0, 10, 34}}, {{22800, 0, 31, 95}, {14200, 0, 15, 92}}},
+    {{{20900, 350, 30, 55}, {17700, 300, 23, 43}}, {{27400, 335, 46, 97}, {21000, 300, 27, 94}}}};
+// Turns that the membrane terms of a batch of every state may take.
 constexpr int kMostTurns = 8;
 
 }  // namespace
 
 bool resident_plan(const TissueDev* T, int32_t ntissues, int64_t n, int precision, int max_cand,
-                   const LaunchCfg& lc, ResidentPlan* out) {
+                   int32_t nsteps, const LaunchCfg& lc, ResidentPlan* out) {
   if (n <= 0 || n > kResidentParticles) return false;
   ResidentPlan P{};
   // an even share of the particles over all SMs, one block each
@@ -598,9 +613,12 @@ bool resident_plan(const TissueDev* T, int32_t ntissues, int64_t n, int precisio
   // membrane touches, dealt round
   bool tri = false;
   int64_t membs = 0, most = 0, of = 0;
+  double row = 0.0;  // membrane particles within reach of the largest cell
   for (int32_t t = 0; t < ntissues; ++t) {
     tri |= T[t].lattice == kLatticeTriangular;
     if (!T[t].nmemb) continue;
+    const double reach = T[t].P.lj_thresh * (T[t].rmax_nm + T[t].rmax);
+    row = std::max(row, 3.14159265 * reach * reach * T[t].nmemb / (T[t].lx * T[t].ly));
     const int64_t per = (int64_t)P.group * P.slots, end = T[t].pbase + T[t].nmemb;
     for (int64_t g = T[t].pbase / per; g <= (end - 1) / per; ++g) {
       if (g != of) membs = 0;
@@ -613,7 +631,10 @@ bool resident_plan(const TissueDev* T, int32_t ntissues, int64_t n, int precisio
     }
   }
   P.membs = (int32_t)std::min<int64_t>(P.slots, most);
-  if (lc.simple && P.membs > kMostMembs) return false;
+  const Gain& gain = kGain[lc.simple ? 0 : 1][tri ? 1 : 0][precision == 1 ? 1 : 0];
+  if (gain.base + kGainRun / nsteps + gain.row * std::min(row, (double)max_cand) <
+      (double)gain.slot * P.slots + (double)gain.memb * P.membs)
+    return false;
   P.terms = tri ? kTriTerms : kSquareTerms + 2;
   P.turn = P.membs;
   auto bytes = [&](int tasks) {

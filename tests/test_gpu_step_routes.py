@@ -36,6 +36,44 @@ def test_a_batch_that_fills_the_gpu_steps_in_the_sequence(built):
         assert counted(ctx, 2, "eager") == (16, 0, 0)
 
 
+def paired(ts):
+    """One dividing pair in the middle of the first tissue's cells."""
+    t = ts[0]
+    i = (t.nmemb + t.n) // 2
+    t.pair[i], t.pair[i + 1] = i + 1, i
+    t.spr_nat_len[i:i + 2] = 1.0
+    return ts
+
+
+# batches of up to 131,072 particles on either side of the line where the
+# kernel sequence becomes the faster one in a run of 50 steps: (tissues, resident
+# in FP64, in mixed precision)
+def routes():
+    tri = lambda side, layers, k: T.tri_layered_tissue(side, T.tri_rows(side), layers, k)
+    return {
+        "tri, few": (lambda: [tri(24, 3, k) for k in range(6)], True, True),
+        "tri, wide": (lambda: [tri(50, 3, k) for k in range(6)], False, False),
+        "one": (lambda: [T.layered_tissue(64, 8, 1)], True, True),
+        "one, large": (lambda: [T.layered_tissue(120, 7, 1)], False, False),
+        "a pair, small": (lambda: paired([T.layered_tissue(48, 5, 1)]), True, True),
+        "a pair, many": (lambda: paired([T.layered_tissue(48, 3, k) for k in range(12)]), False, False),
+        "a pair, tri": (lambda: paired([tri(48, 3, k) for k in range(10)]), False, False),
+        "all states, 40": (lambda: [T.mixed_state_tissue(k) for k in range(40)], True, True),
+        "all states, 100 tri": (lambda: [T.mixed_state_tissue(k, T.TRIANGULAR) for k in range(100)],
+                                False, False),
+    }
+
+
+@pytest.mark.parametrize("name", sorted(routes()))
+def test_the_faster_route_is_taken(built, name):
+    make, *resident = routes()[name]
+    ts = make()
+    for precision, want in zip((FP64, MIXED), resident):
+        with capi.Context(precision=precision, max_conn=96, max_cand=192) as ctx:
+            ctx.upload(ts)
+            assert counted(ctx, 50, "eager")[1] == (1 if want else 0), precision
+
+
 @pytest.mark.parametrize("precision", [FP64, MIXED])
 @pytest.mark.parametrize("named", [dict(variant=v) for v in (1, 2, 3, 4)] +
                          [dict(rebuild_gate=g) for g in (1, 2)])

@@ -2,8 +2,9 @@
 column and row of a membrane particle in 16 bits each) meets rows from 32,768
 on: against the kernel sequence, bit for bit, and the oracle. The three columns
 stand on a triangle, so that neighbours are nearer than half the box from each
-other; one DER cell far below makes the batch general, the form that takes this
-many membrane particles per block."""
+other; one DER cell far below makes the batch general, and the rows lie close, as
+those of a batch of every state do: the form that takes this many membrane
+particles per block."""
 import numpy as np
 import pytest
 
@@ -18,24 +19,29 @@ STEPS = 4
 
 
 def thin(rows, lattice):
-    s, nm = 1.8, 3 * rows
+    s, nm = 0.05, 3 * rows
     jj, kk = np.meshgrid(np.arange(3), np.arange(rows), indexing="xy")
     jj, kk = jj.ravel(), kk.ravel()
-    jit = (2.0 * T.splitmix64_uniform(rows, 3 * nm).reshape(nm, 3) - 1.0) * 0.05
+    jit = (2.0 * T.splitmix64_uniform(rows, 3 * nm).reshape(nm, 3) - 1.0) * s / 36
     x = np.append(3.0 + np.array([0.0, s, s / 2])[jj] + jit[:, 0], 4.0)
     y = np.append((kk + 0.5) * s + jit[:, 1], 4.0)
     z = np.append(8.0 + np.array([0.0, 0.0, s * 0.75 ** 0.5])[jj] + jit[:, 2], 1.5)
     n = nm + 1
+    # constants for the small spacing: displacements per step as at 1.8
+    p = T.Params(der_der_const=0.2 * s / 1.8, kbend=0.5 * (s / 1.8) ** 2,
+                 eps_m=0.01 * (s / 1.8) ** 2)
     t = T.Tissue(nmx=3, nmy=rows, lx=10.0, ly=rows * s, lz=20.0, x=x, y=y, z=z,
-                 radius=np.full(n, 1.3), state=np.append(np.full(nm, T.MEMB), T.DER).astype(np.uint8),
+                 radius=np.append(np.full(nm, 1.3 / 1.8 * s), 1.4),
+                 state=np.append(np.full(nm, T.MEMB), T.DER).astype(np.uint8),
                  agek=np.zeros(n), spr_nat_len=np.zeros(n), pair=np.full(n, -1, np.int32),
-                 rest_div_times=np.zeros(n, np.int32), nmemb=nm, nder=1, lattice=lattice)
+                 rest_div_times=np.zeros(n, np.int32), nmemb=nm, nder=1, lattice=lattice,
+                 params=p)
     t.validate()
     return t
 
 
 @pytest.mark.parametrize("precision", [capi.EPI_PREC_FP64, capi.EPI_PREC_MIXED])
-@pytest.mark.parametrize("rows,lattice", [(32770, T.SQUARE), (32800, T.SQUARE),
+@pytest.mark.parametrize("rows,lattice", [(32780, T.SQUARE), (32800, T.SQUARE),
                                           (32800, T.TRIANGULAR), (43600, T.SQUARE)])
 def test_rows_beyond_15_bits(built, rows, lattice, precision):
     t = thin(rows, lattice)
@@ -43,7 +49,7 @@ def test_rows_beyond_15_bits(built, rows, lattice, precision):
     fits = rows < 43600 or precision == capi.EPI_PREC_MIXED
     got = []
     for mode in ("eager", "per_tissue"):
-        with capi.Context(precision=precision) as ctx:
+        with capi.Context(precision=precision, max_cand=256) as ctx:
             ctx.upload([t])
             ctx.step(STEPS, mode)
             assert ctx.resident_count()[0] == (1 if fits and mode == "eager" else 0)
