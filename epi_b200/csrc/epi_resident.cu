@@ -580,7 +580,11 @@ constexpr int kLeastTasks = 8, kLeastTasksGeneral = 3;
 // With 144 membrane particles per block as the only limit, and none in batches
 // of every state, 20 % lost more than 2 %, up to 2.5 times: 28 us a step
 // against 22 for six tissues of 63,116 particles under triangular membranes
-// (mixed), 118 against 99 for 105 small tissues of every state.
+// (mixed), 118 against 99 for 105 small tissues of every state. (A rebuild
+// costs a resident run more, 0.8 ns per particle, 5 with every state: of 3,046
+// resident runs from a jittered start, which rebuild most, 8 % lose more than
+// 2 %, up to 1.5 times in runs of four steps. Sizes do not tell how often a
+// run rebuilds; a line for those runs would leave as much in the others.)
 struct Gain {
   int32_t base, row, slot, memb;
 };
