@@ -18,9 +18,8 @@
 //              thread its first 15 candidates without a dependent load.
 //   nbr[N][C]  i32 exact connection lists, materialised on request; nn[N].
 //              Membrane lattice links are implicit in both.
-//   sn/sm[N]   membrane bending scratch (unit vector + length to the right /
-//              upper lattice neighbour), the reference's Memb_data
-//              (epi5_MT/cell.h:42-69)
+//   fmemb[N]   membrane particles: bending, lattice springs and wall, summed
+//              by k_memb_force for the step kernel
 //   bins       counting-sort cell list over the reference's 2.0 grid
 #pragma once
 #include <cstdint>

@@ -55,7 +55,7 @@ __global__ void k_scan_partial(const int32_t* __restrict__ in, int32_t n,
   for (int k = 0; k < kScanItems; ++k)
     if (base + k < n) s += in[base + k];
   int32_t tot;
-  block_excl_scan(s, &tot);
+  block_excl_scan<kScanThreads>(s, &tot);
   if (threadIdx.x == 0) partial[blockIdx.x] = tot;
 }
 
@@ -71,7 +71,7 @@ __global__ void k_scan_top(int32_t* partial, int32_t nb, const int32_t* gate) {
     const int32_t i = base + threadIdx.x;
     const int32_t v = i < nb ? partial[i] : 0;
     int32_t tot;
-    const int32_t ex = block_excl_scan(v, &tot);
+    const int32_t ex = block_excl_scan<kScanThreads>(v, &tot);
     if (i < nb) partial[i] = carry + ex;
     carry += tot;
   }
@@ -90,7 +90,7 @@ __global__ void k_scan_final(const int32_t* __restrict__ in, int32_t* __restrict
     s += v[k];
   }
   int32_t tot;
-  int32_t run = block_excl_scan(s, &tot) + partial[blockIdx.x] + init;
+  int32_t run = block_excl_scan<kScanThreads>(s, &tot) + partial[blockIdx.x] + init;
 #pragma unroll
   for (int k = 0; k < kScanItems; ++k) {
     if (base + k < n) out[base + k] = run;

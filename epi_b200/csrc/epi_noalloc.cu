@@ -256,7 +256,6 @@ __global__ void __launch_bounds__(kThreads) na_connect(Args A) {
   const float tz = R + A.tol;
   int32_t z0 = cz < 2 ? 0 : cz - 2, z1 = cz + 2 < A.anz ? cz + 2 : A.anz - 1;
   while (z0 < cz && zf - (float)(z0 + 1) * agf > tz) ++z0;
-  
   while (z1 > cz && (float)z1 * agf - zf > tz) --z1;
   int32_t w0 = 0, w1 = -1;
   if (cz < 2) {

@@ -21,29 +21,10 @@ __device__ __forceinline__ int32_t warp_incl_scan(int32_t v) {
   return v;
 }
 
-// Block-wide exclusive scan of one value per thread; returns the prefix and
-// writes the block total to *total.
-__device__ __forceinline__ int32_t block_excl_scan(int32_t v, int32_t* total) {
-  __shared__ int32_t wsum[kScanThreads / 32];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  const int32_t incl = warp_incl_scan(v);
-  if (lane == 31) wsum[wid] = incl;
-  __syncthreads();
-  if (wid == 0) {
-    int32_t w = lane < kScanThreads / 32 ? wsum[lane] : 0;
-    w = warp_incl_scan(w);
-    if (lane < kScanThreads / 32) wsum[lane] = w;
-  }
-  __syncthreads();
-  const int32_t before = wid == 0 ? 0 : wsum[wid - 1];
-  *total = wsum[kScanThreads / 32 - 1];
-  __syncthreads();
-  return before + incl - v;
-}
-
-// Same for NT threads (a multiple of 32, at most 1024).
+// Block-wide exclusive scan of one value per thread over NT threads (a multiple
+// of 32, at most 1024); returns the prefix and writes the block total to *total.
 template <int NT>
-__device__ __forceinline__ int32_t block_excl_scan_n(int32_t v, int32_t* total) {
+__device__ __forceinline__ int32_t block_excl_scan(int32_t v, int32_t* total) {
   __shared__ int32_t wsum[NT / 32];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int32_t incl = warp_incl_scan(v);
@@ -133,9 +114,9 @@ __device__ __forceinline__ void gate_compact(const DevState& S, int32_t t0, int3
       nb = T.anx * T.any * T.anz;
     }
     int32_t tc, tp, tb;
-    const int32_t oc = block_excl_scan_n<NT>(g ? 1 : 0, &tc);
-    const int32_t op = block_excl_scan_n<NT>(np, &tp);
-    const int32_t ob = block_excl_scan_n<NT>(nb, &tb);
+    const int32_t oc = block_excl_scan<NT>(g ? 1 : 0, &tc);
+    const int32_t op = block_excl_scan<NT>(np, &tp);
+    const int32_t ob = block_excl_scan<NT>(nb, &tb);
     if (g) {
       S.rl_list[cc + oc] = t;
       S.rl_ppre[cc + oc] = cp + op;
@@ -256,7 +237,7 @@ __device__ __forceinline__ void rebuild_scan(const DevState& S) {
         sum += v[q];
       }
       int32_t tot;
-      int32_t run = carry + block_excl_scan_n<NT>(sum, &tot);
+      int32_t run = carry + block_excl_scan<NT>(sum, &tot);
 #pragma unroll
       for (int q = 0; q < kScanItems; ++q) {
         if (b0 + q < hi) out[b0 + q] = run;
@@ -476,7 +457,7 @@ struct SearchWindow {
   // that can be connected. kWrap = false: only for windows with neither
   // wrap_x nor wrap_y.
   template <bool kWrap>
-  __device__ __forceinline__ bool hit_t(int32_t s, const float4& q, float ex, float ey) const {
+  __device__ __forceinline__ bool hit(int32_t s, const float4& q, float ex, float ey) const {
     if (s == s_self || q.w < memb_lim) return false;
     float dx = ex - q.x, dy = ey - q.y;
     if (kWrap && wrap_x) dx = dx > fhx ? dx - flx : (dx <= -fhx ? dx + flx : dx);
@@ -484,9 +465,6 @@ struct SearchWindow {
     const float dz = pz - q.z;
     const float reach = rw + fabsf(q.w);
     return dx * dx + dy * dy + dz * dz <= reach * reach;
-  }
-  __device__ __forceinline__ bool hit(int32_t s, const float4& q, float ex, float ey) const {
-    return hit_t<true>(s, q, ex, ey);
   }
 };
 
@@ -568,7 +546,7 @@ __device__ __forceinline__ void cand_search_groups(const DevState& S, int32_t cn
         uint32_t key = 0;
         if (f < total) {
           key = S.skey[s];
-          hit = W.hit(s, S.spos[s], ex, ey);
+          hit = W.hit<true>(s, S.spos[s], ex, ey);
         }
         const unsigned m = (__ballot_sync(kAll, hit) >> gbase) & gmask;
         if (hit && in) {
@@ -685,7 +663,7 @@ __device__ __forceinline__ void search_particle(const DevState& S, const TissueD
     }
 #pragma unroll
     for (int u = 0; u < kWide; ++u) {
-      if (s + u < s_hi && W.template hit_t<kWrap>(s + u, q[u], ex, ey)) {
+      if (s + u < s_hi && W.template hit<kWrap>(s + u, q[u], ex, ey)) {
         if (count < cap) row.put(S, i, (key[u] & 0x7fffffffu) - pbase);
         ++count;
       }

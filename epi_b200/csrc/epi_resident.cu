@@ -233,8 +233,8 @@ __device__ __forceinline__ BendTerm<R> bend_task(const DevState& S, int32_t i,
 // constants each block has in shared memory (those of a single one, kOne, are
 // arguments), and deals them round in tiles of kTile particles, so that every
 // block gets its share of the membrane and of the long rows.
-template <typename R, bool kSimple, bool kOld, bool kOne, int NT, int kMin>
-__global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ DevState S0,
+template <typename R, bool kSimple, bool kOld, bool kOne, int NT>
+__global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ DevState S0,
                                                        const __grid_constant__ ResidentArgs A,
                                                        const __grid_constant__ TissueDev T0) {
   using Part = Particle<R, kSimple, kOld>;
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(NT, kMin) k_resident(const __grid_constant__ D
           }
         }
         int32_t total;
-        const int32_t before = block_excl_scan_n<NT>(nc, &total);
+        const int32_t before = block_excl_scan<NT>(nc, &total);
         if (s < slots) K.off[s] = carry + before;
         carry += total;
       }
@@ -553,9 +553,9 @@ template <typename R, bool kOne>
 const void* kernel_of(const LaunchCfg& lc, int* form) {
   const int kind = lc.simple ? (lc.any_old ? 1 : 0) : 2;
   *form = kind + (kOne ? 3 : 0) + (sizeof(R) == 4 ? 6 : 0);
-  if (kind == 1) return (const void*)k_resident<R, true, true, kOne, kThreads, 1>;
-  if (kind == 0) return (const void*)k_resident<R, true, false, kOne, kThreads, 1>;
-  return (const void*)k_resident<R, false, true, kOne, kThreads, 1>;
+  if (kind == 1) return (const void*)k_resident<R, true, true, kOne, kThreads>;
+  if (kind == 0) return (const void*)k_resident<R, true, false, kOne, kThreads>;
+  return (const void*)k_resident<R, false, true, kOne, kThreads>;
 }
 
 // Of 227 KB, less the static parts. The limit that every kernel is given,
