@@ -527,22 +527,27 @@ __global__ void __launch_bounds__(NT, 1) k_resident(const __grid_constant__ DevS
     }
   }
   if (blockIdx.x == 0 && tid == 0) {
-    if (done) flags.hand_on(A.nsteps);
     if (S0.launches) {
       atomicAdd(S0.launches, counted);
       atomicAdd(S0.launches + 1, 1ull);
       atomicAdd(S0.launches + 2, counted);
     }
     // past the last barrier every block has raised what it had to: the host
-    // finds the status after its wait for the stream, without a copy
-    if (A.post && done) {
+    // finds the status after its wait for the stream, without a copy. (All is
+    // read before anything is written: one trip to L2.)
+    if (done) {
+      const int32_t raised = *(const volatile int32_t*)flags.read_by(A.nsteps);
       const volatile DevStatus* from = S0.status;
-      volatile DevStatus* to = A.post;
-      to->code = from->code;
-      to->a = from->a;
-      to->b = from->b;
-      to->v = from->v;
-      to->flags = from->flags | kStatusPosted;
+      const DevStatus s{from->flags | kStatusPosted, from->code, from->a, from->b, from->v};
+      if (raised) flags.hand_on(A.nsteps);
+      if (A.post) {
+        volatile DevStatus* to = A.post;
+        to->code = s.code;
+        to->a = s.a;
+        to->b = s.b;
+        to->v = s.v;
+        to->flags = s.flags;
+      }
     }
   }
 }

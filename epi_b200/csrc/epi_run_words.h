@@ -27,12 +27,10 @@ struct RunFlags {
   EPI_HD int32_t* raised_by(int32_t step) const { return words + (step & 1); }
   EPI_HD int32_t* read_by(int32_t step) const { return step == 0 ? gate : raised_by(step - 1); }
   // After the last barrier, by one block (nobody else reads the words any
-  // more): what the last step raised becomes the next run's first flag.
+  // more), if the last step raised its word: the next run's first flag.
   EPI_HD void hand_on(int32_t nsteps) const {
-    volatile int32_t* last = read_by(nsteps);
-    if (!*last) return;
-    *last = 0;
-    *(volatile int32_t*)gate = 1;
+    *read_by(nsteps) = 0;
+    *gate = 1;
   }
 };
 

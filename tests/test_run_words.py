@@ -67,7 +67,7 @@ template <typename F> bool walk(int nb, int ns, unsigned raises, int first) {
         case REBUILT: b.at = COMMIT; break;
         case COMMIT: if (raised(k, b.step)) *f.raised_by(b.step) = 1; arrive(); b.at = READ; break;
         case READ: {
-          if (b.step + 1 == ns) { if (k == 0) f.hand_on(ns); b.at = OUT; break; }
+          if (b.step + 1 == ns) { if (k == 0 && *f.read_by(ns)) f.hand_on(ns); b.at = OUT; break; }
           const int got = *f.read_by(b.step + 1);
           ++b.step;
           if (got != expect(b.step)) return false;
